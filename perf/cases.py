@@ -368,11 +368,16 @@ class Plain:
         got = [torch.roll(f, tuple(-x for x in o), dims) for f in (self.r,) + fields]
         d = self.r - got[0]
         d = d - torch.round(d)
-        return d, (d ** 2).sum(0), got[1:]
+        r2 = (d ** 2).sum(0)
+        # the list's distance counts every axis, those beyond the dimension too
+        self.list_r2 = r2.detach()
+        if self.dim < 3:
+            self.list_r2 = self.list_r2 + ((self.rest - torch.roll(self.rest, tuple(-x for x in o), dims)) ** 2).sum(0)
+        return d, r2, got[1:]
 
-    def listed(self, m, r2):
-        """m where the pair is on the neighbour list, made with the h a pass starts from."""
-        return torch.where(r2 <= (self.krad * self.h_list) ** 2, m, torch.zeros_like(m))
+    def listed(self, m):
+        """m where the last shift's pair is on the neighbour list, made with the h a pass starts from."""
+        return torch.where(self.list_r2 <= (self.krad * self.h_list) ** 2, m, torch.zeros_like(m))
 
     def sums(self, h):
         """rho and its derivative in h."""
@@ -380,7 +385,7 @@ class Plain:
         w, q_ = self.m * f0, self.m * f0 * self.dim
         for o in self.offsets(h):
             _, r2, (mj,) = self.near(o, self.m)
-            mj = self.listed(mj, r2)
+            mj = self.listed(mj)
             q = r2.sqrt() / h
             f, df, _ = _shape(q, self.kernel)
             w = w + mj * f
@@ -441,7 +446,7 @@ class Plain:
         for o in self.offsets(h):
             x, r2, (m_, h_, rho_, Pi_, K_, P_, c_, u_, v_) = self.near(o, self.m, h, rho, Pi, K, P, c, self.u, self.v)
             r = r2.sqrt()
-            m_ = self.listed(m_, r2)
+            m_ = self.listed(m_)
             ga = K * _shape(r / h, self.kernel)[1] / r
             gb = K_ * _shape(r / h_, self.kernel)[1] / r
             v = self.v - v_
@@ -480,7 +485,7 @@ class Plain:
         D, a, du, dh, db = self.dim, self.a, self.du, self.dh, self.db
         r = self.r + dt * self.v[:D] + 0.5 * dt * dt * a[:D]
         self.r = r - torch.floor(r)
-        self.rest = self.rest + dt * self.v[D:] + 0.5 * dt * dt * a[D:]
+        self.rest = (self.rest + dt * self.v[D:] + 0.5 * dt * dt * a[D:]).detach()
         self.v, self.u, self.h = self.v + dt * a, self.u + dt * du, self.h + dt * dh
         self.b = self.b + dt * db
         density()
@@ -503,14 +508,14 @@ class Plain:
             for o in self.offsets(h):
                 x, r2, (m_, rho_, T_) = self.near(o, self.m, rho, T)
                 r = r2.sqrt()
-                w = mask(m_, r2) / rho / om * (T_ * rho_ - T * rho) * K * _shape(r / h, self.kernel)[1] / r
+                w = mask(m_) / rho / om * (T_ * rho_ - T * rho) * K * _shape(r / h, self.kernel)[1] / r
                 g = [g[k] + w * x[k] for k in range(D)]
             flux = torch.stack(g) * kk
             for o in self.offsets(h):
                 x, r2, (m_, h_, K_, Pi_, f_) = self.near(o, self.m, h, K, Pi, flux)
                 r = r2.sqrt()
                 ga, gb = K * _shape(r / h, self.kernel)[1] / r, K_ * _shape(r / h_, self.kernel)[1] / r
-                out = out + mask(m_, r2) * (ga * Pi * (flux * x).sum(0) + gb * Pi_ * (f_ * x).sum(0))
+                out = out + mask(m_) * (ga * Pi * (flux * x).sum(0) + gb * Pi_ * (f_ * x).sum(0))
             return out
         for o in self.offsets(h):
             x, r2, (m_, rho_, T_, k_) = self.near(o, self.m, rho, T, kk)
@@ -522,7 +527,7 @@ class Plain:
                 c = K / h * ddf * rr + ga * (tr - rr)
             else:
                 c = -ga * ((D + 2) * rr - tr)
-            out = out + mask(m_, r2) / (rho * rho_) * (T_ * rho_ - T * rho) * c
+            out = out + mask(m_) / (rho * rho_) * (T_ * rho_ - T * rho) * c
         return out
 
     def sts(self, s):
