@@ -298,7 +298,7 @@ struct sph_handle {
   // search afresh, keep), the fresh-search flag, its scan and those centres
   DevBuf skin_nl, skin_rowoff, skin_rowcap, skin_rowcap64, skin_cnt, skin_count_prev,
       skin_h_prev, skin_bx, skin_by, skin_bz, skin_hb, skin_sig, skin_dsp, skin_fcell,
-      skin_mcell, skin_ctmp, skin_gap, skin_hdev, skin_mode, skin_dflag, skin_dpos, skin_dlist,
+      skin_mcell, skin_ctmp, skin_gap, skin_href, skin_hdev, skin_mode, skin_dflag, skin_dpos, skin_dlist,
       skin_hrec, skin_ways, skin_wpos, skin_flist;
   // the rows of the centres searched afresh, laid out anew every skin-list
   // iterate after the end of the table's fixed part (skin_end[0]): their
@@ -827,6 +827,7 @@ struct sph_handle {
     RC(skin_dpos.ensure(sizeof(int32_t) * (nreal + 1)));
     RC(skin_dlist.ensure(sizeof(int32_t) * nreal));
     RC(skin_gap.ensure(sizeof(float) * nreal));
+    RC(skin_href.ensure(sizeof(double) * nreal));
     RC(skin_hdev.ensure(sizeof(double) * nreal));
     RC(skin_mode.ensure(sizeof(uint8_t) * nreal));
     RC(skin_ways.ensure(sizeof(int64_t) * (nreal + 1)));
@@ -909,12 +910,14 @@ struct sph_handle {
       if (!m.ghosts) for (int k = 0; k < 3; ++k) gg.periodic[k] = 0;
       launch_skin_sig(cols.as<double>(), nrows, gg, d, skin_sig.as<uint8_t>(), s);
       CK(cudaMemsetAsync(skin_dsp.p, 0, sizeof(float) * nall, s));
+      CK(cudaMemcpyAsync(skin_href.p, skin_hb.p, sizeof(double) * nreal, cudaMemcpyDeviceToDevice, s));
       CK(cudaMemsetAsync(skin_hdev.p, 0, sizeof(double) * nreal, s));
+      CK(cudaMemsetAsync(skin_gap.p, 0, sizeof(float) * nreal, s));  // (every centre records its gap)
       CK(cudaMemsetAsync(skin_mode.p, 0, sizeof(uint8_t) * nreal, s));
       CK(cudaMemsetAsync(skin_dflag.p, 0, sizeof(int32_t) * (nreal + 1), s));
     }
     skin_tau = 0.25 * skin * P.krad * hmin;
-    skin_eps = 1e-4 * P.krad * hmin;
+    skin_eps = 1e-5 * P.krad * hmin;
     skin_hmin = hmin;
     RC(fill_table(exact_table(), P, true, [&](NeibArgs& na, int) {
       launch_skin_filter(filter_args(na, false, true), s);
@@ -1005,7 +1008,7 @@ struct sph_handle {
       CK(cudaMemsetAsync(overflow.p, 0, sizeof(int32_t), s));
       dyn(ndirty);
       NeibArgs na = neib_args(T, P);
-      SkinFilterArgs fa = filter_args(na, true, false);
+      SkinFilterArgs fa = filter_args(na, true, true);
       fa.list = skin_flist.as<int32_t>();  // (the centres that filter)
       fa.nc = nfilter;
       launch_skin_filter(fa, s);
@@ -1105,7 +1108,8 @@ struct sph_handle {
                         skin_fcell.as<uint8_t>(), skin_mcell.as<uint8_t>(),
                         skin_ctmp.as<uint8_t>(), s);
       launch_skin_classify(nreal, centre_k.as<int32_t>(), skin_hrec.as<double>(),
-                           skin_hb.as<double>(), skin_hdev.as<double>(), skin_gap.as<float>(),
+                           skin_hb.as<double>(), skin_href.as<double>(),
+                           skin_hdev.as<double>(), skin_gap.as<float>(),
                            P.krad, 1.0 + skin_s, tau, eps, skin_dsp.as<float>(),
                            keys_alt.as<uint32_t>(), skin_fcell.as<uint8_t>(),
                            skin_mcell.as<uint8_t>(), skin_mode.as<uint8_t>(),

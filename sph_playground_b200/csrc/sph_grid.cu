@@ -980,13 +980,19 @@ k_neighbours(NeibArgs a) {
 //    widened by the largest displacement D): a record that moved more than
 //    tau ("fast") is within reach, the centre moved more than tau itself, or
 //    its h grew too far for the inequality above;
-//  * keep: no record of its skin list moved more than eps, nor did the
-//    centre, and 2 eps + krad |h_t - h_b| (running maximum) stays below the
-//    gap of step b (the smallest distance of a skin-list record from the
-//    sphere krad h_b): no record crossed the sphere, so the row written at
-//    b is the set at t (the row is not touched; the ways are monotone, so a
-//    kept row was never rewritten since b);
-//  * filter: its skin list through the FP64 predicate.
+//  * keep: no record of its skin list moved more than eps since b, nor did
+//    the centre, and 4 eps + krad |h_t - h_f| (running maximum since f) stays
+//    below the gap of f, the step its row was last written (the smallest
+//    distance then of a skin-list record from the sphere krad h_f): between
+//    f and t each of a pair's two records moved at most 2 eps, so no record
+//    crossed the sphere, and the row written at f is the set at t (the row
+//    is not touched while it is kept);
+//  * filter: its skin list through the FP64 predicate, with a new gap when
+//    the centre is as quiet as keeping asks (it moved at most eps and so did
+//    its list): what failed it was h, which may have settled since (the
+//    first Newton solve moves every h from the caller's guess; without the
+//    new gap its centres filtered every iterate from then on: 93 % of the
+//    rows at 128^3).
 // Either way each centre's set is the FP64 predicate's over all records,
 // i.e. that of a fresh search.  The image records of step b are reused when
 // no row's image signature changed (the image set is then the one the image
@@ -1145,7 +1151,8 @@ __global__ void k_dilate(const uint8_t* __restrict__ in, uint8_t* __restrict__ o
 // are the dilated cell flags (near_m == NULL: no centre keeps its row).
 __global__ void k_skin_classify(int64_t nc, const int32_t* __restrict__ centre_k,
                                 const double* __restrict__ hrec, const double* __restrict__ hb,
-                                double* __restrict__ hdev, const float* __restrict__ gap,
+                                double* __restrict__ href, double* __restrict__ hdev,
+                                float* __restrict__ gap,
                                 double krad, double kfac, float tau, float eps,
                                 const float* __restrict__ dsp,
                                 const uint32_t* __restrict__ keys,
@@ -1160,18 +1167,25 @@ __global__ void k_skin_classify(int64_t nc, const int32_t* __restrict__ centre_k
     const bool was_searched = mode[c] == 1;  // (a centre once searched afresh stays so)
     const int32_t k = centre_k[c];
     const double h = hrec[k], h0 = hb[c];
-    const double hd = fmax(hdev[c], fabs(h - h0));
-    hdev[c] = hd;
+    const double hd = fmax(hdev[c], fabs(h - href[c]));
     const double di = double(dsp[k]);
     const double lhs = krad * h * (1.0 + 1e-12) + di + double(tau);
     const double rhs = krad * h0 * kfac * (1.0 - 1e-12);
     const uint32_t cell = keys[k];  // the cell the centre was sorted into
     const bool clean = !was_searched && !near_f[cell] && dsp[k] <= tau && lhs < rhs;
     if (clean) {
-      const bool keep = near_m && !near_m[cell] && dsp[k] <= eps &&
-                        2.0 * double(eps) + krad * hd * (1.0 + 1e-12) + 1e-12 * krad * h0 <
-                            double(gap[c]);
+      const bool quiet = near_m && !near_m[cell] && dsp[k] <= eps;
+      const bool keep = quiet && 4.0 * double(eps) + krad * hd * (1.0 + 1e-12) +
+                                         1e-12 * krad * h0 <
+                                     double(gap[c]);
       w = keep ? 2 : 0;
+      if (keep) {
+        hdev[c] = hd;
+      } else {  // the filter writes the row at this h, and the new gap if quiet
+        href[c] = h;
+        hdev[c] = 0.0;
+        gap[c] = quiet ? 0.f : -1.f;
+      }
     }
     mode[c] = w;
     // one scan counts both lists: fresh searches in the low word, filters
@@ -1228,8 +1242,10 @@ k_gather_h(int64_t nc, const int32_t* __restrict__ centre_p, const double* __res
 // together; FP32 test with the search's guard band, FP64 predicate in the
 // band (the same arithmetic as the search, so the same decisions); the
 // round's hits go to the row in list order (prefix of the lanes' counts).
-// With gap != NULL each centre also records the smallest distance of a
-// list record from its sphere, less the FP32 images' error bound.
+// With gap != NULL the centres whose gap is not negative also record the
+// smallest distance of a list record from their sphere, less the error bound
+// of the FP32 images (a record that comes within 4 of those bounds is
+// measured in FP64, so that the bound does not eat the gap).
 // Counters and the longest row are summed over the block's whole share of
 // centres (a grid of a few blocks per SM strides over them) and leave it as
 // one atomic each: one atomic per centre on a single address would
@@ -1291,6 +1307,8 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
     const int rounds = __reduce_max_sync(FULL, active ? (n + PER - 1) / PER : 0);
     int cnt = 0;
     float gmin = 3.0e38f;
+    const bool want = active && a.gap && a.gap[c] >= 0.f;
+    const float gerr = a.eimg + 8e-7f * Rf * 1.2f;
     int32_t* const dst = a.nl + off;
     for (int r = 0; r < rounds; ++r) {
       const int base = r * PER + lane * V;
@@ -1310,11 +1328,16 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
           const float sd32 = dist2_f32(pj[j], pi);
           if ((sd32 < lo_thr && sd32 > 0.f) || sd32 > hi_thr) {
             if (sd32 <= hi_thr) m |= 1u << j;
-            if (a.gap) {
+            if (want) {
               // |r - R| from the images: their error (eimg) and the FP32
               // rounding of the distance, the root and the difference
               const float r32 = sqrtf(sd32);
-              gmin = fminf(gmin, fabsf(r32 - Rf) - (a.eimg + 4e-7f * (Rf + r32)));
+              float gj = fabsf(r32 - Rf) - (a.eimg + 4e-7f * (Rf + r32));
+              if (gj < gmin && gj < 4.f * gerr) {
+                const double e0 = a.sx[q[j]] - xi, e1 = a.sy[q[j]] - yi, e2 = a.sz[q[j]] - zi;
+                gj = __double2float_rd(fabs(sqrt(e0 * e0 + e1 * e1 + e2 * e2) - Rx) - 1e-9 * Rx);
+              }
+              gmin = fminf(gmin, gj);
             }
           } else if (q[j] != k) {
             ++nexact;
@@ -1324,7 +1347,7 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
             const double sd = __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)),
                                         __dmul_rn(d2, d2));
             if (!(sd > R2)) m |= 1u << j;
-            if (a.gap) gmin = fminf(gmin, __double2float_rd(fabs(sqrt(sd) - Rx) - 1e-9 * Rx));
+            if (want) gmin = fminf(gmin, __double2float_rd(fabs(sqrt(sd) - Rx) - 1e-9 * Rx));
           }
         }
       }
@@ -1355,7 +1378,7 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
       a.ncnt[c] = cnt;
       a.count_prev[a.orig[p]] = cnt;
       a.h_prev[a.orig[p]] = float(hi_);
-      if (a.gap) a.gap[c] = gmin;
+      if (want) a.gap[c] = gmin;
       maxc = max(maxc, cnt);
       ovf |= cnt > rcap;
       nfound += unsigned(cnt);
@@ -2498,14 +2521,14 @@ void launch_skin_gate(const unsigned long long* red, SkinGateIn in, int* gate, c
   note_launch();
 }
 void launch_skin_classify(int64_t nc, const int32_t* centre_k, const double* hrec,
-                          const double* hb, double* hdev, const float* gap, double krad,
+                          const double* hb, double* href, double* hdev, float* gap, double krad,
                           double kfac, float tau, float eps, const float* dsp,
                           const uint32_t* keys, const uint8_t* near_f, const uint8_t* near_m,
                           uint8_t* mode, int64_t* ways, int64_t* pos, int32_t* dlist,
                           int32_t* flist, void* scan_tmp, size_t scan_bytes,
                           const int32_t* ncnt, unsigned long long* nkept, cudaStream_t s) {
   if (nc <= 0) return;
-  k_skin_classify<<<nblocks(nc), TPB, 0, s>>>(nc, centre_k, hrec, hb, hdev, gap, krad, kfac, tau,
+  k_skin_classify<<<nblocks(nc), TPB, 0, s>>>(nc, centre_k, hrec, hb, href, hdev, gap, krad, kfac, tau,
                                               eps, dsp, keys, near_f, near_m, mode, ways, ncnt,
                                               nkept);
   cudaMemsetAsync(ways + nc, 0, sizeof(int64_t), s);

@@ -355,12 +355,12 @@ void launch_skin_marks(int64_t n, const float* dsp, float tau, float eps, const 
 // mode[c] = 0 (filter the skin list), 1 (search afresh) or 2 (keep the row)
 // for every centre (see sph_grid.cu), near_f / near_m the dilated cell
 // flags looked up by the cell keys[k] each centre's record was sorted into,
-// h of the centres from hrec (per record); hdev[c] = running maximum of
-// |h - hb[c]|.  The centres searched afresh go to dlist, those that filter
+// h of the centres from hrec (per record); href[c] = h when the row was last
+// written, hdev[c] = running maximum of |h - href[c]| since.  The centres searched afresh go to dlist, those that filter
 // to flist (in centre order); pos[nc] = their counts (low / high 32 bits);
 // ways and pos hold nc + 1 entries.  nkept[0..1] += rows kept, their pairs.
 void launch_skin_classify(int64_t nc, const int32_t* centre_k, const double* hrec,
-                          const double* hb, double* hdev, const float* gap, double krad,
+                          const double* hb, double* href, double* hdev, float* gap, double krad,
                           double kfac, float tau, float eps, const float* dsp,
                           const uint32_t* keys, const uint8_t* near_f, const uint8_t* near_m,
                           uint8_t* mode, int64_t* ways, int64_t* pos, int32_t* dlist,
@@ -435,6 +435,7 @@ struct SkinFilterArgs {
                         // (NULL with list NULL: every centre filters)
   int keep;
   float* gap;           // optional: per centre, the smallest |r - krad h| of its list
+                        // (written where it is not negative)
   float eimg;           // error bound of a distance between two FP32 images
   const int32_t* centre_k;
   const int32_t* centre_p;
