@@ -173,7 +173,7 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
           if (DIM == 3) r2 += dz * dz;
           const R r = rsq<R>(r2);
           const R q = r * ih;
-          bad |= !(q >= R(0));
+          bad |= q_bad(q);
           R f, df;
           if constexpr (sizeof(R) == 4) {
             // q carries the FP32 rounding of r/h; its residual (exact via FMA)
@@ -294,7 +294,7 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
         if (DIM == 3) r2 += dz * dz;
         const R r = rsq<R>(r2);
         const R q = r * ih;
-        bad |= !(q >= R(0));
+        bad |= q_bad(q);
         R f, df;
         if constexpr (sizeof(R) == 4) kshape_f_df_res<K>(q, fmaf(r, ih, -q) + r * ih_lo, f, df);
         else kshape_f_df<K, R>(q, f, df);

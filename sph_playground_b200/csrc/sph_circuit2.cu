@@ -27,8 +27,9 @@ inline int nblocks(int64_t n, int tpb = TPB) {
 
 template <class R> struct Part {
   PairPos<R> pos;
-  R m, invh, rho, Pi, P, c, u, vx, vy, vz;
-  R hrho, ac;  // rho / 2 and alpha c (the FP32 record's own fields)
+  // Pi of a neighbour is the record's wCv / (h^(d+1) rho^2 Omega), of the
+  // centre 1 / (rho^2 Omega); hrho = rho / 2, ac = alpha c, u = au u
+  R m, invh, rho, hrho, Pi, P, ac, u, vx, vy, vz;
 };
 template <class R> struct PartX {
   R T, kappa, gx, gy, gz, bx, by, bz;
@@ -41,7 +42,7 @@ template <> struct Loader<double> {
             d = __ldg(&pb.p[3][j]), e = __ldg(&pb.p[4][j]), f = __ldg(&pb.p[5][j]),
             g = __ldg(&pb.p[6][j]);
     o.pos.x = a.x; o.pos.y = a.y; o.pos.z = b.x; o.m = b.y;
-    o.invh = c.x; o.rho = c.y; o.Pi = d.x; o.P = d.y; o.c = e.x; o.u = e.y;
+    o.invh = c.x; o.hrho = c.y; o.rho = 2.0 * c.y; o.Pi = d.x; o.P = d.y; o.ac = e.x; o.u = e.y;
     o.vx = f.x; o.vy = f.y; o.vz = g.x;
   }
   static __device__ __forceinline__ void extra(const PackBufs& pb, int64_t j, PartX<double>& o) {
@@ -115,28 +116,26 @@ k_c2(C2Args a, PackBufs pb, Params P) {
     const int64_t ld = a.ld;
     Part<R> A;
     Loader<R>::hydro(pb, k, A);
-    if constexpr (sizeof(R) == 4) {
-      // the FP32 record's second rho field is wCv Pi / h^(d+1), the
+    {
+      // the record's second rho field is wCv Pi / h^(d+1), the
       // neighbour-side product; the centre takes Pi itself
       const double rr = cols[es_den * ld + p], oo = cols[es_om * ld + p];
-      A.Pi = float(1.0 / (rr * rr * oo));
+      A.Pi = R(1.0 / (rr * rr * oo));
     }
-    const R wcv = R(P.wCv);
-    R Ka = A.invh;
-    for (int d = 0; d < DIM; ++d) Ka *= A.invh;
-    Ka *= wcv;  // wCv / h_a^(d+1)
-    const R alpha = R(P.alpha), beta = R(P.beta), au = R(P.au);
+    R Kh = A.invh;
+    for (int d = 0; d < DIM; ++d) Kh *= A.invh;
+    Kh *= R(P.wCv);                      // wCv / h_a^(d+1)
+    const R Ka = Kh * R(KDfScale<K>::v);  // with f'(q) as kshape_df_scaled
+    const R beta = R(P.beta);
     const bool artts = P.artts == 1, adden = P.adden == 1, hydro = P.eq_hydro != 0;
     // the artificial conductivity term (circuit2.f90:316-331) is scaled by
     // au: au = -1 switches it off in the reference, and au = 0 makes it
     // vanish, so it is skipped for both
     const bool use_au = P.au != -1.0 && P.au != 0.0;
     const R rPiA = A.rho * A.Pi;  // 1 / (rho_a Omega_a)
-    R alpha_ca;
-    if constexpr (sizeof(R) == 4) alpha_ca = A.ac;
-    else alpha_ca = alpha * A.c;
+    const R alpha_ca = A.ac;
     const R hrhoa = R(-0.5) * A.rho, hrho_a = R(0.5) * A.rho, rPiA_h = R(0.5) * rPiA;
-    const R PiPa = hydro ? A.Pi * A.P : R(0);  // Pi_a P_a (the FP32 path's F and du)
+    const R PiPa = hydro ? A.Pi * A.P : R(0);  // Pi_a P_a
     // force-type sums: plain per lane (a few tens of terms), FP64 over lanes
     SumAcc<R> dv[3], du, drho, ddt, db[3];
     for (int d = 0; d < 3; ++d) { dv[d].init(); db[d].init(); }
@@ -206,91 +205,51 @@ k_c2(C2Args a, PackBufs pb, Params P) {
       if (DIM >= 2) vr += vab[1] * rab[1];
       if (DIM == 3) vr += vab[2] * rab[2];
       const R qa = r * A.invh, qb = r * B.invh;
-      bad |= !(qa >= R(0)) || !(qb >= R(0));
+      bad |= q_bad(qa) || q_bad(qb);
       R fa = R(0), dfa, ddfa = R(0);
       if constexpr (GENERAL) {
-        if (P.eq_diff && (P.ddw == esd_n2w || P.ddw == esd_fw)) kshape_all<K, R>(qa, fa, dfa, ddfa);
-        else dfa = kshape_df<K, R>(qa);
-      } else {
-        dfa = kshape_df<K, R>(qa);
+        if (P.eq_diff && (P.ddw == esd_n2w || P.ddw == esd_fw)) {
+          R d1;
+          kshape_all<K, R>(qa, fa, d1, ddfa);
+        }
       }
-      const R dfb = kshape_df<K, R>(qb);
+      dfa = kshape_df_scaled<K, R>(qa);
+      const R dfb = kshape_df_scaled<K, R>(qb);
       const R ga = (Ka * invr) * dfa;  // nabla W_a = ga * r_ab
       // nabla W_b = gb r_ab, which always meets Pi_b: gbPi = gb Pi_b, and
-      // cbr = wCv f'_b rho_b Pi_b / h_b^(d+1) for the conductivity.  The FP32
-      // record carries wCv Pi_b / h_b^(d+1) (a product formed in FP64 when
-      // packed, five products per pair fewer); FP64 forms them per pair.
-      R gb = R(0), gbPi, cbr;
-      if constexpr (sizeof(R) == 4) {
-        gbPi = (B.Pi * invr) * dfb;
-        cbr = (B.Pi * dfb) * B.hrho;  // half of it: the conductivity's 1/2 is folded in
-      } else {
-        R Kb = B.invh;
-        for (int d = 0; d < DIM; ++d) Kb *= B.invh;
-        Kb *= wcv;
-        gb = (Kb * invr) * dfb;
-        gbPi = gb * B.Pi;
-        cbr = Kb * dfb * B.rho * B.Pi;
-      }
-      // the neighbour's term gb x Pi_b of the general path
-      auto gbx = [&](R x) {
-        if constexpr (sizeof(R) == 4) return gbPi * x;
-        else return gb * x * B.Pi;
-      };
+      // cbr = wCv f'_b rho_b Pi_b / (2 h_b^(d+1)) for the conductivity (its
+      // 1/2 folded in).  The record carries wCv Pi_b / h_b^(d+1) with the
+      // scale of f', a product formed in FP64 when packed.
+      const R gbPi = (B.Pi * invr) * dfb;
+      const R cbr = (B.Pi * dfb) * B.hrho;
       const R mb = B.m;
       const R mgv = mb * ga * vr;      // m_b nabla W_a . v_ab
       if (adden) drho.add(mgv);        // circuit2.f90:265-267
-      // F = ga Pi_a Fa + gb Pi_b Fb (dv -= mb F r_ab); du += mgv Pi_a Da.
+      // F = ga (Pi_a Fa) + gbPi Fb (dv -= mb F r_ab); du += mgv (Pi_a Da).
       // With faba = Ka f'_a = ga r the viscous heating
       // mb dvr qav faba / (rho_a Omega_a) of circuit2.f90:329-334 is
       // mgv Pi_a (qav rho_a), and the pressure work of :343-344 is
-      // mgv Pi_a P_a.
-      R Fa = R(0), Fb = R(0), Da = R(0);
-      R FaPi = PiPa, DaPi = PiPa;  // FP32: Pi_a Fa and Pi_a Da, Pi_a folded in
+      // mgv Pi_a P_a.  Pi_a is folded into the centre's terms.
+      R FaPi = PiPa, Fb = R(0), DaPi = PiPa;
       if (artts) {
         // circuit2.f90:294-336; the Monaghan switch dvr < 0 as a clamp
+        // (the record carries rho_b / 2 and alpha c_b)
         const R dvr = vr * invr;
-        const R dneg = dvr < R(0) ? dvr : R(0);
+        const R dneg = -rmax0<R>(-dvr);
         const R qav = hrhoa * (alpha_ca - beta * dneg) * dneg;
-        // (FP32: the record carries rho_b / 2 and alpha c_b; the halvings
-        // are exact, so only alpha c_b is rounded differently)
-        R hrhob, acb;
-        if constexpr (sizeof(R) == 4) {
-          hrhob = B.hrho;
-          acb = B.ac;
-        } else {
-          hrhob = R(0.5) * B.rho;
-          acb = alpha * B.c;
-        }
-        const R qbv = (-hrhob) * (acb - beta * dneg) * dneg;
-        Fa = qav;
+        const R qbv = (-B.hrho) * (B.ac - beta * dneg) * dneg;
         Fb = qbv;
-        Da = qav * A.rho;
         FaPi = A.Pi * qav + PiPa;
         DaPi = qav * rPiA + PiPa;
-        if (use_au) {
+        if (use_au) {  // (u is au u)
           const R faba = Ka * dfa;
-          const R vsigu = fsqrt<R>(fdiv<R>(fabs(A.P - B.P), hrho_a + hrhob));
-          if constexpr (sizeof(R) == 4)
-            du.add(mb * (vsigu * (A.u - B.u) * (faba * rPiA_h + cbr)));  // (FP32 u is au u)
-          else
-            du.add(mb * (au * (vsigu * (A.u - B.u) * R(0.5) * (faba * rPiA + cbr))));
+          const R vsigu = froot_ratio(R(fabs(A.P - B.P)), hrho_a + B.hrho);
+          du.add(mb * (vsigu * (A.u - B.u) * (faba * rPiA_h + cbr)));
         }
       }
-      if (hydro) {
-        // circuit2.f90:338-345
-        Fa += A.P;
-        Fb += B.P;
-        Da += A.P;
-      }
-      R F;
-      if constexpr (sizeof(R) == 4) {
-        F = ga * FaPi + gbPi * Fb;
-        du.add(mgv * DaPi);
-      } else {
-        F = ga * A.Pi * Fa + gbPi * Fb;
-        du.add(mgv * A.Pi * Da);
-      }
+      if (hydro) Fb += B.P;  // circuit2.f90:338-345
+      const R F = ga * FaPi + gbPi * Fb;
+      du.add(mgv * DaPi);
       if constexpr (GENERAL) {
         PartX<R> BX;
         Loader<R>::extra(pb, j, BX);
@@ -321,9 +280,9 @@ k_c2(C2Args a, PackBufs pb, Params P) {
             rr = rr * (invr * invr);
             R contr;
             if (ddw == esd_n2w) {
-              contr = Ka * A.invh * ddfa * rr + ga * (tr - rr);
+              contr = Kh * A.invh * ddfa * rr + ga * (tr - rr);
             } else {
-              const R f2 = (ddw == esd_fab) ? -ga : R(0.5) * R(P.fwc) * Ka * A.invh * fa;
+              const R f2 = (ddw == esd_fab) ? -ga : R(0.5) * R(P.fwc) * Kh * A.invh * fa;
               contr = f2 * (R(DIM + 2) * rr - tr);
             }
             ddt.add(fdiv<R>(mb, B.rho * A.rho) * (BX.T * B.rho - AX.T * A.rho) * contr);
@@ -333,7 +292,7 @@ k_c2(C2Args a, PackBufs pb, Params P) {
             for (int x = 0; x < 3; ++x) kgb[x] = ktb[x][0] * gb3[0] + ktb[x][1] * gb3[1] + ktb[x][2] * gb3[2];
             R ka_r = R(0), kb_r = R(0);
             for (int x = 0; x < DIM; ++x) { ka_r += kga[x] * rab[x]; kb_r += kgb[x] * rab[x]; }
-            if (ddw == esd_2nw_ds) ddt.add(mb * (ga * ka_r * A.Pi + gbx(kb_r)));
+            if (ddw == esd_2nw_ds) ddt.add(mb * (ga * ka_r * A.Pi + gbPi * kb_r));
             else ddt.add(mb * A.Pi * ga * (kb_r - ka_r));  // esd_2nw_sd
           }
         }
@@ -347,7 +306,7 @@ k_c2(C2Args a, PackBufs pb, Params P) {
             const R rx = x < DIM ? rab[x] : R(0);
             const R ma_x = (halfB2a * rx - Ba[x] * Bar) * mu0inv;  // MPa . r_ab
             const R mb_x = (halfB2b * rx - Bb[x] * Bbr) * mu0inv;
-            dv[x].add(-mb * (ga * ma_x * A.Pi + gbx(mb_x)));
+            dv[x].add(-mb * (ga * ma_x * A.Pi + gbPi * mb_x));
             db[x].add(-mb * rPiA * ga * (vab[x] * Bar - Bb[x] * vr));
           }
         }

@@ -40,7 +40,18 @@ template <> struct KRad<KM4> { static constexpr double v = 2.0; };
 template <> struct KRad<KM6> { static constexpr double v = 3.0; };
 template <> struct KRad<KGAUSS> { static constexpr double v = 10.0; };
 
+// max(x, 0).  FP64: cleared by its sign bit, three integer operations in
+// place of a comparison on the FP64 pipe and two selects (a NaN with a clear
+// sign passes; every sum that meets one is reported through q_bad).
 template <class R> __device__ __forceinline__ R rmax0(R x) { return x > R(0) ? x : R(0); }
+template <> __device__ __forceinline__ double rmax0<double>(double x) {
+  const int hi = __double2hiint(x), m = ~(hi >> 31);
+  return __hiloint2double(hi & m, __double2loint(x) & m);
+}
+// q = r / h is negative or NaN (its high word, as unsigned, is above that of
+// infinity)
+__device__ __forceinline__ bool q_bad(float q) { return !(q >= 0.f); }
+__device__ __forceinline__ bool q_bad(double q) { return unsigned(__double2hiint(q)) > 0x7ff00000u; }
 
 template <int K, class R>
 __device__ __forceinline__ void kshape_f_df(R q, R& f, R& df) {
@@ -73,6 +84,27 @@ __device__ __forceinline__ R kshape_df(R q) {
     return R(-0.75) * (t2 * t2) + R(3) * (t1 * t1);
   } else {
     return R(-2) * exp(-q * q) * q;
+  }
+}
+
+// f'(q) / KDfScale<K>::v, for the force pass: the common factor of the
+// pieces goes into wCv / h^(d+1) once per particle instead of into every
+// pair (one product per kernel value fewer).
+template <int K> struct KDfScale;
+template <> struct KDfScale<KM4> { static constexpr double v = -0.75; };
+template <> struct KDfScale<KM6> { static constexpr double v = -5.0; };
+template <> struct KDfScale<KGAUSS> { static constexpr double v = -2.0; };
+template <int K, class R>
+__device__ __forceinline__ R kshape_df_scaled(R q) {
+  if constexpr (K == KM6) {
+    R t3 = rmax0(R(3) - q), t2 = rmax0(R(2) - q), t1 = rmax0(R(1) - q);
+    R s3 = t3 * t3, s2 = t2 * t2, s1 = t1 * t1;
+    return s3 * s3 - R(6) * (s2 * s2) + R(15) * (s1 * s1);
+  } else if constexpr (K == KM4) {
+    R t2 = rmax0(R(2) - q), t1 = rmax0(R(1) - q);
+    return t2 * t2 - R(4) * (t1 * t1);
+  } else {
+    return exp(-q * q) * q;
   }
 }
 
@@ -147,20 +179,44 @@ __device__ __forceinline__ R kshape_f(R q) {
   return f;
 }
 
+// 1 / sqrt(x) in FP64 from the hardware's approximation y (PTX
+// rsqrt.approx.ftz.f64, relative error below 2^-20): with e = 1 - x y^2,
+// 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 + 3 e^2 / 8 + O(e^3)), the
+// binomial series, whose next term is below 2^-58; within 2 ulp (the test of
+// the pair arithmetic compares it with 1 / sqrt).  No branch: x = 0 and
+// subnormal x (flushed to 0) give NaN.
+__device__ __forceinline__ double rsqrt_series(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 // Reciprocal square root, square root and division of the pair arithmetic.
-// FP64 keeps IEEE operations (the parity path); FP32 uses the MUFU
-// approximations (about 2 ulp), inside the FP32 path's error budget.
+// FP32 uses the MUFU approximations (about 2 ulp), inside the FP32 path's
+// error budget.  FP64 takes every root from rsqrt_series: a correctly rounded
+// square root or quotient is a longer sequence with a branch of its own, and
+// a pair of the force pass had two of each (the parity tolerance is 1e-12).
 template <class R> __device__ __forceinline__ R frsqrt(R x);
-template <> __device__ __forceinline__ double frsqrt<double>(double x) { return 1.0 / sqrt(x); }
+template <> __device__ __forceinline__ double frsqrt<double>(double x) { return rsqrt_series(x); }
 template <> __device__ __forceinline__ float frsqrt<float>(float x) { return rsqrtf(x); }
 template <class R> __device__ __forceinline__ R fsqrt(R x);
-template <> __device__ __forceinline__ double fsqrt<double>(double x) { return sqrt(x); }
+template <> __device__ __forceinline__ double fsqrt<double>(double x) {
+  // (below the normal range a separation counts as 0; a NaN stays one)
+  return x < 2.2250738585072014e-308 ? 0.0 : x * rsqrt_series(x);
+}
 template <> __device__ __forceinline__ float fsqrt<float>(float x) {
   return x > 0.f ? x * rsqrtf(x) : 0.f;
 }
 template <class R> __device__ __forceinline__ R fdiv(R a, R b);
 template <> __device__ __forceinline__ double fdiv<double>(double a, double b) { return a / b; }
 template <> __device__ __forceinline__ float fdiv<float>(float a, float b) { return __fdividef(a, b); }
+// sqrt(a / b) for a >= 0, b > 0 (FP32: as the quotient's root, which
+// measured faster there than one rsqrt of the product)
+__device__ __forceinline__ float froot_ratio(float a, float b) { return fsqrt<float>(fdiv<float>(a, b)); }
+__device__ __forceinline__ double froot_ratio(double a, double b) {
+  const double x = a * b;
+  return x < 2.2250738585072014e-308 ? 0.0 : a * rsqrt_series(x);
+}
 
 // h^n for small non-negative n (the reference's h**dim, h**(dim+2)).
 template <int N, class R>

@@ -1459,7 +1459,7 @@ struct sph_handle {
     // the positions (PACK_POS) were packed for circuit1 in this iterate and
     // have not moved; h, rho, Omega, P, c and grad T are new
     int groups = PACK_HYDRO | ((eq_diff || eq_magneto) ? PACK_EXTRA : 0);
-    pb.kp_wcv = P.wCv;
+    pb.kp_wcv = P.wCv * c2_df_scale(kernel_id);
     pb.kp_alpha = P.alpha;
     pb.kp_au = P.au;
     pb.kp_dim = P.dim;

@@ -1701,9 +1701,13 @@ __global__ void k_pack(int prec, int groups, int64_t n, const int32_t* __restric
     }
     if (groups & PACK_HYDRO) {
       double h = C(es_h), rho = C(es_den), om = C(es_om), P = C(es_p);
-      pb.p[2][k] = make_double2(1.0 / h, rho);
-      pb.p[3][k] = make_double2(1.0 / (rho * rho * om), P);
-      pb.p[4][k] = make_double2(C(es_c), C(es_u));
+      // (the same forms as the FP32 records below)
+      const double ih = 1.0 / h;
+      double kp = pb.kp_wcv;
+      for (int d = 0; d <= pb.kp_dim; ++d) kp *= ih;
+      pb.p[2][k] = make_double2(ih, 0.5 * rho);
+      pb.p[3][k] = make_double2(kp / (rho * rho * om), P);
+      pb.p[4][k] = make_double2(pb.kp_alpha * C(es_c), pb.kp_au * C(es_u));
       pb.p[5][k] = make_double2(C(es_vx), C(es_vy));
       pb.p[6][k] = make_double2(C(es_vz), C(es_t));
     }

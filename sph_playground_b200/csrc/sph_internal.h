@@ -492,6 +492,9 @@ void exclusive_scan64(void* tmp, size_t tmp_bytes, const int64_t* in, int64_t* o
 // sweeps of the diffusion paths read)
 enum PackGroup : int { PACK_POS = 1, PACK_HYDRO = 2, PACK_EXTRA = 4, PACK_TEMP = 8 };
 struct PackBufs {
+  // FP64: p[0], p[1] = x, y, z, m; p[2] = (1/h, rho / 2), p[3] =
+  // (wCv / (h^(d+1) rho^2 Omega), P), p[4] = (alpha c, au u), p[5], p[6] =
+  // v and T, p[7] .. p[10] the diffusion and field quantities
   double2* p[11];
   // FP32: q[0] = (x, y, z high parts, m), q[1] = (x, y, z low parts, 1/h),
   // q[2] = (rho / 2, wCv / (h^(d+1) rho^2 Omega), P, alpha c), q[3] = (au u, v), q[4] / q[5] the
@@ -502,7 +505,7 @@ struct PackBufs {
   // the length of one fixed-point unit (shift 2^-31), written by the pack
   // kernel (the frame may be planned on the device)
   float* unit;
-  // the force pass's FP32 factor wCv / h^(d+1), the viscosity's alpha and
+  // the force pass's factor wCv / h^(d+1) (times c2_df_scale), the viscosity's alpha and
   // the conductivity's au (set before its packing)
   double kp_wcv = 0.0, kp_alpha = 0.0, kp_au = 0.0;
   int kp_dim = 0;
@@ -626,6 +629,10 @@ struct C2Args {
   int* status;
   unsigned long long* dcnt;
 };
+// the factor of f' that the packed wCv / h^(d+1) carries (KDfScale)
+inline double c2_df_scale(int kernel) {
+  return kernel == KM6 ? KDfScale<KM6>::v : kernel == KM4 ? KDfScale<KM4>::v : KDfScale<KGAUSS>::v;
+}
 void launch_c2(int prec, int kernel, int dim, const C2Args& a, PackBufs pb, Params P,
                cudaStream_t s);
 
