@@ -101,8 +101,11 @@ __device__ __forceinline__ unsigned group_mask() {
 // G lanes per centre: each lane sums every G-th neighbour of the centre's
 // row of the neighbour list (coalesced), the group adds its lanes' two-sum
 // partials in FP64, and every lane takes the same FP64 Newton step.
+// (FP32: 6 blocks per SM, 80 registers, no spill: 128^3, 4 lanes, density
+// pass 3.22 ms, blast step 0.955; 7 blocks 3.39 / 0.936, 8 with 24 spilled
+// bytes 3.46 / 1.026.)
 template <int K, int DIM, class R, int G>
-__global__ void __launch_bounds__(TPB, 8)
+__global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 8)
 k_c1_newton(C1Args a, PackBufs pb, Params P) {
   const int64_t c = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G;
   const int lane = threadIdx.x & (G - 1);
@@ -139,10 +142,7 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
       // the density sum keeps its two-sum partials (its smoothness in h is
       // what the Newton iteration needs); the d rho / dh sum only scales the
       // Newton step and Omega, so a plain per-lane sum suffices
-      Acc<R> sw;
-      SumAcc<R> so;
-      sw.init();
-      so.init();
+      double sw_lane, so_lane;
       // U neighbours per lane per round: their pair data are all requested
       // before the first is used, so the gathers overlap; the list entries
       // of the next round are read one round ahead
@@ -150,48 +150,99 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
       int32_t jn[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) jn[u] = (lane + u * G < n) ? row[lane + u * G] : -1;
-      for (int l0 = lane; l0 < n; l0 += G * U) {
-        int64_t jj[U];
+      if constexpr (sizeof(R) == 4) {
+        // FP32: two neighbours per packed instruction.  The kernel is bound
+        // by instruction issue (83 instructions a pair one at a time, NA_C1)
+        // and has FMA time to spare.  An entry past the row's end is record
+        // 0 with mass 0.  Separations are whole fixed-point units, so r2 is 0
+        // or at least 1 and rsqrt(max(r2, 1)) serves both; q = r / h is NaN
+        // or negative only if 1/h is.
+        bad |= n > 0 && q_bad(float(ih));
+        Acc2 sw;
+        sw.init();
+        F2 so(0.f);
+        const F2 ih2(ih), nih2(-ih), ihl2(ih_lo);
+        for (int l0 = lane; l0 < n; l0 += G * U) {
+          FixPos pj[U];
+          float mj[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) jj[u] = jn[u];
-        typename PosAccess<R>::Pos pj[U];
-        R mj[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) pj[u] = PosAccess<R>::load(pb, jj[u] >= 0 ? jj[u] : 0, mj[u]);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int l = l0 + (U + u) * G;
-          jn[u] = l < n ? row[l] : -1;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (jj[u] < 0) continue;
-          R dx, dy, dz;
-          pos_delta(pi, pj[u], dx, dy, dz, R(1));
-          R r2 = dx * dx;
-          if (DIM >= 2) r2 += dy * dy;
-          if (DIM == 3) r2 += dz * dz;
-          const R r = rsq<R>(r2);
-          const R q = r * ih;
-          bad |= q_bad(q);
-          R f, df;
-          if constexpr (sizeof(R) == 4) {
-            // q carries the FP32 rounding of r/h; its residual (exact via FMA)
-            // and the residuals of the kernel pieces enter f to first order,
-            // so the density sum varies smoothly with h below FP32 resolution
-            // and the Newton iterates converge instead of cycling between
-            // neighbouring FP32 values (kshape_f_df_res).
-            const R q_lo = fmaf(r, ih, -q) + r * ih_lo;
-            kshape_f_df_res<K>(q, q_lo, f, df);
-          } else {
-            kshape_f_df<K, R>(q, f, df);
+          for (int u = 0; u < U; ++u) {
+            pj[u] = PosAccess<float>::load(pb, jn[u] >= 0 ? jn[u] : 0, mj[u]);
+            if (jn[u] < 0) mj[u] = 0.f;
           }
-          sw.add(mj[u] * f);
-          so.add(mj[u] * (R(DIM) * f + q * df));
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int l = l0 + (U + u) * G;
+            jn[u] = l < n ? row[l] : -1;
+          }
+#pragma unroll
+          for (int u = 0; u < U; u += 2) {
+            const F2 dx(__int2float_rn(pi.x - pj[u].x), __int2float_rn(pi.x - pj[u + 1].x));
+            F2 r2 = f2_mul(dx, dx);
+            if (DIM >= 2) {
+              const F2 dy(__int2float_rn(pi.y - pj[u].y), __int2float_rn(pi.y - pj[u + 1].y));
+              r2 = f2_fma(dy, dy, r2);
+            }
+            if (DIM == 3) {
+              const F2 dz(__int2float_rn(pi.z - pj[u].z), __int2float_rn(pi.z - pj[u + 1].z));
+              r2 = f2_fma(dz, dz, r2);
+            }
+            const F2 r = f2_mul(r2, F2(rsqrtf(fmaxf(r2.x(), 1.f)), rsqrtf(fmaxf(r2.y(), 1.f))));
+            const F2 q = f2_mul(r, ih2);
+            // q carries the FP32 rounding of r/h; its residual (exact via
+            // FMA) and the residuals of the kernel pieces enter f to first
+            // order, so the density sum varies smoothly with h below FP32
+            // resolution and the Newton iterates converge instead of cycling
+            // between neighbouring FP32 values (kshape_f_df_res).
+            F2 f, df;
+            kshape_f_df_res2<K>(q, r, nih2, ihl2, f, df);
+            const F2 m2(mj[u], mj[u + 1]);
+            sw.add(f2_mul(m2, f));
+            so = f2_fma(m2, f2_fma(q, df, f2_mul(F2(float(DIM)), f)), so);
+          }
         }
+        sw_lane = sw.dval();
+        so_lane = double(so.x()) + double(so.y());
+      } else {
+        Acc<R> sw;
+        SumAcc<R> so;
+        sw.init();
+        so.init();
+        for (int l0 = lane; l0 < n; l0 += G * U) {
+          int64_t jj[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) jj[u] = jn[u];
+          typename PosAccess<R>::Pos pj[U];
+          R mj[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) pj[u] = PosAccess<R>::load(pb, jj[u] >= 0 ? jj[u] : 0, mj[u]);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int l = l0 + (U + u) * G;
+            jn[u] = l < n ? row[l] : -1;
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (jj[u] < 0) continue;
+            R dx, dy, dz;
+            pos_delta(pi, pj[u], dx, dy, dz, R(1));
+            R r2 = dx * dx;
+            if (DIM >= 2) r2 += dy * dy;
+            if (DIM == 3) r2 += dz * dz;
+            const R r = rsq<R>(r2);
+            const R q = r * ih;
+            bad |= q_bad(q);
+            R f, df;
+            kshape_f_df<K, R>(q, f, df);
+            sw.add(mj[u] * f);
+            so.add(mj[u] * (R(DIM) * f + q * df));
+          }
+        }
+        sw_lane = sw.dval();
+        so_lane = so.dval();
       }
-      const double swt = group_sum<G>(sw.dval(), gmask);
-      const double sot = group_sum<G>(so.dval(), gmask);
+      const double swt = group_sum<G>(sw_lane, gmask);
+      const double sot = group_sum<G>(so_lane, gmask);
       // W = wCv f / h^d; dW/dh = -wCv / h^(d+1) (d f + q f')  (kernel.f90:178-187, 239-249)
       const double ihd = 1.0 / ipow<DIM>(ha);
       const double wsum = wcv * ihd * (a.mref * swt + ma * double(f0));

@@ -132,6 +132,47 @@ __device__ __forceinline__ void kshape_all(R q, R& f, R& df, R& ddf) {
   }
 }
 
+// ---- two FP32 values per instruction ----------------------------------------
+// Blackwell's packed FP32 operations (PTX f32x2): one instruction for two
+// independent multiply-adds, each rounded as the scalar one.  They halve the
+// issue slots of FP32 arithmetic, not its time on the FMA pipe, so they pay
+// where a kernel is bound by instruction issue.
+struct F2 {
+  unsigned long long v;
+  F2() = default;
+  __device__ __forceinline__ F2(float a, float b) {
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  }
+  __device__ __forceinline__ explicit F2(float a) : F2(a, a) {}
+  __device__ __forceinline__ float x() const {
+    float a;
+    asm("mov.b64 {%0, _}, %1;" : "=f"(a) : "l"(v));
+    return a;
+  }
+  __device__ __forceinline__ float y() const {
+    float b;
+    asm("mov.b64 {_, %0}, %1;" : "=f"(b) : "l"(v));
+    return b;
+  }
+};
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, F2(-1.f), a); }  // (exact product)
+__device__ __forceinline__ F2 f2_max0(F2 a) { return F2(fmaxf(a.x(), 0.f), fmaxf(a.y(), 0.f)); }
+
 // FP32 f(q) that follows q below FP32 resolution, for the Newton iteration on
 // h.  q_lo is the rounding residual of q = r/h.  q is split as qh + dq with
 // qh on the 2^-21 grid (for q < 4, q + 4 carries an ulp of 2^-21, so the add
@@ -169,6 +210,39 @@ __device__ __forceinline__ void kshape_f_df_res(float q, float q_lo, float& f, f
     f = e;
     df = -2.f * e * q;
     f = fmaf(df, q_lo, f);
+  }
+}
+
+// The same for two values, from q = r ih rounded and r, ih_lo: q_lo, the
+// residual of q, is r ih_lo - (q - r ih), the bracket exact by FMA.  nqh is
+// -qh.  (The Gauss kernel: one after the other.)
+template <int K>
+__device__ __forceinline__ void kshape_f_df_res2(F2 q, F2 r, F2 neg_ih, F2 ih_lo, F2& f, F2& df) {
+  const F2 ne = f2_fma(r, neg_ih, q);
+  if constexpr (K == KM6 || K == KM4) {
+    const F2 nqh = f2_sub(F2(4.0f), f2_add(q, F2(4.0f)));
+    const F2 dq = f2_fma(r, ih_lo, f2_sub(f2_add(q, nqh), ne));
+    constexpr int NP = (K == KM6) ? 3 : 2;
+    const float cs[3] = {K == KM6 ? 3.f : 2.f, K == KM6 ? 2.f : 1.f, 1.f};
+    const float as[3] = {K == KM6 ? 1.f : 0.25f, K == KM6 ? -6.f : -1.f, 15.f};
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      const F2 th = f2_max0(f2_add(F2(cs[k]), nqh));  // exact: both on the 2^-21 grid
+      const F2 s = f2_mul(th, th);
+      const F2 p = K == KM6 ? f2_mul(s, s) : s;
+      const F2 pt = f2_mul(p, th);
+      const float d = (K == KM6 ? -5.f : -3.f) * as[k];
+      f = k == 0 ? (as[0] == 1.f ? pt : f2_mul(F2(as[0]), pt)) : f2_fma(F2(as[k]), pt, f);
+      df = k == 0 ? f2_mul(F2(d), p) : f2_fma(F2(d), p, df);
+    }
+    f = f2_fma(df, dq, f);
+  } else {
+    const F2 q_lo = f2_sub(f2_mul(r, ih_lo), ne);
+    float f0, d0, f1, d1;
+    kshape_f_df_res<K>(q.x(), q_lo.x(), f0, d0);
+    kshape_f_df_res<K>(q.y(), q_lo.y(), f1, d1);
+    f = F2(f0, f1);
+    df = F2(d0, d1);
   }
 }
 
@@ -245,6 +319,21 @@ template <class R> struct Acc {
   }
   __device__ __forceinline__ R val() const { return s + c; }
   __device__ __forceinline__ double dval() const { return double(s) + double(c); }
+};
+// two of them side by side
+struct Acc2 {
+  F2 s, c;
+  __device__ __forceinline__ void init() { s = F2(0.f); c = F2(0.f); }
+  __device__ __forceinline__ void add(F2 x) {
+    const F2 t = f2_add(s, x);
+    const F2 bp = f2_sub(t, s);
+    const F2 e = f2_add(f2_sub(s, f2_sub(t, bp)), f2_sub(x, bp));
+    s = t;
+    c = f2_add(c, e);
+  }
+  __device__ __forceinline__ double dval() const {
+    return (double(s.x()) + double(c.x())) + (double(s.y()) + double(c.y()));
+  }
 };
 // Plain running sum in R with the same interface: a lane's share of a pair
 // loop (n terms) carries at most gamma_n * sum|t| of rounding, about 2e-6

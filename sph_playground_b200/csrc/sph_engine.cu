@@ -457,9 +457,22 @@ struct sph_handle {
     int g = lanes_ok(int(st[SPH_P_LANES_SEARCH]));
     return g ? g : (dim() == 3 ? 8 : 8);
   }
+  // Lanes per centre of the pair passes: 4 waste least on a row's tail and
+  // on the sums over the lanes, more keep the GPU busy when the centres are
+  // few.  circuit1 + circuit2 of a blast (3D) or shear (2D) step in us, FP64:
+  //   3D 16^3  4 lanes 134, 8  83, 16  54   2D  32^2  4 lanes 33, 8 26, 16 23, 32 21
+  //      32^3          184,   140,    134       64^2          33,   28,    25,    31
+  //      48^3          373,   345,    386      128^2          38,   41,    52
+  //      64^3          732,   750,    874      256^2          83,   97,   130
+  // (FP32 3D: 48^3 201 / 198, 64^3 409 / 429, 128^3 2913 / 3160 with 4 / 8.)
+  // 1D rows hold about 7 neighbours: at most 8.
   int lanes_pair() const {
     int g = lanes_ok(int(st[SPH_P_LANES_PAIR]));
-    return g ? g : (dim() == 3 ? 8 : 4);
+    if (g) return g;
+    if (dim() == 3) return nreal >= 200000 ? 4 : nreal >= 16000 ? 8 : 16;
+    if (nreal >= 12000) return 4;
+    if (dim() == 1 || nreal >= 6000) return 8;
+    return nreal >= 2000 ? 16 : 32;
   }
 
   int params(Params& P) {
