@@ -251,7 +251,7 @@ struct sph_handle {
   DevBuf pk[11], qk[7], qunit;
   // neighbours: one row per centre inside nl, rows sized from each
   // particle's previous count (CSR with slack)
-  DevBuf nl, ncnt, rowoff, rowcap, rowcap64, count_prev, h_prev, scan64_tmp, overflow;
+  DevBuf nl, ncnt, rowoff, rowcap, rowcap64, count_prev, h_prev, scan64_tmp;
   // adjoint: per-row adjoint columns, d/d(alpha, beta), checkpoints of the
   // particle table (the run's initial state, every k-th step, the final one)
   // and the states of the segment being replayed
@@ -298,13 +298,15 @@ struct sph_handle {
   // search afresh, keep), the fresh-search flag, its scan and those centres
   DevBuf skin_nl, skin_rowoff, skin_rowcap, skin_rowcap64, skin_cnt, skin_count_prev,
       skin_h_prev, skin_bx, skin_by, skin_bz, skin_hb, skin_sig, skin_dsp, skin_fcell,
-      skin_mcell, skin_ctmp, skin_gap, skin_href, skin_hdev, skin_mode, skin_dflag, skin_dpos, skin_dlist,
-      skin_hrec, skin_ways, skin_wpos, skin_flist;
+      skin_mcell, skin_gap, skin_href, skin_hdev, skin_mode, skin_dflag, skin_dpos, skin_dlist,
+      skin_hrec, skin_flist;
   // the rows of the centres searched afresh, laid out anew every skin-list
   // iterate after the end of the table's fixed part (skin_end[0]): their
   // capacities and the scan of those
   DevBuf skin_end, skin_dcap, skin_doff;
-  DevBuf skin_gate;  // the iterate's checks and mark windows (k_skin_gate)
+  DevBuf skin_out, skin_bcnt;  // a served iterate's result (SkinOut), its blocks' list lengths
+  SkinOut* h_skin = nullptr;   // (pinned)
+  int skin_most = 0;           // blocks of k_skin_serve resident at once
   // rows renamed: spare signatures, the two permutations, the old types, a flag
   DevBuf skin_sig_alt, skin_inv, skin_perm, skin_type, skin_flag;
   int64_t skin_nl_size = 0;
@@ -582,8 +584,7 @@ struct sph_handle {
     RC(status.ensure(sizeof(int)));
     RC(red.ensure(sizeof(unsigned long long) * RED_TOTAL));
     RC(dcnt.ensure(sizeof(unsigned long long) * DC_TOTAL));
-    RC(maxcnt.ensure(sizeof(int32_t)));
-    RC(overflow.ensure(sizeof(int32_t)));
+    RC(maxcnt.ensure(2 * sizeof(int32_t)));  // the longest row, and the overflow flag
     RC(count_prev.ensure(sizeof(int32_t) * nrows));
     RC(h_prev.ensure(sizeof(float) * nrows));
     RC(rowoff.ensure(sizeof(int64_t) * nreal));
@@ -637,6 +638,7 @@ struct sph_handle {
     return pb;
   }
 
+  int32_t* overflow_p() const { return maxcnt.as<int32_t>() + 1; }
   int check_status() {
     int code = 0;
     CK(cudaMemcpyAsync(h_i32, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -743,7 +745,7 @@ struct sph_handle {
     na.count_prev = T.count_prev->as<int32_t>();
     na.h_prev = T.h_prev->as<float>();
     na.maxcnt = maxcnt.as<int32_t>();
-    na.overflow = overflow.as<int32_t>();
+    na.overflow = overflow_p();
     na.dcnt = dcnt.as<unsigned long long>();
     return na;
   }
@@ -781,12 +783,10 @@ struct sph_handle {
           RC(T.nl->ensure(sizeof(int32_t) * *T.nl_size));
         }
       }
-      CK(cudaMemsetAsync(maxcnt.p, 0, sizeof(int32_t), s));
-      CK(cudaMemsetAsync(overflow.p, 0, sizeof(int32_t), s));
+      CK(cudaMemsetAsync(maxcnt.p, 0, 2 * sizeof(int32_t), s));
       NeibArgs na = neib_args(T, P);
       pass(na, attempt);
-      CK(cudaMemcpyAsync(h_i32, maxcnt.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(h_i32 + 1, overflow.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(h_i32, maxcnt.p, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       CK(cudaGetLastError());
       int mc = h_i32[0];
@@ -835,7 +835,7 @@ struct sph_handle {
   }
   int skin_alloc(int64_t nall) {
     RC(skin_alloc_common(nall));
-    RC(skin_gate.ensure(sizeof(int) * 4));
+    RC(skin_out.ensure(sizeof(SkinOut)));
     RC(skin_dflag.ensure(sizeof(int32_t) * (nreal + 1)));
     RC(skin_dpos.ensure(sizeof(int32_t) * (nreal + 1)));
     RC(skin_dlist.ensure(sizeof(int32_t) * nreal));
@@ -843,8 +843,6 @@ struct sph_handle {
     RC(skin_href.ensure(sizeof(double) * nreal));
     RC(skin_hdev.ensure(sizeof(double) * nreal));
     RC(skin_mode.ensure(sizeof(uint8_t) * nreal));
-    RC(skin_ways.ensure(sizeof(int64_t) * (nreal + 1)));
-    RC(skin_wpos.ensure(sizeof(int64_t) * (nreal + 1)));
     RC(skin_flist.ensure(sizeof(int32_t) * nreal));
     RC(skin_end.ensure(sizeof(int64_t)));
     // (renaming rows: re-sorts and uploads allocate nothing while lists serve)
@@ -943,6 +941,28 @@ struct sph_handle {
     cnt_host[SPH_CNT_SKIN_BUILDS]++;
     return SPH_OK;
   }
+  SkinRefresh refresh_args(const BoxGeom& g, int d, float tau, float eps) {
+    SkinRefresh r{};
+    r.sidx = vals_alt.as<int32_t>();
+    r.nrows = nrows;
+    r.nreal = nreal;
+    r.cols = cols.as<double>();
+    r.ld = nrows;
+    r.gsrc = gsrc.as<int32_t>();
+    r.gcode = gcode.as<int8_t>();
+    r.g = g;
+    r.dim = d;
+    r.sig_b = skin_sig.as<uint8_t>();
+    r.bx = skin_bx.as<double>(); r.by = skin_by.as<double>(); r.bz = skin_bz.as<double>();
+    r.sx = sx.as<double>(); r.sy = sy.as<double>(); r.sz = sz.as<double>();
+    r.s32 = s32.as<float4>();
+    r.dsp = skin_dsp.as<float>();
+    r.tau = tau;
+    r.eps = eps;
+    r.hrec = skin_hrec.as<double>();
+    r.red = red.as<unsigned long long>();
+    return r;
+  }
   FewArgs few_args(const NeibArgs& na, const int32_t* list, int64_t n, double reach) {
     FewArgs f{};
     f.n = n;
@@ -971,12 +991,12 @@ struct sph_handle {
     return f;
   }
   // The exact table of a skin-list iterate.  The kept rows stay where they
-  // are; the filtered ones are written in place; the centres searched afresh
-  // (skin_dlist, ndirty of them) get rows laid out anew after the table's
-  // fixed part.  A filter row that overflows joins the centres searched
+  // are; the filtered ones have been written in place (longest row mc, ov:
+  // a row overflowed); the centres searched afresh (skin_dlist, ndirty of
+  // them) get rows laid out anew after the table's fixed part.  A filter row that overflows joins the centres searched
   // afresh (for good: mode 1); when their rows find no room either, the
   // whole table is laid out anew and every row written.
-  int skin_fill(const Params& P, int64_t ndirty, int64_t nfilter, double reach) {
+  int skin_fill(const Params& P, int64_t ndirty, int mc, int ov, double reach) {
     const int d = P.dim;
     Table T = exact_table();
     // the centres searched afresh (skin_dlist): a lane group each when they
@@ -1003,8 +1023,7 @@ struct sph_handle {
                       rowcap.as<int32_t>(), s);
     };
     auto read_flags = [&](int& mc, int& ov) -> int {
-      CK(cudaMemcpyAsync(h_i32, maxcnt.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(h_i32 + 1, overflow.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(h_i32, maxcnt.p, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       CK(cudaGetLastError());
       mc = h_i32[0];
@@ -1014,21 +1033,14 @@ struct sph_handle {
                                      "complete within its wait limit");
       return SPH_OK;
     };
-    int mc = 0, ov = 0;
-    {
+    int mc_all = mc;
+    if (ndirty > 0) {
       Phase ph(this, SPH_T_NEIGHBOURS);
-      CK(cudaMemsetAsync(maxcnt.p, 0, sizeof(int32_t), s));
-      CK(cudaMemsetAsync(overflow.p, 0, sizeof(int32_t), s));
       dyn(ndirty);
       NeibArgs na = neib_args(T, P);
-      SkinFilterArgs fa = filter_args(na, true, true);
-      fa.list = skin_flist.as<int32_t>();  // (the centres that filter)
-      fa.nc = nfilter;
-      launch_skin_filter(fa, s);
       search_dirty(na, ndirty, reach);
-      RC(read_flags(mc, ov));
+      RC(read_flags(mc_all, ov));
     }
-    int mc_all = mc;
     if (ov) {
       // overflowed filter rows join the fresh searches; all of those anew
       Phase ph(this, SPH_T_NEIGHBOURS);
@@ -1043,7 +1055,7 @@ struct sph_handle {
                          cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       ndirty = h_i32[3];
-      CK(cudaMemsetAsync(overflow.p, 0, sizeof(int32_t), s));
+      CK(cudaMemsetAsync(overflow_p(), 0, sizeof(int32_t), s));
       dyn(ndirty);
       NeibArgs na = neib_args(T, P);
       search_dirty(na, ndirty, reach);
@@ -1075,103 +1087,80 @@ struct sph_handle {
     const int d = P.dim;
     const int64_t nall = nrows + nghost;
     BoxGeom g = box(m);
-    {
-      Phase ph(this, SPH_T_GHOSTS);
-      if (m.ghosts) launch_reflect(cols.as<double>(), nrows, nreal, g, s);
-    }
-    BoxGeom gg = g;
-    if (!m.ghosts) for (int k = 0; k < 3; ++k) gg.periodic[k] = 0;
-    const float tau = float(skin_tau), eps = float(skin_eps);
-    unsigned long long* rb = red.as<unsigned long long>();
+    if (!m.ghosts) for (int k = 0; k < 3; ++k) g.periodic[k] = g.reflect[k] = 0;
+    const int64_t ncell = int64_t(grid.nx) * grid.ny * grid.nz;
+    if (skin_most <= 0) skin_most = skin_serve_most_blocks();
+    const int blocks = skin_most > 0 ? skin_serve_blocks(nall, skin_most) : 0;
+    if (blocks <= 0) return fail(SPH_ERR_CUDA, "skin lists: no cooperative launch");
+    RC(skin_fcell.ensure(2 * size_t(ncell)));
+    RC(skin_mcell.ensure(2 * size_t(ncell)));
+    RC(skin_bcnt.ensure(sizeof(int2) * size_t(blocks)));
     {
       Phase ph(this, SPH_T_NEIGHBOURS);
-      SlotInit si{};
-      for (int k = 0; k < 3; ++k) {
-        si.off[si.n] = RED_LO_X + k; si.val[si.n++] = dkey(1e308);
-        si.off[si.n] = RED_HI_X + k; si.val[si.n++] = dkey(-1e308);
+      SkinServe a{};
+      a.r = refresh_args(g, d, float(skin_tau), float(skin_eps));
+      a.wrap = m.ghosts ? 1 : 0;
+      a.nall = nall;
+      a.pg = pgeom;
+      a.grid = grid;
+      a.keys = keys_alt.as<uint32_t>();
+      for (int k = 0; k < 2; ++k) {
+        a.fcell[k] = skin_fcell.as<uint8_t>() + k * ncell;
+        a.mcell[k] = skin_mcell.as<uint8_t>() + k * ncell;
       }
-      si.off[si.n] = RED_SKIN_D; si.val[si.n++] = dkey(0.0);
-      si.off[si.n] = RED_SKIN_HMAX; si.val[si.n++] = dkey(0.0);
-      launch_init_slots(rb, si, s);
-      // (the signature flag and the four counts are plain integers)
-      CK(cudaMemsetAsync(rb + RED_SKIN_SIG, 0, 5 * sizeof(unsigned long long), s));
-      launch_skin_refresh(vals_alt.as<int32_t>(), nall, nrows, nreal, cols.as<double>(),
-                          gsrc.as<int32_t>(), gcode.as<int8_t>(), gg, d, skin_sig.as<uint8_t>(),
-                          skin_bx.as<double>(), skin_by.as<double>(), skin_bz.as<double>(),
-                          sx.as<double>(), sy.as<double>(), sz.as<double>(), s32.as<float4>(),
-                          pgeom, skin_dsp.as<float>(), tau, eps, skin_hrec.as<double>(), rb, s);
-      // the checks and the marks' windows on the device, then the marks and
-      // every centre's way: the iterate asks the host once, after the ways
-      // (when a check failed, the host ends the lists and drops the ways)
-      SkinGateIn gi{};
-      gi.dcap = P.krad * skin_hmin;
-      gi.krad = P.krad;
-      gi.tau = skin_tau;
-      gi.kfac = 1.0 + skin_s;
-      gi.invL = grid.invL;
-      gi.pg = pgeom;
-      int* gate = skin_gate.as<int>();
-      launch_skin_gate(rb, gi, gate, s);
-      const int64_t ncell = int64_t(grid.nx) * grid.ny * grid.nz;
-      RC(skin_fcell.ensure(size_t(ncell)));
-      RC(skin_mcell.ensure(size_t(ncell)));
-      RC(skin_ctmp.ensure(size_t(ncell)));
-      launch_skin_marks(nall, skin_dsp.as<float>(), tau, eps, keys_alt.as<uint32_t>(),
-                        sx.as<double>(), sy.as<double>(), sz.as<double>(), grid, d, gate + 1,
-                        skin_fcell.as<uint8_t>(), skin_mcell.as<uint8_t>(),
-                        skin_ctmp.as<uint8_t>(), s);
-      launch_skin_classify(nreal, centre_k.as<int32_t>(), skin_hrec.as<double>(),
-                           skin_hb.as<double>(), skin_href.as<double>(),
-                           skin_hdev.as<double>(), skin_gap.as<float>(),
-                           P.krad, 1.0 + skin_s, tau, eps, skin_dsp.as<float>(),
-                           keys_alt.as<uint32_t>(), skin_fcell.as<uint8_t>(),
-                           skin_mcell.as<uint8_t>(), skin_mode.as<uint8_t>(),
-                           skin_ways.as<int64_t>(), skin_wpos.as<int64_t>(),
-                           skin_dlist.as<int32_t>(), skin_flist.as<int32_t>(), scan64_tmp.p,
-                           scan64_tmp.bytes, ncnt.as<int32_t>(), rb + RED_SKIN_NKEPT, s);
-      CK(cudaMemcpyAsync(h_red, rb, sizeof(unsigned long long) * RED_TOTAL,
-                         cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(h_red + RED_TOTAL, skin_wpos.as<int64_t>() + nreal, sizeof(int64_t),
-                         cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(h_i32 + 8, gate, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
+      a.nc = nreal;
+      a.centre_k = centre_k.as<int32_t>();
+      a.hb = skin_hb.as<double>();
+      a.href = skin_href.as<double>();
+      a.hdev = skin_hdev.as<double>();
+      a.gap = skin_gap.as<float>();
+      a.mode = skin_mode.as<uint8_t>();
+      a.ncnt = ncnt.as<int32_t>();
+      a.krad = P.krad;
+      a.kfac = 1.0 + skin_s;
+      a.dcap = P.krad * skin_hmin;
+      a.dirty_share = kSkinDirtyShare;
+      a.block_counts = skin_bcnt.as<int2>();
+      a.dlist = skin_dlist.as<int32_t>();
+      a.flist = skin_flist.as<int32_t>();
+      a.flags = maxcnt.as<int32_t>();
+      a.out = skin_out.as<SkinOut>();
+      CK(launch_skin_serve(a, blocks, s));
+      // the centres that filter, their number known to the device alone; the
+      // host is asked once for both
+      SkinFilterArgs fa = filter_args(neib_args(exact_table(), P), true, true);
+      fa.list = skin_flist.as<int32_t>();
+      fa.nc_dev = &skin_out.as<SkinOut>()->nfilter;
+      launch_skin_filter(fa, s);
+      CK(cudaMemcpyAsync(h_skin, skin_out.p, sizeof(SkinOut), cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(h_i32, maxcnt.p, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       CK(cudaGetLastError());
     }
-    const double D = dkey_inv(h_red[RED_SKIN_D]);
-    const unsigned long long nfast = h_red[RED_SKIN_NFAST], nmove = h_red[RED_SKIN_NMOVE];
+    const double D = h_skin->D;
     // (SPH_SKIN_TRACE in the environment: why lists end, on stderr)
     auto end_lists = [&](const char* why) {
       if (skin_trace)
-        std::fprintf(stderr, "skin lists end after %d iterates: %s (D %.3g, fast %llu, moving %llu)\n",
-                     skin_age, why, D, nfast, nmove);
+        std::fprintf(stderr, "skin lists end after %d iterates: %s (D %.3g, fast %lld, moving %lld)\n",
+                     skin_age, why, D, h_skin->nfast, h_skin->nmove);
       return SPH_OK;
     };
-    switch (h_i32[8]) {
+    switch (h_skin->why) {
       case 0: break;
       case 1: return end_lists("an image set changed");
       case 2: return end_lists("records moved a search radius");
       case 3: return end_lists("h");
       case 4: return end_lists("a record left the FP32 binade");
-      default: return end_lists("a search radius spans too many cells");
+      case 5: return end_lists("a search radius spans too many cells");
+      default: return end_lists("too many centres to search afresh");
     }
-    const int64_t counts = reinterpret_cast<const int64_t*>(h_red + RED_TOTAL)[0];
-    const int64_t ndirty = counts & 0xffffffffll, nfilter = counts >> 32;
-    const int64_t nkept = int64_t(h_red[RED_SKIN_NKEPT]);
-    // Their search over cells of step b, its range widened by D, costs
-    // several times a search's share per centre (measured on the 128^3
-    // Sedov blast: about 20 ns a centre against 1 ns); the iterate is
-    // served only while that stays well below a plain search (images, sort
-    // and search) with the widening of the smallest radius
-    const double rmin = P.krad * skin_hmin;
-    const double widen = std::pow((rmin + D) / rmin, double(d));
-    if (double(ndirty) * widen > kSkinDirtyShare * double(nreal))
-      return end_lists("too many centres to search afresh");
+    const int64_t nkept = h_skin->nkept, kept = h_skin->kept_pairs;
     const double reach_d = D * (1.0 + 1e-9);
-    RC(skin_fill(P, ndirty, nfilter, reach_d));
+    RC(skin_fill(P, h_skin->ndirty, h_i32[0], h_i32[1], reach_d));
     ++skin_age;
     cnt_host[SPH_CNT_SKIN_REUSES]++;
     cnt_host[SPH_CNT_SKIN_KEPT] += nkept;
-    kept_pairs += int64_t(h_red[RED_SKIN_NKEPT_PAIRS]);
+    kept_pairs += kept;
     served = true;
     return SPH_OK;
   }
@@ -1619,12 +1608,7 @@ struct sph_handle {
     si.off[si.n] = RED_DSKIN_FAIL; si.val[si.n++] = 0ull;
     si.off[si.n] = RED_SKIN_SIG; si.val[si.n++] = 0ull;
     launch_init_slots(rb, si, s);
-    launch_skin_refresh(vals_alt.as<int32_t>(), nall_cap, nrows, nreal, cols.as<double>(),
-                        gsrc.as<int32_t>(), gcode.as<int8_t>(), gg, d, skin_sig.as<uint8_t>(),
-                        skin_bx.as<double>(), skin_by.as<double>(), skin_bz.as<double>(),
-                        sx.as<double>(), sy.as<double>(), sz.as<double>(), s32.as<float4>(),
-                        PackGeom{}, skin_dsp.as<float>(), 0.f, 0.f, skin_hrec.as<double>(), rb, s,
-                        plan, ds);
+    launch_skin_refresh(refresh_args(gg, d, 0.f, 0.f), nall_cap, s, plan, ds);
     launch_dskin_check(nreal, centre_p.as<int32_t>(), col(es_h), skin_hb.as<double>(), P.krad, ds,
                        rb, s);
     RC(capture_if(
@@ -1654,7 +1638,7 @@ struct sph_handle {
     f.count_prev = count_prev.as<int32_t>();
     f.h_prev = h_prev.as<float>();
     f.maxcnt = maxcnt.as<int32_t>();
-    f.overflow = overflow.as<int32_t>();
+    f.overflow = overflow_p();
     f.dcnt = dcnt.as<unsigned long long>();
     f.plan = plan;
     f.skin_cap = skin_rowcap.as<int32_t>();
@@ -1746,7 +1730,7 @@ struct sph_handle {
     na.count_prev = t_cp.as<int32_t>();
     na.h_prev = t_hp.as<float>();
     na.maxcnt = maxcnt.as<int32_t>();
-    na.overflow = overflow.as<int32_t>();
+    na.overflow = overflow_p();
     na.dcnt = dcnt.as<unsigned long long>();
     if (skin) {
       DevSkin* ds = dskin.as<DevSkin>();
@@ -1866,7 +1850,7 @@ struct sph_handle {
   // the work of one step, with every size and decision on the device
   int step_body_dev() {
     CK(cudaMemsetAsync(drs_err.p, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(overflow.p, 0, sizeof(int32_t), s));
+    CK(cudaMemsetAsync(overflow_p(), 0, sizeof(int32_t), s));
     Params P{};
     RC(params(P));
     unsigned long long* r = red.as<unsigned long long>();
@@ -1973,7 +1957,7 @@ struct sph_handle {
     // one read-back per step: the clock, the error words
     CK(cudaMemcpyAsync(h_ctrl + 1, drs_clock.p, sizeof(DevClock), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(h_i32 + 4, drs_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(h_i32 + 5, overflow.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(h_i32 + 5, overflow_p(), sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(h_i32 + 6, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(h_plan, drs_plan.p, sizeof(DevPlan), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -2017,7 +2001,7 @@ struct sph_handle {
                          skin_fraction() > 0 ? dskin.as<DevSkin>() : nullptr, s);
     RC(copy_table(drs_save.p, cols.p));
     RC(step_body_dev());
-    launch_inst_end(b, drs_err.as<int>(), overflow.as<int32_t>(), status.as<int>(), s);
+    launch_inst_end(b, drs_err.as<int>(), overflow_p(), status.as<int>(), s);
     return SPH_OK;
   }
   // host view of the clock before a device loop
@@ -2668,6 +2652,7 @@ struct sph_handle {
     for (auto e : ev_pool) cudaEventDestroy(e);
     drop_graph();
     if (h_plan) cudaFreeHost(h_plan);
+    if (h_skin) cudaFreeHost(h_skin);
     if (h_red) cudaFreeHost(h_red);
     if (h_ctrl) cudaFreeHost(h_ctrl);
     if (h_i32) cudaFreeHost(h_i32);
@@ -3041,6 +3026,7 @@ int sph_create(const double* state49, const double* store, int64_t n_rows, int k
   if (cudaMallocHost(&h->h_red, sizeof(unsigned long long) * (RED_TOTAL + 2)) != cudaSuccess ||
       cudaMallocHost(&h->h_ctrl, sizeof(double) * 16) != cudaSuccess ||
       cudaMallocHost(&h->h_plan, sizeof(DevPlan)) != cudaSuccess ||
+      cudaMallocHost(&h->h_skin, sizeof(SkinOut)) != cudaSuccess ||
       cudaMallocHost(&h->h_i32, sizeof(int32_t) * 16) != cudaSuccess) {
     cudaGetLastError();
     h->destroy();

@@ -6,6 +6,8 @@
 // predictor/corrector (main.f90:323-362), timestep reductions
 // (timestep.f90:40-166), EOS (eos.f90:21-45) and the STS stage update
 // (sts_integrator.f90:87-124).
+#include <algorithm>
+#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -107,9 +109,7 @@ __global__ void k_reorder(const double* __restrict__ cin, double* __restrict__ c
 }
 
 // ---- periodic wrap of real particles (BC.f90:102-194) ----------------------------
-__global__ void k_reflect(double* __restrict__ cols, int64_t ld, int64_t nreal, BoxGeom g) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i >= nreal) return;
+__device__ __forceinline__ void reflect_row(double* cols, int64_t ld, int64_t i, const BoxGeom& g) {
   double r[3], dxmin[3], dxmax[3];
   for (int k = 0; k < 3; ++k) {
     r[k] = cols[(es_rx + k) * ld + i];
@@ -123,6 +123,10 @@ __global__ void k_reflect(double* __restrict__ cols, int64_t ld, int64_t nreal, 
     if (dxmin[k] > 0) v = __dadd_rn(g.emax[k], -dxmin[k]);
     cols[(es_rx + k) * ld + i] = v;
   }
+}
+__global__ void k_reflect(double* __restrict__ cols, int64_t ld, int64_t nreal, BoxGeom g) {
+  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (i < nreal) reflect_row(cols, ld, i, g);
 }
 
 // ---- periodic images --------------------------------------------------------------
@@ -1019,21 +1023,9 @@ __global__ void k_skin_sig(const double* __restrict__ cols, int64_t ld, int64_t 
   sig[i] = ghost_source(cols[es_type * ld + i]) ? image_sig(r, g, dim) : uint8_t(0);
 }
 
-__global__ void __launch_bounds__(TPB)
-k_skin_refresh(const int32_t* __restrict__ sidx, int64_t n, int64_t nrows, int64_t nreal,
-               const double* __restrict__ cols, int64_t ld, const int32_t* __restrict__ gsrc,
-               const int8_t* __restrict__ gcode, BoxGeom g, int dim,
-               const uint8_t* __restrict__ sig_b, const double* __restrict__ bx,
-               const double* __restrict__ by, const double* __restrict__ bz,
-               double* __restrict__ sx, double* __restrict__ sy, double* __restrict__ sz,
-               float4* __restrict__ s32, PackGeom pg, float* __restrict__ dsp, float tau,
-               float eps, double* __restrict__ hrec, unsigned long long* __restrict__ red,
-               const DevPlan* __restrict__ plan, const DevSkin* __restrict__ gate) {
-  if (gate && !gate->live) return;
-  if (plan) {
-    n = plan->nall;
-    pg = plan->pg;
-  }
+// (The arrays that one launch both writes and reads are plain pointers: no
+// loads through the read-only path.)
+__device__ __forceinline__ void skin_refresh(const SkinRefresh& a, int64_t n, const PackGeom& pg) {
   // slots: lo x, y, z (min), hi x, y, z (max), D (max), h of the real rows (max)
   double v[8] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300, 0.0, 0.0};
   const bool is_max[8] = {false, false, false, true, true, true, true, true};
@@ -1041,37 +1033,37 @@ k_skin_refresh(const int32_t* __restrict__ sidx, int64_t n, int64_t nrows, int64
   bool sigchg = false;
   for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < n;
        k += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t u = sidx[k];
+    const int64_t u = a.sidx[k];
     double x, y, z;
-    if (u < nrows) {
-      x = cols[es_rx * ld + u]; y = cols[es_ry * ld + u]; z = cols[es_rz * ld + u];
-      const double h = cols[es_h * ld + u];
-      hrec[k] = h;  // (for the centres' ways, read in record order)
-      if (u < nreal) v[7] = fmax(v[7], h);
-      if (ghost_source(cols[es_type * ld + u])) {
+    if (u < a.nrows) {
+      x = a.cols[es_rx * a.ld + u]; y = a.cols[es_ry * a.ld + u]; z = a.cols[es_rz * a.ld + u];
+      const double h = a.cols[es_h * a.ld + u];
+      a.hrec[k] = h;  // (for the centres' ways, read in record order)
+      if (u < a.nreal) v[7] = fmax(v[7], h);
+      if (ghost_source(a.cols[es_type * a.ld + u])) {
         const double r[3] = {x, y, z};
-        sigchg |= image_sig(r, g, dim) != sig_b[u];
+        sigchg |= image_sig(r, a.g, a.dim) != a.sig_b[u];
       }
     } else {
-      const int64_t q = u - nrows;
-      const int64_t src = gsrc[q];
-      const int code = gcode[q];
-      x = image_coord(cols[es_rx * ld + src], code % 3 - 1, g.emin[0], g.emax[0]);
-      y = image_coord(cols[es_ry * ld + src], (code / 3) % 3 - 1, g.emin[1], g.emax[1]);
-      z = image_coord(cols[es_rz * ld + src], code / 9 - 1, g.emin[2], g.emax[2]);
+      const int64_t q = u - a.nrows;
+      const int64_t src = a.gsrc[q];
+      const int code = a.gcode[q];
+      x = image_coord(a.cols[es_rx * a.ld + src], code % 3 - 1, a.g.emin[0], a.g.emax[0]);
+      y = image_coord(a.cols[es_ry * a.ld + src], (code / 3) % 3 - 1, a.g.emin[1], a.g.emax[1]);
+      z = image_coord(a.cols[es_rz * a.ld + src], code / 9 - 1, a.g.emin[2], a.g.emax[2]);
     }
-    sx[k] = x; sy[k] = y; sz[k] = z;
-    s32[k] = make_float4(__double2float_rn((x - pg.ox) + pg.shift),
+    a.sx[k] = x; a.sy[k] = y; a.sz[k] = z;
+    a.s32[k] = make_float4(__double2float_rn((x - pg.ox) + pg.shift),
                          __double2float_rn((y - pg.oy) + pg.shift),
                          __double2float_rn((z - pg.oz) + pg.shift), __int_as_float(int32_t(k)));
-    const double ex = x - bx[k], ey = y - by[k], ez = z - bz[k];
+    const double ex = x - a.bx[k], ey = y - a.by[k], ez = z - a.bz[k];
     // a few ulp of rounding in the differences, squares, sum and root: the
     // factor and the floor make the stored value an upper bound
     const double d = sqrt(ex * ex + ey * ey + ez * ez) * (1.0 + 1e-12) + 1e-300;
-    const float df = fmaxf(dsp[k], __double2float_ru(d));  // running maximum since b
-    dsp[k] = df;
-    nfast += df > tau ? 1u : 0u;
-    nmove += df > eps ? 1u : 0u;
+    const float df = fmaxf(a.dsp[k], __double2float_ru(d));  // running maximum since b
+    a.dsp[k] = df;
+    nfast += df > a.tau ? 1u : 0u;
+    nmove += df > a.eps ? 1u : 0u;
     v[6] = fmax(v[6], double(df));
     v[0] = fmin(v[0], x); v[1] = fmin(v[1], y); v[2] = fmin(v[2], z);
     v[3] = fmax(v[3], x); v[4] = fmax(v[4], y); v[5] = fmax(v[5], z);
@@ -1080,19 +1072,29 @@ k_skin_refresh(const int32_t* __restrict__ sidx, int64_t n, int64_t nrows, int64
   const unsigned wm = __reduce_add_sync(0xffffffffu, nmove);
   const unsigned ws = __ballot_sync(0xffffffffu, sigchg);
   if ((threadIdx.x & 31) == 0) {
-    if (wf) atomicAdd(&red[RED_SKIN_NFAST], (unsigned long long)wf);
-    if (wm) atomicAdd(&red[RED_SKIN_NMOVE], (unsigned long long)wm);
-    if (ws) atomicMax(&red[RED_SKIN_SIG], 1ull);
+    if (wf) atomicAdd(&a.red[RED_SKIN_NFAST], (unsigned long long)wf);
+    if (wm) atomicAdd(&a.red[RED_SKIN_NMOVE], (unsigned long long)wm);
+    if (ws) atomicMax(&a.red[RED_SKIN_SIG], 1ull);
   }
   block_minmax<8>(v, is_max);
   if (threadIdx.x == 0) {
     for (int k = 0; k < 3; ++k) {
-      if (v[k] < 1e300) red_min(&red[RED_LO_X + k], v[k]);
-      if (v[3 + k] > -1e300) red_max(&red[RED_HI_X + k], v[3 + k]);
+      if (v[k] < 1e300) red_min(&a.red[RED_LO_X + k], v[k]);
+      if (v[3 + k] > -1e300) red_max(&a.red[RED_HI_X + k], v[3 + k]);
     }
-    red_max(&red[RED_SKIN_D], v[6]);
-    red_max(&red[RED_SKIN_HMAX], v[7]);
+    red_max(&a.red[RED_SKIN_D], v[6]);
+    red_max(&a.red[RED_SKIN_HMAX], v[7]);
   }
+}
+__global__ void __launch_bounds__(TPB)
+k_skin_refresh(SkinRefresh a, int64_t n, PackGeom pg, const DevPlan* __restrict__ plan,
+               const DevSkin* __restrict__ gate) {
+  if (gate && !gate->live) return;
+  if (plan) {
+    n = plan->nall;
+    pg = plan->pg;
+  }
+  skin_refresh(a, n, pg);
 }
 
 // clamped cell coordinate of an FP64 cell-unit value (NaN -> 0)
@@ -1103,116 +1105,235 @@ __device__ __forceinline__ int clamp_cell(double f, int n) {
   return int(f);
 }
 
+// ---- one launch for an iterate served from skin lists --------------------------------------
+// The periodic wrap, the records' refresh, the checks that the lists may
+// serve, the marks of moving records, every centre's way and the two lists
+// of centres that act on theirs, as the phases of one cooperative launch
+// (grid barriers in between) with one result for the host.  As 20 launches
+// and clears, with a scan, these took 45 us of the 225 us of a step of 1,024
+// particles, whose data passes in 5.  NA_SERVE
+//
 // Marks at the level of cells: a record that moved more than eps flags the
 // cell it was sorted into (its position at b), one that moved more than tau
 // the cell of its position now (clamped to the grid); each flag field is
-// then dilated by a box of w cells per side (k_dilate, one axis per pass),
+// then dilated by a box of w cells per side, one axis per pass,
 // w = ceil(reach / L) + 1, which holds every cell within `reach` of any
-// point of the flagged cell.  A centre is near a fast (moving) record when
-// the cell it was sorted into carries the dilated flag.
-__global__ void k_skin_cells(int64_t n, const float* __restrict__ dsp, float tau, float eps,
-                             const uint32_t* __restrict__ keys, const double* __restrict__ sx,
-                             const double* __restrict__ sy, const double* __restrict__ sz,
-                             Grid g, uint8_t* __restrict__ fast_cell,
-                             uint8_t* __restrict__ move_cell) {
-  const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (k >= n) return;
-  const float d = dsp[k];
-  if (move_cell && d > eps) move_cell[keys[k]] = 1;
-  if (d > tau) {
-    const int cx = clamp_cell((sx[k] - g.ox) * g.invL, g.nx);
-    const int cy = clamp_cell((sy[k] - g.oy) * g.invL, g.ny);
-    const int cz = clamp_cell((sz[k] - g.oz) * g.invL, g.nz);
-    fast_cell[cx + int64_t(g.nx) * (cy + int64_t(g.ny) * cz)] = 1;
+// point of the flagged cell.  A pass writes into the field of the pass
+// before last, whose marks its own result contains, so the two fields are
+// cleared once; every marked cell writes its window, so the work follows the
+// marks (a few per cent of the cells while the lists serve), not the grid.
+// A centre is near a fast (moving) record when the cell it was sorted into
+// carries the dilated flag.
+__device__ __forceinline__ void dilate_axis(const uint8_t* in, uint8_t* out, const Grid& g, int axis,
+                                            int w) {
+  const int64_t ncell = int64_t(g.nx) * g.ny * g.nz;
+  for (int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; c < ncell;
+       c += int64_t(gridDim.x) * blockDim.x) {
+    if (!in[c]) continue;
+    int n, i;
+    int64_t stride;
+    if (axis == 0) { n = g.nx; i = int(c % g.nx); stride = 1; }
+    else if (axis == 1) { n = g.ny; i = int((c / g.nx) % g.ny); stride = g.nx; }
+    else { n = g.nz; i = int(c / (int64_t(g.nx) * g.ny)); stride = int64_t(g.nx) * g.ny; }
+    const int lo = max(0, i - w), hi = min(n - 1, i + w);
+    for (int j = lo; j <= hi; ++j) out[c + int64_t(j - i) * stride] = 1;
   }
 }
-// out[c] = OR of in over the cells within w of c along `axis` (out zeroed
-// before): every marked cell writes its window, so the work follows the
-// marks (a few per cent of the cells while the lists serve), not the grid
-__global__ void k_dilate(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, Grid g,
-                         int axis, const int* __restrict__ wp) {
-  const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int64_t ncell = int64_t(g.nx) * g.ny * g.nz;
-  if (c >= ncell || !in[c]) return;
-  const int w = *wp;
-  int n, i;
-  int64_t stride;
-  if (axis == 0) { n = g.nx; i = int(c % g.nx); stride = 1; }
-  else if (axis == 1) { n = g.ny; i = int((c / g.nx) % g.ny); stride = g.nx; }
-  else { n = g.nz; i = int(c / (int64_t(g.nx) * g.ny)); stride = int64_t(g.nx) * g.ny; }
-  const int a = max(0, i - w), b = min(n - 1, i + w);
-  for (int j = a; j <= b; ++j) out[c + int64_t(j - i) * stride] = 1;
+
+// The checks of a served iterate on the refreshed records (SkinOut::why) and
+// the windows wf, wm of the marks in cells.
+__device__ __forceinline__ int skin_gate(const unsigned long long* red, const SkinServe& a, int& wf,
+                                         int& wm) {
+  const double D = dkey_inv(__ldcg(red + RED_SKIN_D));
+  const double hmax = dkey_inv(__ldcg(red + RED_SKIN_HMAX));
+  const double hmaxb = dkey_inv(__ldcg(red + RED_SKIN_HMAXB));
+  wf = wm = 0;
+  if (__ldcg(red + RED_SKIN_SIG)) return 1;
+  if (!(D <= a.dcap)) return 2;
+  if (!(hmax > 0) || !isfinite(hmax) || !(hmaxb > 0)) return 3;
+  // every record inside the FP32 packing's binade: 0 <= x - origin < shift
+  const double o[3] = {a.pg.ox, a.pg.oy, a.pg.oz};
+  for (int k = 0; k < 3; ++k) {
+    const double lo = dkey_inv(__ldcg(red + RED_LO_X + k)), hi = dkey_inv(__ldcg(red + RED_HI_X + k));
+    if (!(lo >= o[k]) || !(hi - o[k] < a.pg.shift * (1.0 - 1e-9))) return 4;
+  }
+  // around fast records every centre that may see them now (reach_f),
+  // around moving ones every skin list holding them (reach_m)
+  const double reach_f = (a.krad * hmax + double(a.r.tau)) * (1.0 + 1e-9);
+  const double reach_m = a.kfac * a.krad * hmaxb * (1.0 + 1e-9);
+  const double ef = ceil(reach_f * a.grid.invL) + 1.0, em = ceil(reach_m * a.grid.invL) + 1.0;
+  if (!(ef <= 256.0) || !(em <= 256.0)) return 5;
+  wf = int(ef);
+  wm = int(em);
+  return 0;
 }
 
-// The way of each centre (mode: 0 filter, 1 fresh search, 2 keep; dflag =
-// 1 for the fresh search).  The margins of 1e-12 (relative) lie far above
-// the FP64 rounding of the predicate and of the displacements, so that no
-// record outside a list can pass the FP64 predicate at t; near_f / near_m
-// are the dilated cell flags (near_m == NULL: no centre keeps its row).
-__global__ void k_skin_classify(int64_t nc, const int32_t* __restrict__ centre_k,
-                                const double* __restrict__ hrec, const double* __restrict__ hb,
-                                double* __restrict__ href, double* __restrict__ hdev,
-                                float* __restrict__ gap,
-                                double krad, double kfac, float tau, float eps,
-                                const float* __restrict__ dsp,
-                                const uint32_t* __restrict__ keys,
-                                const uint8_t* __restrict__ near_f,
-                                const uint8_t* __restrict__ near_m,
-                                uint8_t* __restrict__ mode, int64_t* __restrict__ ways,
-                                const int32_t* __restrict__ ncnt,
-                                unsigned long long* __restrict__ nkept) {
-  const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  uint8_t w = 1;
-  if (c < nc) {
-    const bool was_searched = mode[c] == 1;  // (a centre once searched afresh stays so)
-    const int32_t k = centre_k[c];
-    const double h = hrec[k], h0 = hb[c];
-    const double hd = fmax(hdev[c], fabs(h - href[c]));
-    const double di = double(dsp[k]);
-    const double lhs = krad * h * (1.0 + 1e-12) + di + double(tau);
-    const double rhs = krad * h0 * kfac * (1.0 - 1e-12);
-    const uint32_t cell = keys[k];  // the cell the centre was sorted into
-    const bool clean = !was_searched && !near_f[cell] && dsp[k] <= tau && lhs < rhs;
-    if (clean) {
-      const bool quiet = near_m && !near_m[cell] && dsp[k] <= eps;
-      const bool keep = quiet && 4.0 * double(eps) + krad * hd * (1.0 + 1e-12) +
-                                         1e-12 * krad * h0 <
-                                     double(gap[c]);
-      w = keep ? 2 : 0;
-      if (keep) {
-        hdev[c] = hd;
-      } else {  // the filter writes the row at this h, and the new gap if quiet
-        href[c] = h;
-        hdev[c] = 0.0;
-        gap[c] = quiet ? 0.f : -1.f;
+// The way of centre c (0 filter, 1 fresh search, 2 keep).  The margins of
+// 1e-12 (relative) lie far above the FP64 rounding of the predicate and of
+// the displacements, so that no record outside a list can pass the FP64
+// predicate at t; near_f / near_m are the dilated cell flags.
+__device__ __forceinline__ uint8_t skin_way(const SkinServe& a, int64_t c, const uint8_t* near_f,
+                                            const uint8_t* near_m) {
+  if (a.mode[c] == 1) return 1;  // (a centre once searched afresh stays so)
+  const int32_t k = a.centre_k[c];
+  const float dk = a.r.dsp[k], tau = a.r.tau, eps = a.r.eps;
+  const double h = a.r.hrec[k], h0 = a.hb[c];
+  const double lhs = a.krad * h * (1.0 + 1e-12) + double(dk) + double(tau);
+  const double rhs = a.krad * h0 * a.kfac * (1.0 - 1e-12);
+  const uint32_t cell = a.keys[k];  // the cell the centre was sorted into
+  if (near_f[cell] || !(dk <= tau) || !(lhs < rhs)) return 1;
+  const double hd = fmax(a.hdev[c], fabs(h - a.href[c]));
+  const bool quiet = !near_m[cell] && dk <= eps;
+  if (quiet && 4.0 * double(eps) + a.krad * hd * (1.0 + 1e-12) + 1e-12 * a.krad * h0 <
+                   double(a.gap[c])) {
+    a.hdev[c] = hd;
+    return 2;
+  }
+  // the filter writes the row at this h, and the new gap if quiet
+  a.href[c] = h;
+  a.hdev[c] = 0.0;
+  a.gap[c] = quiet ? 0.f : -1.f;
+  return 0;
+}
+
+__global__ void __launch_bounds__(TPB) k_skin_serve(SkinServe a) {
+  auto grid = cooperative_groups::this_grid();
+  const int64_t first = blockIdx.x * int64_t(TPB) + threadIdx.x, step = int64_t(gridDim.x) * TPB;
+  unsigned long long* const red = a.r.red;
+  const int64_t ncell = int64_t(a.grid.nx) * a.grid.ny * a.grid.nz;
+  // the wrap; clears
+  if (a.wrap)
+    for (int64_t i = first; i < a.r.nreal; i += step) reflect_row(a.r.cols, a.r.ld, i, a.r.g);
+  for (int64_t i = first; i < ncell; i += step)
+    a.fcell[0][i] = a.fcell[1][i] = a.mcell[0][i] = a.mcell[1][i] = 0;
+  if (first == 0) {
+    for (int k = 0; k < 3; ++k) {
+      red[RED_LO_X + k] = dkey(1e308);
+      red[RED_HI_X + k] = dkey(-1e308);
+    }
+    red[RED_SKIN_D] = red[RED_SKIN_HMAX] = dkey(0.0);
+    red[RED_SKIN_SIG] = red[RED_SKIN_NFAST] = red[RED_SKIN_NMOVE] = 0ull;
+    red[RED_SKIN_NKEPT] = red[RED_SKIN_NKEPT_PAIRS] = 0ull;
+    a.flags[0] = a.flags[1] = 0;
+  }
+  grid.sync();
+  skin_refresh(a.r, a.nall, a.pg);
+  grid.sync();
+  __shared__ int s_gate[3];
+  if (threadIdx.x == 0) s_gate[0] = skin_gate(red, a, s_gate[1], s_gate[2]);
+  __syncthreads();
+  const int why = s_gate[0], wf = s_gate[1], wm = s_gate[2];
+  if (why) {  // (the same on every block)
+    if (first == 0) {
+      SkinOut o{};
+      o.why = why;
+      o.D = dkey_inv(__ldcg(red + RED_SKIN_D));
+      o.nfast = (long long)__ldcg(red + RED_SKIN_NFAST);
+      o.nmove = (long long)__ldcg(red + RED_SKIN_NMOVE);
+      *a.out = o;
+    }
+    return;
+  }
+  const bool fast = __ldcg(red + RED_SKIN_NFAST) != 0, move = __ldcg(red + RED_SKIN_NMOVE) != 0;
+  int at = 0;  // the field that holds the marks
+  if (move) {  // (tau > eps: a fast record moves)
+    for (int64_t k = first; k < a.nall; k += step) {
+      const float d = a.r.dsp[k];
+      if (d > a.r.eps) a.mcell[0][a.keys[k]] = 1;
+      if (d > a.r.tau) {
+        const int cx = clamp_cell((a.r.sx[k] - a.grid.ox) * a.grid.invL, a.grid.nx);
+        const int cy = clamp_cell((a.r.sy[k] - a.grid.oy) * a.grid.invL, a.grid.ny);
+        const int cz = clamp_cell((a.r.sz[k] - a.grid.oz) * a.grid.invL, a.grid.nz);
+        a.fcell[0][cx + int64_t(a.grid.nx) * (cy + int64_t(a.grid.ny) * cz)] = 1;
       }
     }
-    mode[c] = w;
-    // one scan counts both lists: fresh searches in the low word, filters
-    // in the high one
-    ways[c] = (w == 1 ? 1ll : 0ll) | (w == 0 ? (1ll << 32) : 0ll);
+    grid.sync();
+    for (int axis = 0; axis < a.r.dim; ++axis) {
+      dilate_axis(a.mcell[at], a.mcell[1 - at], a.grid, axis, wm);
+      if (fast) dilate_axis(a.fcell[at], a.fcell[1 - at], a.grid, axis, wf);
+      at = 1 - at;
+      grid.sync();
+    }
   }
-  // rows kept and their neighbours: nkept[0], nkept[1]
-  const bool kp = c < nc && w == 2;
-  unsigned long long v[2] = {kp ? 1ull : 0ull, kp ? (unsigned long long)ncnt[c] : 0ull};
-  const bool is_max[2] = {false, false};
-  block_counters<2>(v, is_max);
-  if (threadIdx.x == 0 && v[0]) {
-    atomicAdd(nkept, v[0]);
-    atomicAdd(nkept + 1, v[1]);
+  // every centre's way; a block's centres are consecutive, so that its lists
+  // follow those of the blocks before it
+  const int64_t chunk = ((a.nc + gridDim.x - 1) / gridDim.x + TPB - 1) / TPB * TPB;
+  const int64_t c0 = min(a.nc, blockIdx.x * chunk), c1 = min(a.nc, c0 + chunk);
+  unsigned long long v[4] = {0, 0, 0, 0};  // searched afresh, filtered, kept, their pairs
+  for (int64_t c = c0 + threadIdx.x; c < c1; c += TPB) {
+    const uint8_t w = skin_way(a, c, a.fcell[at], a.mcell[at]);
+    a.mode[c] = w;
+    if (w == 1) ++v[0];
+    else if (w == 0) ++v[1];
+    else { ++v[2]; v[3] += (unsigned long long)a.ncnt[c]; }
   }
-}
-
-// the lists of the centres searched afresh and of those that filter, in
-// centre order, from the scan of k_skin_classify's ways
-__global__ void k_skin_lists(int64_t nc, const int64_t* __restrict__ ways,
-                             const int64_t* __restrict__ pos, int32_t* __restrict__ dlist,
-                             int32_t* __restrict__ flist) {
-  const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (c >= nc) return;
-  const int64_t w = ways[c], p = pos[c];
-  if (w & 1) dlist[p & 0xffffffffll] = int32_t(c);
-  if (w >> 32) flist[p >> 32] = int32_t(c);
+  const bool is_max[4] = {false, false, false, false};
+  block_counters<4>(v, is_max);
+  if (threadIdx.x == 0) {
+    a.block_counts[blockIdx.x] = make_int2(int(v[0]), int(v[1]));
+    if (v[2]) {
+      atomicAdd(red + RED_SKIN_NKEPT, v[2]);
+      atomicAdd(red + RED_SKIN_NKEPT_PAIRS, v[3]);
+    }
+  }
+  grid.sync();
+  // this block's places in the lists
+  __shared__ int s_base[2];
+  {
+    unsigned long long before[2] = {0, 0};
+    for (int b = threadIdx.x; b < int(blockIdx.x); b += TPB) {
+      const int2 n = __ldcg(a.block_counts + b);
+      before[0] += n.x;
+      before[1] += n.y;
+    }
+    const bool mx[2] = {false, false};
+    block_counters<2>(before, mx);
+    if (threadIdx.x == 0) {
+      s_base[0] = int(before[0]);
+      s_base[1] = int(before[1]);
+    }
+    __syncthreads();
+  }
+  __shared__ int s_warp[TPB / 32][2];
+  int base0 = s_base[0], base1 = s_base[1];
+  const int wl = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const unsigned below = (1u << wl) - 1u;
+  for (int64_t t = c0; t < c1; t += TPB) {
+    const int64_t c = t + threadIdx.x;
+    const int w = c < c1 ? a.mode[c] : 2;
+    const unsigned m1 = __ballot_sync(0xffffffffu, w == 1), m0 = __ballot_sync(0xffffffffu, w == 0);
+    if (wl == 0) {
+      s_warp[wi][0] = __popc(m1);
+      s_warp[wi][1] = __popc(m0);
+    }
+    __syncthreads();
+    int p1 = base0 + __popc(m1 & below), p0 = base1 + __popc(m0 & below);
+    for (int i = 0; i < TPB / 32; ++i) {
+      if (i < wi) { p1 += s_warp[i][0]; p0 += s_warp[i][1]; }
+      base0 += s_warp[i][0];
+      base1 += s_warp[i][1];
+    }
+    if (w == 1) a.dlist[p1] = int32_t(c);
+    if (w == 0) a.flist[p0] = int32_t(c);
+    __syncthreads();
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    SkinOut o{};
+    o.D = dkey_inv(__ldcg(red + RED_SKIN_D));
+    o.nfast = (long long)__ldcg(red + RED_SKIN_NFAST);
+    o.nmove = (long long)__ldcg(red + RED_SKIN_NMOVE);
+    o.nkept = (long long)__ldcg(red + RED_SKIN_NKEPT);
+    o.kept_pairs = (long long)__ldcg(red + RED_SKIN_NKEPT_PAIRS);
+    o.ndirty = base0;
+    // the fresh searches cost several times a search's share per centre,
+    // their cells widened by D: past dirty_share of the centres a plain
+    // search of everything is cheaper
+    double widen = 1.0;
+    for (int d = 0; d < a.r.dim; ++d) widen *= (a.dcap + o.D) / a.dcap;
+    if (double(o.ndirty) * widen > a.dirty_share * double(a.nc)) o.why = 6;
+    o.nfilter = o.why ? 0 : base1;
+    *a.out = o;
+  }
 }
 
 __global__ void k_skin_compact(int64_t nc, const int32_t* __restrict__ dflag,
@@ -1254,6 +1375,7 @@ template <int G>
 __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
   constexpr unsigned FULL = 0xffffffffu;
   if (a.plan) a.shift = a.plan->pg.shift;
+  if (a.nc_dev) a.nc = *a.nc_dev;
   constexpr int V = 4;
   constexpr int PER = G * V;
   constexpr int CPB = 128 / G;  // centres per block and pass
@@ -2360,18 +2482,29 @@ void launch_skin_sig(const double* cols, int64_t nrows, BoxGeom g, int dim, uint
   k_skin_sig<<<nblocks(nrows), TPB, 0, s>>>(cols, nrows, nrows, g, dim, sig);
   note_launch();
 }
-void launch_skin_refresh(const int32_t* sidx, int64_t n, int64_t nrows, int64_t nreal,
-                         const double* cols, const int32_t* gsrc, const int8_t* gcode,
-                         BoxGeom g, int dim, const uint8_t* sig_b, const double* bx,
-                         const double* by, const double* bz, double* sx, double* sy, double* sz,
-                         float4* s32, PackGeom pg, float* dsp, float tau, float eps,
-                         double* hrec, unsigned long long* red, cudaStream_t s,
-                         const DevPlan* plan, const DevSkin* gate) {
+void launch_skin_refresh(const SkinRefresh& r, int64_t n, cudaStream_t s, const DevPlan* plan,
+                         const DevSkin* gate) {
   if (n <= 0) return;
-  k_skin_refresh<<<reduce_blocks(n), TPB, 0, s>>>(sidx, n, nrows, nreal, cols, nrows, gsrc, gcode,
-                                                  g, dim, sig_b, bx, by, bz, sx, sy, sz, s32, pg,
-                                                  dsp, tau, eps, hrec, red, plan, gate);
+  k_skin_refresh<<<reduce_blocks(n), TPB, 0, s>>>(r, n, PackGeom{}, plan, gate);
   note_launch();
+}
+int skin_serve_most_blocks() {
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_skin_serve, TPB, 0) != cudaSuccess)
+    return 0;
+  return sms * per_sm;
+}
+int skin_serve_blocks(int64_t n, int most) {
+  return int(std::min<int64_t>(most, std::max<int64_t>(1, (n + TPB - 1) / TPB)));
+}
+cudaError_t launch_skin_serve(const SkinServe& a, int blocks, cudaStream_t s) {
+  SkinServe arg = a;
+  void* args[] = {&arg};
+  note_launch();
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_skin_serve), dim3(blocks),
+                                     dim3(TPB), args, 0, s);
 }
 
 // ---- skin lists of the device-resident step ---------------------------------------------
@@ -2461,84 +2594,6 @@ void launch_dskin_decide(DevSkin* ds, const unsigned long long* red, const DevPl
 void launch_dskin_built(DevSkin* ds, const unsigned long long* red, cudaStream_t s) {
   k_dskin_built<<<1, 32, 0, s>>>(ds, red);
   note_launch();
-}
-void launch_skin_marks(int64_t n, const float* dsp, float tau, float eps, const uint32_t* keys,
-                       const double* sx, const double* sy, const double* sz, Grid g, int dim,
-                       const int* w, uint8_t* fast_cell, uint8_t* move_cell, uint8_t* tmp,
-                       cudaStream_t s) {
-  const int64_t ncell = int64_t(g.nx) * g.ny * g.nz;
-  if (n <= 0 || ncell <= 0) return;
-  cudaMemsetAsync(fast_cell, 0, size_t(ncell), s);
-  if (move_cell) cudaMemsetAsync(move_cell, 0, size_t(ncell), s);
-  k_skin_cells<<<nblocks(n), TPB, 0, s>>>(n, dsp, tau, eps, keys, sx, sy, sz, g, fast_cell,
-                                          move_cell);
-  note_launch();
-  // dilate in place through tmp: axis 0 into tmp, 1 back, 2 into tmp, copy back
-  auto dilate = [&](uint8_t* f, const int* wp) {
-    uint8_t* a = f;
-    uint8_t* b = tmp;
-    for (int axis = 0; axis < dim; ++axis) {
-      cudaMemsetAsync(b, 0, size_t(ncell), s);
-      k_dilate<<<nblocks(ncell), TPB, 0, s>>>(a, b, g, axis, wp);
-      note_launch();
-      std::swap(a, b);
-    }
-    if (a != f) cudaMemcpyAsync(f, a, size_t(ncell), cudaMemcpyDeviceToDevice, s);
-  };
-  dilate(fast_cell, w);
-  if (move_cell) dilate(move_cell, w + 1);
-}
-__global__ void k_skin_gate(const unsigned long long* __restrict__ red, SkinGateIn in,
-                            int* __restrict__ gate) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  const double D = dkey_inv(red[RED_SKIN_D]);
-  const double hmax = dkey_inv(red[RED_SKIN_HMAX]);
-  const double hmaxb = dkey_inv(red[RED_SKIN_HMAXB]);
-  int why = 0;
-  if (red[RED_SKIN_SIG]) why = 1;
-  else if (!(D <= in.dcap)) why = 2;
-  else if (!(hmax > 0) || !isfinite(hmax) || !(hmaxb > 0)) why = 3;
-  if (!why) {
-    // every record inside the FP32 packing's binade: 0 <= x - origin < shift
-    const double o[3] = {in.pg.ox, in.pg.oy, in.pg.oz};
-    for (int k = 0; k < 3; ++k) {
-      const double lo = dkey_inv(red[RED_LO_X + k]), hi = dkey_inv(red[RED_HI_X + k]);
-      if (!(lo >= o[k]) || !(hi - o[k] < in.pg.shift * (1.0 - 1e-9))) why = 4;
-    }
-  }
-  int wf = 0, wm = 0;
-  if (!why) {
-    // around fast records every centre that may see them now (reach_f),
-    // around moving ones every skin list holding them (reach_m)
-    const double reach_f = (in.krad * hmax + in.tau) * (1.0 + 1e-9);
-    const double reach_m = in.kfac * in.krad * hmaxb * (1.0 + 1e-9);
-    const double ef = ceil(reach_f * in.invL) + 1.0, em = ceil(reach_m * in.invL) + 1.0;
-    if (!(ef <= 256.0) || !(em <= 256.0)) why = 5;
-    else { wf = int(ef); wm = int(em); }
-  }
-  gate[0] = why;
-  gate[1] = wf;
-  gate[2] = wm;
-}
-void launch_skin_gate(const unsigned long long* red, SkinGateIn in, int* gate, cudaStream_t s) {
-  k_skin_gate<<<1, 32, 0, s>>>(red, in, gate);
-  note_launch();
-}
-void launch_skin_classify(int64_t nc, const int32_t* centre_k, const double* hrec,
-                          const double* hb, double* href, double* hdev, float* gap, double krad,
-                          double kfac, float tau, float eps, const float* dsp,
-                          const uint32_t* keys, const uint8_t* near_f, const uint8_t* near_m,
-                          uint8_t* mode, int64_t* ways, int64_t* pos, int32_t* dlist,
-                          int32_t* flist, void* scan_tmp, size_t scan_bytes,
-                          const int32_t* ncnt, unsigned long long* nkept, cudaStream_t s) {
-  if (nc <= 0) return;
-  k_skin_classify<<<nblocks(nc), TPB, 0, s>>>(nc, centre_k, hrec, hb, href, hdev, gap, krad, kfac, tau,
-                                              eps, dsp, keys, near_f, near_m, mode, ways, ncnt,
-                                              nkept);
-  cudaMemsetAsync(ways + nc, 0, sizeof(int64_t), s);
-  exclusive_scan64(scan_tmp, scan_bytes, ways, pos, nc + 1, s);
-  k_skin_lists<<<nblocks(nc), TPB, 0, s>>>(nc, ways, pos, dlist, flist);
-  note_launch(2);
 }
 void launch_inverse(const int32_t* p, int64_t n, int32_t* q, cudaStream_t s) {
   if (n <= 0) return;

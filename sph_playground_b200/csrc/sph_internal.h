@@ -309,15 +309,67 @@ void launch_skin_sig(const double* cols, int64_t nrows, BoxGeom g, int dim, uint
 // RED_LO_* / RED_HI_* (bounding box), RED_SKIN_D, RED_SKIN_HMAX (real
 // rows), RED_SKIN_SIG (a row whose image signature differs from sig_b),
 // RED_SKIN_NFAST (displacement > tau) and RED_SKIN_NMOVE (> eps)
-// (device-resident step: with plan set, n and pg come from the plan (n the
-// launch bound); with gate set, nothing is done unless gate->live)
-void launch_skin_refresh(const int32_t* sidx, int64_t n, int64_t nrows, int64_t nreal,
-                         const double* cols, const int32_t* gsrc, const int8_t* gcode,
-                         BoxGeom g, int dim, const uint8_t* sig_b, const double* bx,
-                         const double* by, const double* bz, double* sx, double* sy, double* sz,
-                         float4* s32, PackGeom pg, float* dsp, float tau, float eps,
-                         double* hrec, unsigned long long* red, cudaStream_t s,
-                         const DevPlan* plan = nullptr, const DevSkin* gate = nullptr);
+struct SkinRefresh {
+  const int32_t* sidx;
+  int64_t nrows, nreal;
+  double* cols;
+  int64_t ld;
+  const int32_t* gsrc;
+  const int8_t* gcode;
+  BoxGeom g;
+  int dim;
+  const uint8_t* sig_b;
+  const double *bx, *by, *bz;
+  double *sx, *sy, *sz;
+  float4* s32;
+  float* dsp;
+  float tau, eps;
+  double* hrec;
+  unsigned long long* red;
+};
+// (device-resident step: n the launch bound, the count and the packing frame
+// from the plan; with gate set, nothing is done unless gate->live)
+void launch_skin_refresh(const SkinRefresh& r, int64_t n, cudaStream_t s, const DevPlan* plan,
+                         const DevSkin* gate);
+// What an iterate served from skin lists tells the host: why the lists
+// cannot serve (0 they can, 1 an image set changed, 2 a record moved a search
+// radius, 3 h, 4 a record left the FP32 binade, 5 a window spans more than
+// 256 cells, 6 too many centres to search afresh), the centres searched
+// afresh and filtered, the rows kept and their neighbours, the largest
+// displacement and the records that moved more than tau and eps.
+struct SkinOut {
+  int why, ndirty, nfilter, pad;
+  long long nkept, kept_pairs, nfast, nmove;
+  double D;
+};
+struct SkinServe {
+  SkinRefresh r;
+  int wrap;        // the rows are wrapped into the periodic box first
+  int64_t nall;    // records
+  PackGeom pg;
+  Grid grid;       // cells of the lists' search, keys[k] each record's
+  const uint32_t* keys;
+  uint8_t *fcell[2], *mcell[2];  // two flag fields each (fast, moving)
+  int64_t nc;
+  const int32_t* centre_k;
+  // per centre: h at the lists' search, h when the row was last written, the
+  // running maximum of |h - href| since, the gap of the row, its way
+  const double* hb;
+  double *href, *hdev;
+  float* gap;
+  uint8_t* mode;
+  const int32_t* ncnt;
+  double krad, kfac, dcap, dirty_share;
+  int2* block_counts;     // skin_serve_blocks() entries
+  int32_t *dlist, *flist;  // the centres searched afresh / filtered, in order
+  int32_t* flags;          // longest row, overflow (cleared)
+  SkinOut* out;
+};
+// the blocks of k_skin_serve that the current device holds at once (0: an
+// error of the runtime), and those for n records
+int skin_serve_most_blocks();
+int skin_serve_blocks(int64_t n, int most);
+cudaError_t launch_skin_serve(const SkinServe& a, int blocks, cudaStream_t s);
 // with the lists live, per centre: can its row come from its skin list?
 // Every record now within krad h of the centre was within krad h + 2 D at
 // the lists' search (both moved at most D since), and the list holds all
@@ -333,39 +385,6 @@ void launch_dskin_decide(DevSkin* ds, const unsigned long long* red, const DevPl
                          cudaStream_t s);
 // after the search: its lists are live when it was a skin search
 void launch_dskin_built(DevSkin* ds, const unsigned long long* red, cudaStream_t s);
-// The checks of a skin-list iterate on the refreshed records, on the
-// device so that the iterate asks the host once: gate[0] = 0 when the
-// lists may serve, else why not (1 an image set changed, 2 a record moved
-// a search radius dcap, 3 h, 4 a record left the FP32 binade, 5 a window
-// spans more than 256 cells); gate[1], gate[2] = the windows wf, wm of the
-// marks in cells (0 when gate[0] != 0)
-struct SkinGateIn {
-  double dcap, krad, tau, kfac, invL;
-  PackGeom pg;
-};
-void launch_skin_gate(const unsigned long long* red, SkinGateIn in, int* gate, cudaStream_t s);
-// cell flags of the records that moved more than tau (fast_cell, by their
-// position now) and eps (move_cell, may be NULL; by the cell they were
-// sorted into), dilated by w[0] / w[1] cells per side along each of dim
-// axes (w in device memory; tmp: a spare field of the cell count)
-void launch_skin_marks(int64_t n, const float* dsp, float tau, float eps, const uint32_t* keys,
-                       const double* sx, const double* sy, const double* sz, Grid g, int dim,
-                       const int* w, uint8_t* fast_cell, uint8_t* move_cell, uint8_t* tmp,
-                       cudaStream_t s);
-// mode[c] = 0 (filter the skin list), 1 (search afresh) or 2 (keep the row)
-// for every centre (see sph_grid.cu), near_f / near_m the dilated cell
-// flags looked up by the cell keys[k] each centre's record was sorted into,
-// h of the centres from hrec (per record); href[c] = h when the row was last
-// written, hdev[c] = running maximum of |h - href[c]| since.  The centres searched afresh go to dlist, those that filter
-// to flist (in centre order); pos[nc] = their counts (low / high 32 bits);
-// ways and pos hold nc + 1 entries.  nkept[0..1] += rows kept, their pairs.
-void launch_skin_classify(int64_t nc, const int32_t* centre_k, const double* hrec,
-                          const double* hb, double* href, double* hdev, float* gap, double krad,
-                          double kfac, float tau, float eps, const float* dsp,
-                          const uint32_t* keys, const uint8_t* near_f, const uint8_t* near_m,
-                          uint8_t* mode, int64_t* ways, int64_t* pos, int32_t* dlist,
-                          int32_t* flist, void* scan_tmp, size_t scan_bytes,
-                          const int32_t* ncnt, unsigned long long* nkept, cudaStream_t s);
 // rows renamed under skin lists (old row perm[i] -> row i, inv[perm[i]] =
 // i): sidx / ssrc / gsrc / centre_p renamed through inv, the rows' image
 // signatures moved from sig_in to sig_out
@@ -431,6 +450,7 @@ void launch_gather_h(int64_t nc, const int32_t* centre_p, const double* hcol, do
 struct SkinFilterArgs {
   int64_t nc;           // centres (list == NULL) or list entries
   const int32_t* list;  // optional: the centres to filter
+  const int* nc_dev;    // if set: nc read from the device (nc is the most there can be)
   const uint8_t* mode;  // 0: filter; 1: left to the search; 2: kept when keep != 0
                         // (NULL with list NULL: every centre filters)
   int keep;
