@@ -13,6 +13,10 @@
 // The "ddw device function table" of kernel.f90:19-23 (procedure pointers
 // nw, fab, n2w, hessian) is the run-time switch on P.ddw below; the branch
 // is uniform across a launch, so it does not diverge.
+//
+// One instance per kind of run (C2Mode): an instance that served every set of
+// equations held the conductivity tensors, both fields and every sum at once
+// and spilled 350 bytes (2D FP64) to 680 (3D FP64) per thread.  NA_MODES
 #include "sph_internal.h"
 
 namespace sph {
@@ -24,6 +28,14 @@ inline int nblocks(int64_t n, int tpb = TPB) {
   int64_t b = (n + tpb - 1) / tpb;
   return int(b < 1 ? 1 : b);
 }
+
+enum C2Mode : int {
+  C2_HYDRO,    // hydrodynamics alone
+  C2_MHD,      // with the magnetic field
+  C2_HESSIAN,  // diffusion alone, by a Hessian method (fab, fw, n2w)
+  C2_TWO_NW,   // diffusion alone, by two first derivatives
+  C2_GENERAL   // every other set: flux-limited diffusion, diffusion with hydrodynamics or field
+};
 
 template <class R> struct Part {
   PairPos<R> pos;
@@ -45,10 +57,15 @@ template <> struct Loader<double> {
     o.invh = c.x; o.hrho = c.y; o.rho = 2.0 * c.y; o.Pi = d.x; o.P = d.y; o.ac = e.x; o.u = e.y;
     o.vx = f.x; o.vy = f.y; o.vz = g.x;
   }
+  // (what a mode does not use is not read)
+  template <int MODE>
   static __device__ __forceinline__ void extra(const PackBufs& pb, int64_t j, PartX<double>& o) {
-    double2 g = __ldg(&pb.p[6][j]), h = __ldg(&pb.p[7][j]), i = __ldg(&pb.p[8][j]),
-            k = __ldg(&pb.p[9][j]), l = __ldg(&pb.p[10][j]);
-    o.T = g.y; o.kappa = h.x; o.gx = h.y; o.gy = i.x; o.gz = i.y;
+    if constexpr (MODE != C2_MHD) o.T = __ldg(&pb.p[6][j]).y;
+    if constexpr (MODE == C2_TWO_NW || MODE == C2_GENERAL) {
+      const double2 h = __ldg(&pb.p[7][j]), i = __ldg(&pb.p[8][j]);
+      o.kappa = h.x; o.gx = h.y; o.gy = i.x; o.gz = i.y;
+    }
+    const double2 k = __ldg(&pb.p[9][j]), l = __ldg(&pb.p[10][j]);
     o.bx = k.x; o.by = k.y; o.bz = l.x;
   }
 };
@@ -61,6 +78,7 @@ template <> struct Loader<float> {
     o.hrho = c.x; o.rho = 2.f * c.x; o.Pi = c.y; o.P = c.z; o.ac = c.w;
     o.u = d.x; o.vx = d.y; o.vy = d.z; o.vz = d.w;
   }
+  template <int MODE>
   static __device__ __forceinline__ void extra(const PackBufs& pb, int64_t j, PartX<float>& o) {
     float4 e = __ldg(&pb.q[4][j]), f = __ldg(&pb.q[5][j]);
     o.T = e.x; o.kappa = e.y; o.gx = e.z; o.gy = e.w;
@@ -72,13 +90,45 @@ template <class R> __device__ __forceinline__ R my_sqrt(R x);
 template <> __device__ __forceinline__ double my_sqrt<double>(double x) { return sqrt(x); }
 template <> __device__ __forceinline__ float my_sqrt<float>(float x) { return sqrtf(x); }
 
-// diffusion tensor (3x3, symmetric) built from a unit vector (circuit2.f90:203-205,
-// 371-373: diagonal form; the full k_par b b^T when full_tensor is set)
+// Conductivity tensor of a particle (circuit2.f90:203-205, 371-373): isotropic
+// s I, the diagonal form diag(w) with w = k_par b_x^2, ..., or the full
+// k_par w w^T with w the unit vector; which of them is the run's (KKind).
+enum KKind : int { K_ISO, K_DIAG, K_FULL };
 template <class R>
-__device__ __forceinline__ void aniso_tensor(R difcond, const R* ub, int full, R K[3][3]) {
-  for (int a = 0; a < 3; ++a)
-    for (int b = 0; b < 3; ++b) K[a][b] = (a == b || full) ? difcond * ub[a] * ub[b] : R(0);
-}
+struct Tensor {
+  R s, w[3];
+  __device__ __forceinline__ void init() { s = R(0); w[0] = w[1] = w[2] = R(0); }
+  // from the unit vector of the field
+  __device__ __forceinline__ void aniso(int kind, R k_par, R x, R y, R z) {
+    s = k_par;
+    w[0] = kind == K_FULL ? x : k_par * x * x;
+    w[1] = kind == K_FULL ? y : k_par * y * y;
+    w[2] = kind == K_FULL ? z : k_par * z * z;
+  }
+  template <int DIM>
+  __device__ __forceinline__ R trace(int kind) const {
+    if (kind == K_ISO) return R(DIM) * s;
+    R t = R(0);
+    for (int x = 0; x < DIM; ++x) t += kind == K_FULL ? s * w[x] * w[x] : w[x];
+    return t;
+  }
+  // r . K r over the run's axes
+  template <int DIM>
+  __device__ __forceinline__ R form(int kind, const R* r) const {
+    R t = R(0);
+    if (kind == K_FULL) {
+      for (int x = 0; x < DIM; ++x) t += w[x] * r[x];
+      return s * t * t;
+    }
+    for (int x = 0; x < DIM; ++x) t += (kind == K_ISO ? s : w[x]) * r[x] * r[x];
+    return t;
+  }
+  __device__ __forceinline__ void apply(int kind, const R* g, R* out) const {
+    const R d = kind == K_FULL ? s * (w[0] * g[0] + w[1] * g[1] + w[2] * g[2]) : R(0);
+    for (int x = 0; x < 3; ++x)
+      out[x] = kind == K_FULL ? w[x] * d : (kind == K_ISO ? s : w[x]) * g[x];
+  }
+};
 
 // flux-limited diffusion coefficient (circuit2.f90:180-183, 358-361)
 template <class R>
@@ -101,9 +151,12 @@ __device__ __forceinline__ double group_sum(double v, unsigned gmask) {
 // (FP32: 9 blocks of 128 threads per SM, 56 registers with a 4-byte spill,
 // measured 2.01 -> 1.95 ms on the 128^3 Sedov step against 8 blocks at 64
 // registers; 10 blocks spill 44 bytes and take 2.5 ms)
-template <int K, int DIM, class R, bool GENERAL, int G>
-__global__ void __launch_bounds__(TPB, sizeof(R) == 8 ? 5 : 9)
+template <int K, int DIM, class R, int MODE, int G>
+__global__ void __launch_bounds__(TPB, sizeof(R) == 8 ? 5 : MODE == C2_HYDRO ? 9 : 7)
 k_c2(C2Args a, PackBufs pb, Params P) {
+  constexpr bool HEAT = MODE == C2_HESSIAN || MODE == C2_TWO_NW || MODE == C2_GENERAL;
+  constexpr bool FIELD = MODE == C2_MHD || MODE == C2_GENERAL;
+  constexpr bool PRESSURE = MODE == C2_HYDRO || MODE == C2_MHD || MODE == C2_GENERAL;
   const int64_t c = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G;
   const int lane = threadIdx.x & (G - 1);
   const int wl = threadIdx.x & 31;
@@ -127,7 +180,14 @@ k_c2(C2Args a, PackBufs pb, Params P) {
     Kh *= R(P.wCv);                      // wCv / h_a^(d+1)
     const R Ka = Kh * R(KDfScale<K>::v);  // with f'(q) as kshape_df_scaled
     const R beta = R(P.beta);
-    const bool artts = P.artts == 1, adden = P.adden == 1, hydro = P.eq_hydro != 0;
+    const bool artts = PRESSURE && P.artts == 1, adden = P.adden == 1,
+               hydro = PRESSURE && P.eq_hydro != 0;
+    const bool heat = MODE == C2_GENERAL ? P.eq_diff != 0 : HEAT;
+    const bool field = MODE == C2_GENERAL ? P.eq_magneto != 0 : FIELD;
+    const bool fld = MODE == C2_GENERAL && P.eq_fld != 0;
+    const bool hessian = MODE == C2_HESSIAN ||
+                         (MODE == C2_GENERAL &&
+                          (P.ddw == esd_fab || P.ddw == esd_fw || P.ddw == esd_n2w));
     // the artificial conductivity term (circuit2.f90:316-331) is scaled by
     // au: au = -1 switches it off in the reference, and au = 0 makes it
     // vanish, so it is skipped for both
@@ -141,45 +201,42 @@ k_c2(C2Args a, PackBufs pb, Params P) {
     for (int d = 0; d < 3; ++d) { dv[d].init(); db[d].init(); }
     du.init(); drho.init(); ddt.init();
 
-    // ---- per-centre set-up of the general path ----
+    // ---- per-centre set-up of the other equations ----
     PartX<R> AX;
-    R kta[3][3], ktb[3][3], uba[3] = {R(0), R(0), R(0)}, ubb[3] = {R(0), R(0), R(0)};
+    Tensor<R> kta, ktb;
+    const int kind = fld || P.difiso == 1 ? K_ISO : P.full_tensor ? K_FULL : K_DIAG;
+    R kga[3] = {R(0), R(0), R(0)};  // K_a grad T_a
     R halfB2a = R(0);
     const R mu0inv = R(1.0 / P.muzero);
-    if constexpr (GENERAL) {
-      Loader<R>::extra(pb, k, AX);
-      for (int x = 0; x < 3; ++x)
-        for (int y = 0; y < 3; ++y) { kta[x][y] = R(0); ktb[x][y] = R(0); }
-      R b2 = AX.bx * AX.bx + AX.by * AX.by + AX.bz * AX.bz;
+    SumAcc<R> tension;  // sum of m_b (B_a . r) g_a Pi_a / mu0, which meets B_a
+    tension.init();
+    if constexpr (MODE != C2_HYDRO) {
+      Loader<R>::template extra<MODE>(pb, k, AX);
+      const R b2 = AX.bx * AX.bx + AX.by * AX.by + AX.bz * AX.bz;
       halfB2a = R(0.5) * b2;
-      if (b2 != R(0)) {
-        R ib = frsqrt<R>(b2);
-        uba[0] = AX.bx * ib; uba[1] = AX.by * ib; uba[2] = AX.bz * ib;
-      }
-      if (P.eq_diff) {
-        if (P.eq_fld) {
+      kta.init();
+      ktb.init();
+      if (heat) {
+        if (fld) {
           R lam;
           R gn = my_sqrt<R>(AX.gx * AX.gx + AX.gy * AX.gy + AX.gz * AX.gz);
           R fd = fld_coef<R>(gn, AX.kappa, A.rho, AX.T, lam);
-          kta[0][0] = kta[1][1] = kta[2][2] = fd;
+          kta.s = fd;
           if (lane == 0)
             cols[es_vfld * ld + p] = double(fd) / ((double(AX.T) * double(A.rho)) / double(gn));
         } else if (P.difiso == 1) {
-          R dc = R(P.difcond);
-          kta[0][0] = kta[1][1] = kta[2][2] = dc;
-          ktb[0][0] = ktb[1][1] = ktb[2][2] = dc;
+          kta.s = ktb.s = R(P.difcond);
         } else {
-          aniso_tensor<R>(R(P.difcond), uba, P.full_tensor, kta);
+          const R ib = b2 != R(0) ? frsqrt<R>(b2) : R(0);
+          kta.aniso(kind, R(P.difcond), AX.bx * ib, AX.by * ib, AX.bz * ib);
+        }
+        if (!hessian) {
+          const R ga3[3] = {AX.gx, AX.gy, AX.gz};
+          kta.apply(kind, ga3, kga);
         }
       }
     }
-    R kga[3] = {R(0), R(0), R(0)};  // K_a grad T_a
-    if constexpr (GENERAL) {
-      if (P.eq_diff) {
-        const R ga3[3] = {AX.gx, AX.gy, AX.gz};
-        for (int x = 0; x < 3; ++x) kga[x] = kta[x][0] * ga3[0] + kta[x][1] * ga3[1] + kta[x][2] * ga3[2];
-      }
-    }
+    const R tra = MODE != C2_HYDRO && hessian ? kta.template trace<DIM>(kind) : R(0);
 
     bool bad = false;
     const int n = a.ncnt[c];
@@ -207,8 +264,8 @@ k_c2(C2Args a, PackBufs pb, Params P) {
       const R qa = r * A.invh, qb = r * B.invh;
       bad |= q_bad(qa) || q_bad(qb);
       R fa = R(0), dfa, ddfa = R(0);
-      if constexpr (GENERAL) {
-        if (P.eq_diff && (P.ddw == esd_n2w || P.ddw == esd_fw)) {
+      if constexpr (HEAT) {
+        if (heat && hessian && P.ddw != esd_fab) {
           R d1;
           kshape_all<K, R>(qa, fa, d1, ddfa);
         }
@@ -250,83 +307,88 @@ k_c2(C2Args a, PackBufs pb, Params P) {
       if (hydro) Fb += B.P;  // circuit2.f90:338-345
       const R F = ga * FaPi + gbPi * Fb;
       du.add(mgv * DaPi);
-      if constexpr (GENERAL) {
+      R Fr = F;  // the force's factor along r_ab
+      if constexpr (MODE != C2_HYDRO) {
         PartX<R> BX;
-        Loader<R>::extra(pb, j, BX);
-        if (P.eq_diff) {
+        Loader<R>::template extra<MODE>(pb, j, BX);
+        if (heat) {
           // circuit2.f90:347-425
-          if (P.eq_fld) {
+          if (fld) {
             R lam;
             R gn = my_sqrt<R>(BX.gx * BX.gx + BX.gy * BX.gy + BX.gz * BX.gz);
-            R fd = fld_coef<R>(gn, BX.kappa, B.rho, BX.T, lam);
-            for (int x = 0; x < 3; ++x)
-              for (int y = 0; y < 3; ++y) ktb[x][y] = (x == y) ? fd : R(0);
+            ktb.s = fld_coef<R>(gn, BX.kappa, B.rho, BX.T, lam);
           } else if (P.difiso == 0) {
-            R b2 = BX.bx * BX.bx + BX.by * BX.by + BX.bz * BX.bz;
-            if (b2 != R(0)) {  // a zero B_b keeps the previous unit vector (:220-224)
-              R ib = frsqrt<R>(b2);
-              ubb[0] = BX.bx * ib; ubb[1] = BX.by * ib; ubb[2] = BX.bz * ib;
+            const R b2 = BX.bx * BX.bx + BX.by * BX.by + BX.bz * BX.bz;
+            if (b2 != R(0)) {  // a zero B_b keeps the previous tensor (:220-224)
+              const R ib = frsqrt<R>(b2);
+              ktb.aniso(kind, R(P.difcond), BX.bx * ib, BX.by * ib, BX.bz * ib);
             }
-            aniso_tensor<R>(R(P.difcond), ubb, P.full_tensor, ktb);
           }
-          const int ddw = P.ddw;
-          if (ddw == esd_fab || ddw == esd_fw || ddw == esd_n2w) {
+          if (hessian) {
             // K_bar : Hessian_a  (kernel.f90:377-539, circuit2.f90:390-397)
-            R rr = R(0), tr = R(0);
-            for (int x = 0; x < DIM; ++x) {
-              tr += R(0.5) * (kta[x][x] + ktb[x][x]);
-              for (int y = 0; y < DIM; ++y) rr += R(0.5) * (kta[x][y] + ktb[x][y]) * rab[x] * rab[y];
-            }
-            rr = rr * (invr * invr);
+            const R tr = R(0.5) * (tra + ktb.template trace<DIM>(kind));
+            const R rr = R(0.5) * (kta.template form<DIM>(kind, rab) + ktb.template form<DIM>(kind, rab)) *
+                         (invr * invr);
             R contr;
-            if (ddw == esd_n2w) {
+            if (P.ddw == esd_n2w) {
               contr = Kh * A.invh * ddfa * rr + ga * (tr - rr);
             } else {
-              const R f2 = (ddw == esd_fab) ? -ga : R(0.5) * R(P.fwc) * Kh * A.invh * fa;
+              const R f2 = (P.ddw == esd_fab) ? -ga : R(0.5) * R(P.fwc) * Kh * A.invh * fa;
               contr = f2 * (R(DIM + 2) * rr - tr);
             }
             ddt.add(fdiv<R>(mb, B.rho * A.rho) * (BX.T * B.rho - AX.T * A.rho) * contr);
           } else {
             R kgb[3];
             const R gb3[3] = {BX.gx, BX.gy, BX.gz};
-            for (int x = 0; x < 3; ++x) kgb[x] = ktb[x][0] * gb3[0] + ktb[x][1] * gb3[1] + ktb[x][2] * gb3[2];
+            ktb.apply(kind, gb3, kgb);
             R ka_r = R(0), kb_r = R(0);
             for (int x = 0; x < DIM; ++x) { ka_r += kga[x] * rab[x]; kb_r += kgb[x] * rab[x]; }
-            if (ddw == esd_2nw_ds) ddt.add(mb * (ga * ka_r * A.Pi + gbPi * kb_r));
+            if (P.ddw == esd_2nw_ds) ddt.add(mb * (ga * ka_r * A.Pi + gbPi * kb_r));
             else ddt.add(mb * A.Pi * ga * (kb_r - ka_r));  // esd_2nw_sd
           }
         }
-        if (P.eq_magneto) {
-          // circuit2.f90:427-462
+        if (field) {
+          // circuit2.f90:427-462: the stress of a is (B_a^2 / 2 r_ab -
+          // B_a (B_a . r_ab)) / mu0; its first part joins the pressure's
+          // factor, its second meets the centre's own B_a after the loop
           const R Ba[3] = {AX.bx, AX.by, AX.bz}, Bb[3] = {BX.bx, BX.by, BX.bz};
           R Bar = R(0), Bbr = R(0);
           for (int x = 0; x < DIM; ++x) { Bar += Ba[x] * rab[x]; Bbr += Bb[x] * rab[x]; }
           const R halfB2b = R(0.5) * (Bb[0] * Bb[0] + Bb[1] * Bb[1] + Bb[2] * Bb[2]);
+          const R gam = ga * A.Pi * mu0inv, gbm = gbPi * mu0inv;
+          Fr += gam * halfB2a + gbm * halfB2b;
+          tension.add(mb * (gam * Bar));
+          const R tb = mb * (gbm * Bbr), mga = mb * ga;
           for (int x = 0; x < 3; ++x) {
-            const R rx = x < DIM ? rab[x] : R(0);
-            const R ma_x = (halfB2a * rx - Ba[x] * Bar) * mu0inv;  // MPa . r_ab
-            const R mb_x = (halfB2b * rx - Bb[x] * Bbr) * mu0inv;
-            dv[x].add(-mb * (ga * ma_x * A.Pi + gbPi * mb_x));
-            db[x].add(-mb * rPiA * ga * (vab[x] * Bar - Bb[x] * vr));
+            dv[x].add(tb * Bb[x]);
+            db[x].add(mga * (Bb[x] * vr - vab[x] * Bar));
           }
         }
       }
-      for (int d = 0; d < DIM; ++d) dv[d].add(-mb * F * rab[d]);
+      if constexpr (PRESSURE)
+        for (int d = 0; d < DIM; ++d) dv[d].add(-mb * Fr * rab[d]);
     }
     }
     if (bad) raise_status(a.status, SPH_ERR_Q_NAN);
     const double mref = a.mref;
-    const double ax = group_sum<G>(dv[0].dval(), gmask);
-    const double ay = DIM >= 2 || GENERAL ? group_sum<G>(dv[1].dval(), gmask) : 0.0;
-    const double az = DIM == 3 || GENERAL ? group_sum<G>(dv[2].dval(), gmask) : 0.0;
-    const double dus = group_sum<G>(du.dval(), gmask);
+    double ax = 0.0, ay = 0.0, az = 0.0, dus = 0.0;
+    if constexpr (PRESSURE) {
+      ax = group_sum<G>(dv[0].dval(), gmask);
+      if (DIM >= 2 || FIELD) ay = group_sum<G>(dv[1].dval(), gmask);
+      if (DIM == 3 || FIELD) az = group_sum<G>(dv[2].dval(), gmask);
+      dus = group_sum<G>(du.dval(), gmask);
+    }
     const double drs = group_sum<G>(drho.dval(), gmask);
     double dts = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
-    if constexpr (GENERAL) {
-      dts = group_sum<G>(ddt.dval(), gmask);
-      b0 = group_sum<G>(db[0].dval(), gmask);
-      b1 = group_sum<G>(db[1].dval(), gmask);
-      b2 = group_sum<G>(db[2].dval(), gmask);
+    if constexpr (HEAT) dts = group_sum<G>(ddt.dval(), gmask);
+    if constexpr (FIELD) {
+      const double t = group_sum<G>(tension.dval(), gmask), rp = double(rPiA);
+      ax += t * double(AX.bx);
+      ay += t * double(AX.by);
+      az += t * double(AX.bz);
+      b0 = rp * group_sum<G>(db[0].dval(), gmask);
+      b1 = rp * group_sum<G>(db[1].dval(), gmask);
+      b2 = rp * group_sum<G>(db[2].dval(), gmask);
     }
     if (lane == 0) {
       pairs = n;
@@ -351,20 +413,24 @@ k_c2(C2Args a, PackBufs pb, Params P) {
   if (wl == 0 && wp) atomicAdd(&a.dcnt[DC_C2_PAIRS], wp);
 }
 
-template <int K, int DIM, class R, bool GEN>
+template <int K, int DIM, class R, int MODE>
 void run_g(const C2Args& a, const PackBufs& pb, const Params& P, cudaStream_t s) {
   switch (a.G) {
-    case 4: k_c2<K, DIM, R, GEN, 4><<<nblocks(a.nc * 4), TPB, 0, s>>>(a, pb, P); break;
-    case 8: k_c2<K, DIM, R, GEN, 8><<<nblocks(a.nc * 8), TPB, 0, s>>>(a, pb, P); break;
-    case 16: k_c2<K, DIM, R, GEN, 16><<<nblocks(a.nc * 16), TPB, 0, s>>>(a, pb, P); break;
-    default: k_c2<K, DIM, R, GEN, 32><<<nblocks(a.nc * 32), TPB, 0, s>>>(a, pb, P); break;
+    case 4: k_c2<K, DIM, R, MODE, 4><<<nblocks(a.nc * 4), TPB, 0, s>>>(a, pb, P); break;
+    case 8: k_c2<K, DIM, R, MODE, 8><<<nblocks(a.nc * 8), TPB, 0, s>>>(a, pb, P); break;
+    case 16: k_c2<K, DIM, R, MODE, 16><<<nblocks(a.nc * 16), TPB, 0, s>>>(a, pb, P); break;
+    default: k_c2<K, DIM, R, MODE, 32><<<nblocks(a.nc * 32), TPB, 0, s>>>(a, pb, P); break;
   }
 }
 template <int K, int DIM, class R>
 void run(const C2Args& a, const PackBufs& pb, const Params& P, cudaStream_t s) {
-  const bool general = P.eq_diff || P.eq_magneto;
-  if (general) run_g<K, DIM, R, true>(a, pb, P, s);
-  else run_g<K, DIM, R, false>(a, pb, P, s);
+  const bool alone = P.eq_diff && !P.eq_hydro && !P.eq_magneto && !P.eq_fld && P.artts != 1;
+  if (!P.eq_diff && !P.eq_magneto) run_g<K, DIM, R, C2_HYDRO>(a, pb, P, s);
+  else if (!P.eq_diff) run_g<K, DIM, R, C2_MHD>(a, pb, P, s);
+  else if (!alone) run_g<K, DIM, R, C2_GENERAL>(a, pb, P, s);
+  else if (P.ddw == esd_fab || P.ddw == esd_fw || P.ddw == esd_n2w)
+    run_g<K, DIM, R, C2_HESSIAN>(a, pb, P, s);
+  else run_g<K, DIM, R, C2_TWO_NW>(a, pb, P, s);
   note_launch();
 }
 template <int K, int DIM>
