@@ -296,10 +296,14 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
 }
 
 // ---- one Jacobi sweep (diffusion / FLD, and the direct summation) ------------------------
+// Neighbours are read from the snapshot taken before the sweep, so the sweep
+// stores its own rho, h, Omega and EOS in the table at once; h at the start
+// of the iterate, which eps is relative to, waits in h0.  (Storing them
+// apart cost four copies before the sweeps and a pass after: a 64^2
+// diffusion iterate's circuit1 took 49 us for 8 us of sums.  NA_SWEEP)
 template <int K, int DIM, class R, int G>
 __global__ void __launch_bounds__(TPB)
 k_c1_sweep(C1Args a, PackBufs pb, Params P) {
-  if (a.gate && *a.gate == 0ull) return;  // the previous sweep left no particle active
   const int64_t c = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / G;
   const int lane = threadIdx.x & (G - 1);
   const unsigned gmask = group_mask<G>();
@@ -310,13 +314,14 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
     const int64_t p = a.centre_p[c];
     double* cols = a.cols;
     const int64_t ld = a.ld;
-    if (a.simple || a.eps[p] > P.tol) {
+    const bool first = a.iter_dev ? *a.iter_dev == 0 : a.first != 0;
+    if (a.simple || first || a.eps[p] > P.tol) {
       R mi;
       const typename PosAccess<R>::Pos pi = PosAccess<R>::load(pb, k, mi);
       const R punit = PosAccess<R>::unit(pb);
       const double ma = cols[es_m * ld + p];
-      const double ha0 = cols[es_h * ld + p];
       const double ha = a.hk_s[k], rhoa = a.dk_s[k], oma = a.ok_s[k];
+      const double ha0 = first ? ha : a.h0[p];
       const double ta = cols[es_t * ld + p];
       const int n = a.ncnt[c];
       const int32_t* __restrict__ row = a.nl + a.rowoff[c];
@@ -400,9 +405,10 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
         if (a.simple) {
           // circuit1.f90:293-301
           const double hnew = P.hfac * pow(ma / wsum, 1. / DIM);
-          a.dkp1[p] = wsum;
-          a.hkp1[p] = hnew;
-          a.okp1[p] = 1.;
+          cols[es_den * ld + p] = wsum;
+          cols[es_h * ld + p] = hnew;
+          cols[es_om * ld + p] = 1.;
+          eos_epilogue(cols, ld, p, wsum, P);
         } else {
           const double osum = -P.wCv * ihd / ha * (a.mref * sot + ma * (DIM * double(f0)));
           double rho, om, hn;
@@ -414,13 +420,14 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
             // (a table at rest otherwise takes 2-3 sweeps per iterate that
             // move h only within the FP32 sums' noise)
             const double eps_prev = a.eps[p];
-            const bool first = a.iter_dev ? *a.iter_dev == 0 : a.first != 0;
             if (eps > P.tol && eps < 1e-7 && (first || eps >= 0.5 * eps_prev)) eps = 0.0;
           }
           a.eps[p] = eps;
-          a.dkp1[p] = rho;
-          a.okp1[p] = om;
-          a.hkp1[p] = hn;
+          if (first) a.h0[p] = ha;
+          cols[es_den * ld + p] = rho;
+          cols[es_om * ld + p] = om;
+          cols[es_h * ld + p] = hn;
+          eos_epilogue(cols, ld, p, rho, P);
           active_left = eps > P.tol ? 1 : 0;
         }
       }
@@ -439,36 +446,28 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
   }
 }
 
+// h, rho and Omega of every record from its row; clears the word in which
+// the sweep marks that a particle stays active
 __global__ void k_c1_snapshot(int64_t n, const int32_t* __restrict__ ssrc,
-                              const double* __restrict__ hkp1, const double* __restrict__ dkp1,
-                              const double* __restrict__ okp1, double* __restrict__ hk_s,
-                              double* __restrict__ dk_s, double* __restrict__ ok_s,
-                              const DevPlan* __restrict__ plan,
-                              const unsigned long long* __restrict__ gate) {
-  if (gate && *gate == 0ull) return;
+                              const double* __restrict__ cols, int64_t ld,
+                              double* __restrict__ hk_s, double* __restrict__ dk_s,
+                              double* __restrict__ ok_s, unsigned long long* __restrict__ active,
+                              const DevPlan* __restrict__ plan) {
   int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (k == 0) *active = 0ull;
   if (plan) n = plan->nall;  // launched over the capacity
   if (k >= n) return;
   int64_t p = ssrc[k];
-  hk_s[k] = hkp1[p];
-  dk_s[k] = dkp1[p];
-  ok_s[k] = okp1[p];
+  hk_s[k] = cols[es_h * ld + p];
+  dk_s[k] = cols[es_den * ld + p];
+  ok_s[k] = cols[es_om * ld + p];
 }
 
-// Store the converged iterates (circuit1.f90:213-215 / 299-301) and run the EOS.
-__global__ void k_c1_finalize(int64_t nrows, int64_t nreal, double* __restrict__ cols, int64_t ld,
-                              const double* __restrict__ hkp1, const double* __restrict__ dkp1,
-                              const double* __restrict__ okp1, int simple, Params P) {
-  int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (p >= nrows) return;
-  if (p < nreal) {
-    cols[es_h * ld + p] = hkp1[p];
-    cols[es_den * ld + p] = dkp1[p];
-    cols[es_om * ld + p] = okp1[p];
-    eos_epilogue(cols, ld, p, dkp1[p], P);
-  } else if (simple) {
-    cols[es_om * ld + p] = 1.;  // circuit1.f90:62 sets every row
-  }
+// direct summation: Omega = 1 on the rows that are no centres (circuit1.f90:62)
+__global__ void k_c1_simple_rest(int64_t nrows, int64_t nreal, double* __restrict__ cols,
+                                 int64_t ld) {
+  const int64_t p = nreal + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (p < nrows) cols[es_om * ld + p] = 1.;
 }
 
 template <int K, int DIM, class R>
@@ -526,18 +525,15 @@ void launch_c1_sweep(int prec, int kernel, int dim, const C1Args& a, PackBufs pb
                      cudaStream_t s) {
   dispatch_sweep_all(prec, kernel, dim, a, pb, P, s);
 }
-void launch_c1_finalize(int64_t nrows, int64_t nreal, double* cols, int64_t ld, const double* hkp1,
-                        const double* dkp1, const double* okp1, int simple, Params P,
-                        cudaStream_t s) {
-  k_c1_finalize<<<nblocks(nrows, 256), 256, 0, s>>>(nrows, nreal, cols, ld, hkp1, dkp1, okp1,
-                                                    simple, P);
+void launch_c1_simple_rest(int64_t nrows, int64_t nreal, double* cols, cudaStream_t s) {
+  if (nrows <= nreal) return;
+  k_c1_simple_rest<<<nblocks(nrows - nreal, 256), 256, 0, s>>>(nrows, nreal, cols, nrows);
   note_launch();
 }
-void launch_c1_snapshot(int64_t n, const int32_t* ssrc, const double* hkp1, const double* dkp1,
-                        const double* okp1, double* hk_s, double* dk_s, double* ok_s,
-                        cudaStream_t s, const DevPlan* plan, const unsigned long long* gate) {
-  k_c1_snapshot<<<nblocks(n, 256), 256, 0, s>>>(n, ssrc, hkp1, dkp1, okp1, hk_s, dk_s, ok_s,
-                                                plan, gate);
+void launch_c1_snapshot(int64_t n, const int32_t* ssrc, const double* cols, int64_t ld,
+                        double* hk_s, double* dk_s, double* ok_s, unsigned long long* active,
+                        cudaStream_t s, const DevPlan* plan) {
+  k_c1_snapshot<<<nblocks(n, 256), 256, 0, s>>>(n, ssrc, cols, ld, hk_s, dk_s, ok_s, active, plan);
   note_launch();
 }
 

@@ -238,7 +238,7 @@ struct sph_handle {
   // canonical store, SoA columns of length nrows
   DevBuf cols, cols_alt, orig, orig_alt, staging;
   // predictor saves, STS stages, circuit1 iterates
-  DevBuf save, stsY, hkp1, dkp1, okp1, epsb;
+  DevBuf save, stsY, c1_h0, epsb;
   // images
   DevBuf gcount, goff, gx, gy, gz, gsrc, gcode, scan_tmp;
   int64_t nghost = 0;
@@ -575,9 +575,7 @@ struct sph_handle {
     RC(dl_inv.ensure(sizeof(int32_t) * nrows));
     RC(xfer_setup());  // (the table transfers' copy stream and events)
     RC(save.ensure(sizeof(double) * 9 * nrows));
-    RC(hkp1.ensure(sizeof(double) * nrows));
-    RC(dkp1.ensure(sizeof(double) * nrows));
-    RC(okp1.ensure(sizeof(double) * nrows));
+    RC(c1_h0.ensure(sizeof(double) * nrows));
     RC(epsb.ensure(sizeof(double) * nrows));
     RC(gcount.ensure(sizeof(int32_t) * (nrows + 1)));
     RC(goff.ensure(sizeof(int32_t) * (nrows + 1)));
@@ -1369,16 +1367,13 @@ struct sph_handle {
     a.hk_s = hk_s.as<double>();
     a.dk_s = dk_s.as<double>();
     a.ok_s = ok_s.as<double>();
-    a.hkp1 = hkp1.as<double>();
-    a.dkp1 = dkp1.as<double>();
-    a.okp1 = okp1.as<double>();
+    a.h0 = c1_h0.as<double>();
     a.eps = epsb.as<double>();
     a.mref = mref;
     a.status = status.as<int>();
     a.dcnt = dcnt.as<unsigned long long>();
     a.red = red.as<unsigned long long>();
     a.active_slot = RED_C1_ACTIVE;
-    a.gate = nullptr;
     const bool advanced = ival(ec_adden) == 1;
     if (advanced && P.maxiter == 0) {  // zero sweeps: h, rho, Omega stay (circuit1.f90:114)
       launch_eos(cols.as<double>(), nrows, nreal, P, s);
@@ -1392,10 +1387,6 @@ struct sph_handle {
     }
     // Jacobi sweeps (circuit1.f90:105-211) / direct summation (:237-301)
     a.simple = advanced ? 0 : 1;
-    CK(cudaMemcpyAsync(hkp1.p, col(es_h), sizeof(double) * nrows, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(dkp1.p, col(es_den), sizeof(double) * nrows, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(okp1.p, col(es_om), sizeof(double) * nrows, cudaMemcpyDeviceToDevice, s));
-    launch_set_col(epsb.as<double>(), nrows, 1.0, s);
     int iter = 0;
     if (dplan) {
       // device-resident step: the sweeps as a while node, as many as the
@@ -1404,12 +1395,10 @@ struct sph_handle {
       // sets the error word, which sends the step back to the host path
       unsigned long long* rb = red.as<unsigned long long>();
       a.active_slot = RED_C1_ACTIVE;
-      a.gate = nullptr;
       auto sweep = [&]() {
-        launch_c1_snapshot(nall_cap, ssrc.as<int32_t>(), hkp1.as<double>(), dkp1.as<double>(),
-                           okp1.as<double>(), hk_s.as<double>(), dk_s.as<double>(),
-                           ok_s.as<double>(), s, dplan, nullptr);
-        launch_fill_u64(rb + RED_C1_ACTIVE, 1, 0ull, s);
+        launch_c1_snapshot(nall_cap, ssrc.as<int32_t>(), cols.as<double>(), nrows,
+                           hk_s.as<double>(), dk_s.as<double>(), ok_s.as<double>(),
+                           rb + RED_C1_ACTIVE, s, dplan);
         launch_c1_sweep(prec, kernel_id, P.dim, a, pb, P, s);
       };
       if (a.simple) {
@@ -1436,10 +1425,9 @@ struct sph_handle {
     for (;;) {
       ++iter;
       a.first = iter == 1;
-      launch_c1_snapshot(nall, ssrc.as<int32_t>(), hkp1.as<double>(), dkp1.as<double>(),
-                         okp1.as<double>(), hk_s.as<double>(), dk_s.as<double>(),
-                         ok_s.as<double>(), s);
-      launch_fill_u64(red.as<unsigned long long>() + RED_C1_ACTIVE, 1, 0ull, s);
+      launch_c1_snapshot(nall, ssrc.as<int32_t>(), cols.as<double>(), nrows, hk_s.as<double>(),
+                         dk_s.as<double>(), ok_s.as<double>(),
+                         red.as<unsigned long long>() + RED_C1_ACTIVE, s);
       launch_c1_sweep(prec, kernel_id, P.dim, a, pb, P, s);
       if (a.simple) break;
       CK(cudaMemcpyAsync(h_red + RED_C1_ACTIVE, red.as<unsigned long long>() + RED_C1_ACTIVE,
@@ -1448,8 +1436,7 @@ struct sph_handle {
       CK(cudaGetLastError());
       if (!h_red[RED_C1_ACTIVE] || iter >= P.maxiter) break;
     }
-    launch_c1_finalize(nrows, nreal, cols.as<double>(), nrows, hkp1.as<double>(),
-                       dkp1.as<double>(), okp1.as<double>(), a.simple, P, s);
+    if (a.simple) launch_c1_simple_rest(nrows, nreal, cols.as<double>(), s);
     host_max_sweeps = std::max<int64_t>(host_max_sweeps, iter);
     CK(cudaGetLastError());
     return SPH_OK;

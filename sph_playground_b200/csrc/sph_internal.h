@@ -608,9 +608,7 @@ struct C1Args {
   const double* hk_s;  // snapshots in sorted order
   const double* dk_s;
   const double* ok_s;
-  double* hkp1;
-  double* dkp1;
-  double* okp1;
+  double* h0;  // per row: h at the start of the iterate
   double* eps;
   int simple;  // c1simple
   double mref;
@@ -618,7 +616,6 @@ struct C1Args {
   unsigned long long* dcnt;
   unsigned long long* red;
   int active_slot;                  // red slot the sweep marks when a particle stays active
-  const unsigned long long* gate;   // if set and zero, the sweep has nothing to do
   int first;                        // the iterate's first sweep
   const int* iter_dev;              // if set: the first sweep is the one where *iter_dev == 0
 };
@@ -626,13 +623,10 @@ void launch_c1_newton(int prec, int kernel, int dim, const C1Args& a, PackBufs p
                       cudaStream_t s);
 void launch_c1_sweep(int prec, int kernel, int dim, const C1Args& a, PackBufs pb, Params P,
                      cudaStream_t s);
-void launch_c1_finalize(int64_t nrows, int64_t nreal, double* cols, int64_t ld, const double* hkp1,
-                        const double* dkp1, const double* okp1, int simple, Params P,
-                        cudaStream_t s);
-void launch_c1_snapshot(int64_t n, const int32_t* ssrc, const double* hkp1,
-                        const double* dkp1, const double* okp1, double* hk_s, double* dk_s,
-                        double* ok_s, cudaStream_t s, const DevPlan* plan = nullptr,
-                        const unsigned long long* gate = nullptr);
+void launch_c1_simple_rest(int64_t nrows, int64_t nreal, double* cols, cudaStream_t s);
+void launch_c1_snapshot(int64_t n, const int32_t* ssrc, const double* cols, int64_t ld,
+                        double* hk_s, double* dk_s, double* ok_s, unsigned long long* active,
+                        cudaStream_t s, const DevPlan* plan = nullptr);
 
 // ---- circuit2 (sph_circuit2.cu) ---------------------------------------------------
 struct C2Args {
