@@ -446,15 +446,19 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
   }
 }
 
-// h, rho and Omega of every record from its row; clears the word in which
-// the sweep marks that a particle stays active
+// h, rho and Omega of every record from its row; clears the word active[0]
+// in which the sweep marks that a particle stays active, having counted in
+// active[1] the sweeps before this one that left one
 __global__ void k_c1_snapshot(int64_t n, const int32_t* __restrict__ ssrc,
                               const double* __restrict__ cols, int64_t ld,
                               double* __restrict__ hk_s, double* __restrict__ dk_s,
-                              double* __restrict__ ok_s, unsigned long long* __restrict__ active,
+                              double* __restrict__ ok_s, unsigned long long* __restrict__ active, int first,
                               const DevPlan* __restrict__ plan) {
   int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (k == 0) *active = 0ull;
+  if (k == 0) {
+    active[1] = first ? 0ull : active[1] + (active[0] ? 1ull : 0ull);
+    active[0] = 0ull;
+  }
   if (plan) n = plan->nall;  // launched over the capacity
   if (k >= n) return;
   int64_t p = ssrc[k];
@@ -532,8 +536,9 @@ void launch_c1_simple_rest(int64_t nrows, int64_t nreal, double* cols, cudaStrea
 }
 void launch_c1_snapshot(int64_t n, const int32_t* ssrc, const double* cols, int64_t ld,
                         double* hk_s, double* dk_s, double* ok_s, unsigned long long* active,
-                        cudaStream_t s, const DevPlan* plan) {
-  k_c1_snapshot<<<nblocks(n, 256), 256, 0, s>>>(n, ssrc, cols, ld, hk_s, dk_s, ok_s, active, plan);
+                        int first, cudaStream_t s, const DevPlan* plan) {
+  k_c1_snapshot<<<nblocks(n, 256), 256, 0, s>>>(n, ssrc, cols, ld, hk_s, dk_s, ok_s, active,
+                                                first, plan);
   note_launch();
 }
 

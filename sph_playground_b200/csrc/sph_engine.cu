@@ -304,7 +304,11 @@ struct sph_handle {
   // iterate after the end of the table's fixed part (skin_end[0]): their
   // capacities and the scan of those
   DevBuf skin_end, skin_dcap, skin_doff;
-  DevBuf skin_out, skin_bcnt;  // a served iterate's result (SkinOut), its blocks' list lengths
+  // a served iterate's result (SkinOut); its reduction slots and counts, two
+  // sets used in turn (skin_turn)
+  DevBuf skin_out, skin_slots, skin_counts;
+  int skin_turn = 0;
+  bool pos_packed = false;     // the served iterate wrote circuit1's records
   SkinOut* h_skin = nullptr;   // (pinned)
   int skin_most = 0;           // blocks of k_skin_serve resident at once
   // rows renamed: spare signatures, the two permutations, the old types, a flag
@@ -332,6 +336,7 @@ struct sph_handle {
   // (else the next one starts without lists)
   DevBuf dskin;
   bool dlists_ok = false;
+  int c1_last = 1, c1_open = 0;  // sweeps the last iterate needed; sweeps run ahead, not yet asked about
   DevBuf c1_iter;  // the sweep count of the device-resident Newton loop
   // the device-resident STS loop: its stage index and the coefficients of
   // stages 2 .. s (mu, nu, muhat, gmhat), for the s they were made for
@@ -361,6 +366,7 @@ struct sph_handle {
   int est_count = 0;
   // scalars
   DevBuf status, red, dcnt, maxcnt, ctrl, ciso;
+  void* h_pinned = nullptr;             // the block that holds the next three, h_plan and h_skin
   unsigned long long* h_red = nullptr;  // pinned
   double* h_ctrl = nullptr;             // pinned
   int32_t* h_i32 = nullptr;             // pinned scratch
@@ -834,6 +840,8 @@ struct sph_handle {
   int skin_alloc(int64_t nall) {
     RC(skin_alloc_common(nall));
     RC(skin_out.ensure(sizeof(SkinOut)));
+    RC(skin_slots.ensure(2 * RED_TOTAL * sizeof(unsigned long long)));
+    RC(skin_counts.ensure(2 * 4 * sizeof(int32_t)));
     RC(skin_dflag.ensure(sizeof(int32_t) * (nreal + 1)));
     RC(skin_dpos.ensure(sizeof(int32_t) * (nreal + 1)));
     RC(skin_dlist.ensure(sizeof(int32_t) * nreal));
@@ -932,6 +940,8 @@ struct sph_handle {
       launch_skin_filter(filter_args(na, false, true), s);
     }));
     launch_table_end(rowoff.as<int64_t>(), rowcap.as<int32_t>(), nreal, skin_end.as<int64_t>(), s);
+    skin_turn = 0;
+    launch_skin_slots_clear(skin_slots.as<unsigned long long>(), skin_counts.as<int32_t>(), s);
     skin_valid = true;
     skin_live = true;
     skin_s = skin;
@@ -1092,12 +1102,21 @@ struct sph_handle {
     if (blocks <= 0) return fail(SPH_ERR_CUDA, "skin lists: no cooperative launch");
     RC(skin_fcell.ensure(2 * size_t(ncell)));
     RC(skin_mcell.ensure(2 * size_t(ncell)));
-    RC(skin_bcnt.ensure(sizeof(int2) * size_t(blocks)));
     {
       Phase ph(this, SPH_T_NEIGHBOURS);
       SkinServe a{};
       a.r = refresh_args(g, d, float(skin_tau), float(skin_eps));
-      a.wrap = m.ghosts ? 1 : 0;
+      a.r.wrap = m.ghosts ? 1 : 0;
+      a.r.pack = PACK_POS | ((eq_diff || eq_fld) ? PACK_TEMP : 0);
+      a.r.prec = prec;
+      a.r.pb = packs();
+      const int turn = skin_turn, next = 1 - skin_turn;
+      skin_turn = next;
+      a.r.red = skin_slots.as<unsigned long long>() + turn * RED_TOTAL;
+      a.red_next = skin_slots.as<unsigned long long>() + next * RED_TOTAL;
+      a.counts = skin_counts.as<int32_t>() + turn * 4;
+      a.counts_next = skin_counts.as<int32_t>() + next * 4;
+      a.hmaxb = red.as<unsigned long long>() + RED_SKIN_HMAXB;
       a.nall = nall;
       a.pg = pgeom;
       a.grid = grid;
@@ -1118,7 +1137,6 @@ struct sph_handle {
       a.kfac = 1.0 + skin_s;
       a.dcap = P.krad * skin_hmin;
       a.dirty_share = kSkinDirtyShare;
-      a.block_counts = skin_bcnt.as<int2>();
       a.dlist = skin_dlist.as<int32_t>();
       a.flist = skin_flist.as<int32_t>();
       a.flags = maxcnt.as<int32_t>();
@@ -1160,11 +1178,13 @@ struct sph_handle {
     cnt_host[SPH_CNT_SKIN_KEPT] += nkept;
     kept_pairs += kept;
     served = true;
+    pos_packed = true;
     return SPH_OK;
   }
 
   // ---- neighbour phase: images, grid, sort, lists --------------------------------------------
   int neighbour_phase(const Mode& m, const Params& P) {
+    pos_packed = false;
     double skin = skin_fraction();
     if (skin > 0 && skin_valid && skin == skin_s) {
       bool served = false;
@@ -1328,8 +1348,35 @@ struct sph_handle {
     return SPH_OK;
   }
 
+  int read_c1_active() {
+    CK(cudaMemcpyAsync(h_red + RED_C1_ACTIVE, red.as<unsigned long long>() + RED_C1_ACTIVE,
+                       2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    CK(cudaGetLastError());
+    return SPH_OK;
+  }
+  // The end of an iterate: the status, and whether the sweeps that circuit1
+  // ran ahead were enough; if not, it sweeps on from where they left and the
+  // force pass runs again on the result.
+  int finish_iterate(const Mode& m, Params& P) {
+    const int ran = c1_open;
+    c1_open = 0;
+    if (ran) {
+      CK(cudaMemcpyAsync(h_red + RED_C1_ACTIVE, red.as<unsigned long long>() + RED_C1_ACTIVE,
+                         2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    }
+    RC(check_status());  // (waits for the copy too)
+    if (!ran) return SPH_OK;
+    c1_last = 1 + int(h_red[RED_C1_MORE]);
+    if (!h_red[RED_C1_ACTIVE] || ran >= P.maxiter) return SPH_OK;
+    RC(circuit1(m, P, false, ran));
+    RC(circuit2(m, P));
+    return check_status();
+  }
+
   // ---- circuit1 + EOS ----------------------------------------------------------------------
-  int circuit1(const Mode& m, Params& P) {
+  // (defer: see the sweeps; ran > 0: sweep on after that many)
+  int circuit1(const Mode& m, Params& P, bool defer = false, int ran = 0) {
     const int64_t nall = nrows + nghost;
     PackBufs pb = packs();
     P.eos_kind = m.eos_kind;
@@ -1349,7 +1396,7 @@ struct sph_handle {
       if (dplan)
         launch_pack_dev(prec, groups, nall_cap, ssrc.as<int32_t>(), sx.as<double>(),
                         sy.as<double>(), sz.as<double>(), cols.as<double>(), nrows, dplan, pb, s);
-      else
+      else if (!pos_packed)
         launch_pack(prec, groups, nall, ssrc.as<int32_t>(), sx.as<double>(), sy.as<double>(),
                     sz.as<double>(), cols.as<double>(), nrows, pgeom, pb, s);
     }
@@ -1387,7 +1434,7 @@ struct sph_handle {
     }
     // Jacobi sweeps (circuit1.f90:105-211) / direct summation (:237-301)
     a.simple = advanced ? 0 : 1;
-    int iter = 0;
+    int iter = ran;
     if (dplan) {
       // device-resident step: the sweeps as a while node, as many as the
       // particles need (up to kDrsSweeps) without looking at the host; a
@@ -1398,7 +1445,7 @@ struct sph_handle {
       auto sweep = [&]() {
         launch_c1_snapshot(nall_cap, ssrc.as<int32_t>(), cols.as<double>(), nrows,
                            hk_s.as<double>(), dk_s.as<double>(), ok_s.as<double>(),
-                           rb + RED_C1_ACTIVE, s, dplan);
+                           rb + RED_C1_ACTIVE, 0, s, dplan);
         launch_c1_sweep(prec, kernel_id, P.dim, a, pb, P, s);
       };
       if (a.simple) {
@@ -1422,22 +1469,32 @@ struct sph_handle {
         iter = sweeps;
       }
     } else
-    for (;;) {
-      ++iter;
-      a.first = iter == 1;
-      launch_c1_snapshot(nall, ssrc.as<int32_t>(), cols.as<double>(), nrows, hk_s.as<double>(),
-                         dk_s.as<double>(), ok_s.as<double>(),
-                         red.as<unsigned long long>() + RED_C1_ACTIVE, s);
-      launch_c1_sweep(prec, kernel_id, P.dim, a, pb, P, s);
-      if (a.simple) break;
-      CK(cudaMemcpyAsync(h_red + RED_C1_ACTIVE, red.as<unsigned long long>() + RED_C1_ACTIVE,
-                         sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-      CK(cudaStreamSynchronize(s));
-      CK(cudaGetLastError());
-      if (!h_red[RED_C1_ACTIVE] || iter >= P.maxiter) break;
+    {
+      // As many sweeps as the iterate before needed run without asking the
+      // host; with `defer` the question waits for the iterate's own end
+      // (finish_iterate), which mostly answers that they were enough.  A
+      // sweep too many finds no active particle and changes nothing.
+      const int ahead = std::min(P.maxiter, defer && !a.simple ? std::max(1, c1_last) : 1);
+      for (;;) {
+        ++iter;
+        a.first = iter == 1;
+        launch_c1_snapshot(nall, ssrc.as<int32_t>(), cols.as<double>(), nrows, hk_s.as<double>(),
+                           dk_s.as<double>(), ok_s.as<double>(),
+                           red.as<unsigned long long>() + RED_C1_ACTIVE, a.first, s);
+        launch_c1_sweep(prec, kernel_id, P.dim, a, pb, P, s);
+        if (a.simple) break;
+        if (iter < ahead) continue;
+        if (defer) {
+          c1_open = iter;
+          break;
+        }
+        RC(read_c1_active());
+        if (!h_red[RED_C1_ACTIVE] || iter >= P.maxiter) break;
+      }
     }
     if (a.simple) launch_c1_simple_rest(nrows, nreal, cols.as<double>(), s);
     host_max_sweeps = std::max<int64_t>(host_max_sweeps, iter);
+    if (!dplan && !c1_open) c1_last = iter;
     CK(cudaGetLastError());
     return SPH_OK;
   }
@@ -1496,9 +1553,9 @@ struct sph_handle {
     Mode m;
     RC(mode(m));
     RC(neighbour_phase(m, P));
-    RC(circuit1(m, P));
+    RC(circuit1(m, P, full));
     if (full) RC(circuit2(m, P));
-    RC(check_status());
+    RC(finish_iterate(m, P));
     cnt_host[SPH_CNT_ITERATES] += full ? 1 : 0;
     cnt_host[SPH_CNT_CENTRES] += nreal;
     return SPH_OK;
@@ -2088,19 +2145,22 @@ struct sph_handle {
       return fail(SPH_ERR_IC_MUZERO, "mhd_magneticconstant <= 0");
     if (ival(ec_disotropic) > 0 && st[ec_dcondconst] <= 0)
       return fail(SPH_ERR_IC_DIFFCOND, "diff_conductivity <= 0");
-    std::vector<double> h(NCOL * nrows);
-    CK(cudaMemcpyAsync(h.data(), cols.p, sizeof(double) * NCOL * nrows, cudaMemcpyDeviceToHost, s));
+    // the first row (of the table's order) with a bad value, and its first one
+    unsigned long long* bad = red.as<unsigned long long>() + RED_BAD_ROW;
+    CK(cudaMemsetAsync(bad, 0xff, sizeof(unsigned long long), s));
+    launch_check_rows(cols.as<double>(), nrows, bad, s);
+    CK(cudaMemcpyAsync(h_red + RED_BAD_ROW, bad, sizeof(unsigned long long),
+                       cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    auto C = [&](int f, int64_t i) { return h[size_t(f) * nrows + i]; };
-    for (int64_t i = 0; i < nrows; ++i) {
-      if (int(C(es_type, i)) == ept_empty) continue;
-      if (C(es_den, i) <= 0.) return fail(SPH_ERR_IC_DENSITY, "density <= 0");
-      if (C(es_c, i) <= 0.) return fail(SPH_ERR_IC_CSOUND, "csound <= 0");
-      if (C(es_h, i) <= 0.) return fail(SPH_ERR_IC_H, "smoothing length <= 0");
-      if (C(es_p, i) <= 0.) return fail(SPH_ERR_IC_PRESSURE, "pressure <= 0");
-      if (C(es_u, i) <= 0.) return fail(SPH_ERR_IC_ENERGY, "internal energy <= 0");
+    CK(cudaGetLastError());
+    if (h_red[RED_BAD_ROW] == ~0ull) return SPH_OK;
+    switch (h_red[RED_BAD_ROW] & 7ull) {
+      case 0: return fail(SPH_ERR_IC_DENSITY, "density <= 0");
+      case 1: return fail(SPH_ERR_IC_CSOUND, "csound <= 0");
+      case 2: return fail(SPH_ERR_IC_H, "smoothing length <= 0");
+      case 3: return fail(SPH_ERR_IC_PRESSURE, "pressure <= 0");
+      default: return fail(SPH_ERR_IC_ENERGY, "internal energy <= 0");
     }
-    return SPH_OK;
   }
 
   // ---- time loop (main.f90:216-373) ------------------------------------------------------------
@@ -2638,11 +2698,7 @@ struct sph_handle {
     }
     for (auto e : ev_pool) cudaEventDestroy(e);
     drop_graph();
-    if (h_plan) cudaFreeHost(h_plan);
-    if (h_skin) cudaFreeHost(h_skin);
-    if (h_red) cudaFreeHost(h_red);
-    if (h_ctrl) cudaFreeHost(h_ctrl);
-    if (h_i32) cudaFreeHost(h_i32);
+    if (h_pinned) cudaFreeHost(h_pinned);
     for (auto c : cap_s) cudaStreamDestroy(c);
     for (auto e : xfer_ev) cudaEventDestroy(e);
     if (xs) {
@@ -3010,11 +3066,23 @@ int sph_create(const double* state49, const double* store, int64_t n_rows, int k
     delete h;
     return fail(SPH_ERR_CUDA, "cudaStreamCreate failed");
   }
-  if (cudaMallocHost(&h->h_red, sizeof(unsigned long long) * (RED_TOTAL + 2)) != cudaSuccess ||
-      cudaMallocHost(&h->h_ctrl, sizeof(double) * 16) != cudaSuccess ||
-      cudaMallocHost(&h->h_plan, sizeof(DevPlan)) != cudaSuccess ||
-      cudaMallocHost(&h->h_skin, sizeof(SkinOut)) != cudaSuccess ||
-      cudaMallocHost(&h->h_i32, sizeof(int32_t) * 16) != cudaSuccess) {
+  // the handle's small host buffers, one pinned block (a pinned allocation
+  // takes about 0.45 ms, giving it back 0.25 ms)
+  struct Pinned {
+    unsigned long long red[RED_TOTAL + 2];
+    double ctrl[16];
+    DevPlan plan;
+    SkinOut skin;
+    int32_t i32[16];
+  };
+  if (cudaMallocHost(&h->h_pinned, sizeof(Pinned)) == cudaSuccess) {
+    auto* q = static_cast<Pinned*>(h->h_pinned);
+    h->h_red = q->red;
+    h->h_ctrl = q->ctrl;
+    h->h_plan = &q->plan;
+    h->h_skin = &q->skin;
+    h->h_i32 = q->i32;
+  } else {
     cudaGetLastError();
     h->destroy();
     delete h;

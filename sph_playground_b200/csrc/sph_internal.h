@@ -64,13 +64,14 @@ __host__ __device__ inline bool grid_dims(const double e[3], int64_t cap, int n3
 enum RedSlot : int {
   RED_LO_X = 0, RED_LO_Y, RED_LO_Z, RED_HI_X, RED_HI_Y, RED_HI_Z, RED_HMIN,
   RED_TS_HMIN, RED_TS_CMAX, RED_TS_DENMIN, RED_TS_CMIN, RED_TS_KAPMAX,
-  RED_TS_BMAX, RED_TS_KAPMIN, RED_TS_LAMMAX, RED_C1_ACTIVE, RED_C1_ACTIVE2,
+  RED_TS_BMAX, RED_TS_KAPMIN, RED_TS_LAMMAX, RED_C1_ACTIVE, RED_C1_MORE,  // a particle stays active; earlier sweeps that left one
   // skin lists: largest displacement and h (dkey max), image signature
   // changed (0/1), records that moved more than tau and eps (plain counts)
   RED_SKIN_D, RED_SKIN_HMAX, RED_SKIN_SIG, RED_SKIN_NFAST, RED_SKIN_NMOVE,
   RED_SKIN_NKEPT,   // rows a skin-list iterate keeps (plain count)
   RED_SKIN_NKEPT_PAIRS,  // their neighbours (plain count)
   RED_SKIN_HMAXB,   // largest h of the centres at the skin search (dkey max)
+  RED_BAD_ROW,      // run-start check: 8 row + kind of the first bad value (~0: none)
   RED_DSKIN_FAIL,   // device-resident lists: a centre whose row cannot be filtered (0/1)
   RED_TOTAL
 };
@@ -303,6 +304,29 @@ struct NeibArgs {
 // image set is a function of it), 0 for rows that get no images
 void launch_skin_sig(const double* cols, int64_t nrows, BoxGeom g, int dim, uint8_t* sig,
                      cudaStream_t s);
+// pack groups
+// (PACK_TEMP: with PACK_POS, also the temperature stream the circuit1
+// sweeps of the diffusion paths read)
+enum PackGroup : int { PACK_POS = 1, PACK_HYDRO = 2, PACK_EXTRA = 4, PACK_TEMP = 8 };
+struct PackBufs {
+  // FP64: p[0], p[1] = x, y, z, m; p[2] = (1/h, rho / 2), p[3] =
+  // (wCv / (h^(d+1) rho^2 Omega), P), p[4] = (alpha c, au u), p[5], p[6] =
+  // v and T, p[7] .. p[10] the diffusion and field quantities
+  double2* p[11];
+  // FP32: q[0] = (x, y, z high parts, m), q[1] = (x, y, z low parts, 1/h),
+  // q[2] = (rho / 2, wCv / (h^(d+1) rho^2 Omega), P, alpha c), q[3] = (au u, v), q[4] / q[5] the
+  // temperature, diffusion and field quantities (the force pass); q[6] =
+  // (x, y, z as 31-bit fixed point over the packing frame, m) (the density
+  // pass: one 16-byte record per neighbour)
+  float4* q[7];
+  // the length of one fixed-point unit (shift 2^-31), written by the pack
+  // kernel (the frame may be planned on the device)
+  float* unit;
+  // the force pass's factor wCv / h^(d+1) (times c2_df_scale), the viscosity's alpha and
+  // the conductivity's au (set before its packing)
+  double kp_wcv = 0.0, kp_alpha = 0.0, kp_au = 0.0;
+  int kp_dim = 0;
+};
 // per record (sorted order) from the rows' current positions: sx/sy/sz and
 // the FP32 images, the displacement since the skin search (FP64, rounded
 // up, kept in dsp as the running maximum, FP32 rounded up) and the slots
@@ -326,6 +350,11 @@ struct SkinRefresh {
   float tau, eps;
   double* hrec;
   unsigned long long* red;
+  int wrap;  // the rows are wrapped into the periodic box first
+  // PACK_POS, with PACK_TEMP or not: the density pass's records are written
+  // too (0: they are not)
+  int pack, prec;
+  PackBufs pb;
 };
 // (device-resident step: n the launch bound, the count and the packing frame
 // from the plan; with gate set, nothing is done unless gate->live)
@@ -343,8 +372,7 @@ struct SkinOut {
   double D;
 };
 struct SkinServe {
-  SkinRefresh r;
-  int wrap;        // the rows are wrapped into the periodic box first
+  SkinRefresh r;   // (r.red: this launch's slots, cleared before it)
   int64_t nall;    // records
   PackGeom pg;
   Grid grid;       // cells of the lists' search, keys[k] each record's
@@ -360,8 +388,13 @@ struct SkinServe {
   uint8_t* mode;
   const int32_t* ncnt;
   double krad, kfac, dcap, dirty_share;
-  int2* block_counts;     // skin_serve_blocks() entries
-  int32_t *dlist, *flist;  // the centres searched afresh / filtered, in order
+  const unsigned long long* hmaxb;  // largest h of the centres at the lists' search (dkey)
+  // centres searched afresh, filtered, blocks done (cleared before it); and
+  // the slots and counts of the next launch, which this one clears
+  int32_t* counts;
+  unsigned long long* red_next;
+  int32_t* counts_next;
+  int32_t *dlist, *flist;  // the centres searched afresh / filtered
   int32_t* flags;          // longest row, overflow (cleared)
   SkinOut* out;
 };
@@ -369,6 +402,7 @@ struct SkinServe {
 // error of the runtime), and those for n records
 int skin_serve_most_blocks();
 int skin_serve_blocks(int64_t n, int most);
+void launch_skin_slots_clear(unsigned long long* red, int32_t* counts, cudaStream_t s);
 cudaError_t launch_skin_serve(const SkinServe& a, int blocks, cudaStream_t s);
 // with the lists live, per centre: can its row come from its skin list?
 // Every record now within krad h of the centre was within krad h + 2 D at
@@ -507,29 +541,6 @@ void launch_rowcap(int64_t nc, const int32_t* centre_p, const int32_t* orig,
 size_t scan64_temp_bytes(int64_t n);
 void exclusive_scan64(void* tmp, size_t tmp_bytes, const int64_t* in, int64_t* out, int64_t n,
                       cudaStream_t s);
-// pack groups
-// (PACK_TEMP: with PACK_POS, also the temperature stream the circuit1
-// sweeps of the diffusion paths read)
-enum PackGroup : int { PACK_POS = 1, PACK_HYDRO = 2, PACK_EXTRA = 4, PACK_TEMP = 8 };
-struct PackBufs {
-  // FP64: p[0], p[1] = x, y, z, m; p[2] = (1/h, rho / 2), p[3] =
-  // (wCv / (h^(d+1) rho^2 Omega), P), p[4] = (alpha c, au u), p[5], p[6] =
-  // v and T, p[7] .. p[10] the diffusion and field quantities
-  double2* p[11];
-  // FP32: q[0] = (x, y, z high parts, m), q[1] = (x, y, z low parts, 1/h),
-  // q[2] = (rho / 2, wCv / (h^(d+1) rho^2 Omega), P, alpha c), q[3] = (au u, v), q[4] / q[5] the
-  // temperature, diffusion and field quantities (the force pass); q[6] =
-  // (x, y, z as 31-bit fixed point over the packing frame, m) (the density
-  // pass: one 16-byte record per neighbour)
-  float4* q[7];
-  // the length of one fixed-point unit (shift 2^-31), written by the pack
-  // kernel (the frame may be planned on the device)
-  float* unit;
-  // the force pass's factor wCv / h^(d+1) (times c2_df_scale), the viscosity's alpha and
-  // the conductivity's au (set before its packing)
-  double kp_wcv = 0.0, kp_alpha = 0.0, kp_au = 0.0;
-  int kp_dim = 0;
-};
 void launch_pack_dev(int prec, int groups, int64_t ncap, const int32_t* ssrc, const double* sx,
                      const double* sy, const double* sz, const double* cols, int64_t ld,
                      const DevPlan* plan, PackBufs pb, cudaStream_t s);
@@ -574,6 +585,10 @@ void launch_sts_loop_ctl(int* jdev, int sts_s, cudaGraphConditionalHandle h, cud
 void launch_eos(double* cols, int64_t ld, int64_t nreal, Params P, cudaStream_t s);
 void launch_apply_mti(double* cols, int64_t ld, const int32_t* orig, int64_t nrows,
                       int64_t nreal, int lowres, cudaStream_t s);
+// bad = min over the rows that hold a particle of 8 row + k, k the first of
+// density (0), sound speed (1), h (2), pressure (3), energy (4) that is <= 0
+// (preruncheck.f90:36-60)
+void launch_check_rows(const double* cols, int64_t nrows, unsigned long long* bad, cudaStream_t s);
 void launch_set_col(double* col, int64_t n, double v, cudaStream_t s);
 
 // CUB wrappers (sph_grid.cu)
@@ -626,7 +641,7 @@ void launch_c1_sweep(int prec, int kernel, int dim, const C1Args& a, PackBufs pb
 void launch_c1_simple_rest(int64_t nrows, int64_t nreal, double* cols, cudaStream_t s);
 void launch_c1_snapshot(int64_t n, const int32_t* ssrc, const double* cols, int64_t ld,
                         double* hk_s, double* dk_s, double* ok_s, unsigned long long* active,
-                        cudaStream_t s, const DevPlan* plan = nullptr);
+                        int first, cudaStream_t s, const DevPlan* plan = nullptr);
 
 // ---- circuit2 (sph_circuit2.cu) ---------------------------------------------------
 struct C2Args {
