@@ -693,8 +693,13 @@ k_neighbours(NeibArgs a) {
     // Row selection in cell units and FP32: every quantity is widened by a
     // margin far above its rounding, so the selected cells are a superset of
     // the ones the spheres touch; membership is decided per candidate below.
-    ux = float((xi - g.ox) * g.invL); uy = float((yi - g.oy) * g.invL);
-    uz = float((zi - g.oz) * g.invL);
+    // (a NaN coordinate counts as the first cell, where the sort put it: the
+    // box of a segment that holds only such a centre must not be empty)
+    auto cell_unit = [&](double x, double o) {
+      const float u = float((x - o) * g.invL);
+      return u == u ? u : 0.f;
+    };
+    ux = cell_unit(xi, g.ox); uy = cell_unit(yi, g.oy); uz = cell_unit(zi, g.oz);
     mrg = 1e-3f + 1e-6f * (fabsf(ux) + fabsf(uy) + fabsf(uz));
     rc = float((R + a.reach) * g.invL) * (1.f + 1e-5f) + mrg;
     home = (DIM >= 2 ? clampc(uy, g.ny) : 0) + (DIM == 3 ? clampc(uz, g.nz) : 0) * g.ny;
@@ -781,7 +786,9 @@ k_neighbours(NeibArgs a) {
           const float sd32 = dist2_f32(pj, pi);
           if ((sd32 < lo_thr && sd32 > 0.f) || sd32 > hi_thr) continue;
           const int32_t q = __float_as_int(pj.w);
-          if (q == k) continue;
+          // (q < 0: the sentinel past the end, which a centre at a NaN
+          // position does not find far away)
+          if (q == k || q < 0) continue;
           ++nexact;
           double d0 = __dadd_rn(a.sx[q], -xi);
           double d1 = __dadd_rn(a.sy[q], -yi);
