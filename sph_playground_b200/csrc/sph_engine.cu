@@ -167,6 +167,48 @@ class DevCache {
   std::map<int, size_t> cached_;
 };
 
+// The small pinned host block of a handle (reductions, counts, plans read
+// back), from a pool: allocating one takes 3 ms here and freeing it 0.8, of
+// the 14 ms that a gradient of a 16,384-particle rollout took, which makes a
+// handle each time.  A block comes back when its handle's streams are idle;
+// at most kMost wait (4 KB each), the others go back to the driver.  Any
+// thread and device may take one (portable).
+class PinnedPool {
+ public:
+  static PinnedPool& get() {
+    static PinnedPool* p = new PinnedPool();  // (never destroyed: handles may outlive statics)
+    return *p;
+  }
+  void* take(size_t bytes) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      if (!free_.empty()) {
+        void* p = free_.back();
+        free_.pop_back();
+        return p;
+      }
+    }
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    return p;
+  }
+  void give(void* p) {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      if (free_.size() < kMost) {
+        free_.push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr size_t kMost = 32;
+  std::mutex mu_;
+  std::vector<void*> free_;
+};
+
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -225,6 +267,7 @@ constexpr int64_t kFewCentres = 65536;
 // fresh searches of a served iterate (centres x widening) as a share of all
 // centres, above which the iterate searches plainly instead
 constexpr double kSkinDirtyShare = 0.15;
+constexpr float kRowSlack = 1.2f;  // room of a list row over its expected count
 
 struct sph_handle {
   int dev = 0;  // the device current at sph_create
@@ -244,7 +287,7 @@ struct sph_handle {
   int64_t nghost = 0;
   // sort + cells
   DevBuf keys, keys_alt, vals, vals_alt, sort_tmp, cstart;
-  DevBuf cell_count, cell_ctr;  // the counting sort's counts and counters
+  DevBuf cell_count;  // the counting sort's counts
   // sorted arrays
   DevBuf sx, sy, sz, s32, ssrc, cflag, cpos, centre_k, centre_p;
   DevBuf hk_s, dk_s, ok_s;
@@ -310,7 +353,15 @@ struct sph_handle {
   int skin_turn = 0;
   bool pos_packed = false;     // the served iterate wrote circuit1's records
   SkinOut* h_skin = nullptr;   // (pinned)
-  int skin_most = 0;           // blocks of k_skin_serve resident at once
+  // cooperative launches: blocks resident at once, scratch, the images' result
+  int coop_cache[COOP_COUNT] = {0};
+  DevBuf coop_part, coop_box, img_out;
+  ImageOut* h_img = nullptr;   // (pinned)
+  int coop_most(int which, int& most) {
+    if (coop_cache[which] <= 0) coop_cache[which] = resident_blocks(which);
+    most = coop_cache[which];
+    return most > 0 ? SPH_OK : fail(SPH_ERR_CUDA, "no cooperative launch on this device");
+  }
   // rows renamed: spare signatures, the two permutations, the old types, a flag
   DevBuf skin_sig_alt, skin_inv, skin_perm, skin_type, skin_flag;
   int64_t skin_nl_size = 0;
@@ -366,7 +417,7 @@ struct sph_handle {
   int est_count = 0;
   // scalars
   DevBuf status, red, dcnt, maxcnt, ctrl, ciso;
-  void* h_pinned = nullptr;             // the block that holds the next three, h_plan and h_skin
+  void* h_pinned = nullptr;             // the block that holds the next three, h_plan, h_skin and h_img
   unsigned long long* h_red = nullptr;  // pinned
   double* h_ctrl = nullptr;             // pinned
   int32_t* h_i32 = nullptr;             // pinned scratch
@@ -481,6 +532,14 @@ struct sph_handle {
     if (nreal >= 12000) return 4;
     if (dim() == 1 || nreal >= 6000) return 8;
     return nreal >= 2000 ? 16 : 32;
+  }
+
+  // circuit2's: in 3D FP32 at least 8, which costs nothing there (128^3: 7.82
+  // against 7.84 ms for 4 steps) and halves a lane's plain FP32 sum
+  int lanes_force() const {
+    const int g = lanes_pair();
+    if (lanes_ok(int(st[SPH_P_LANES_PAIR])) || prec == SPH_PREC_FP64 || dim() != 3) return g;
+    return std::max(g, 8);
   }
 
   int params(Params& P) {
@@ -756,17 +815,19 @@ struct sph_handle {
   // runs `pass` (which fills the table's rows given its NeibArgs) until no
   // row overflows; `exact`: the table the pair passes read (its longest row
   // is reported and checked against the reference's maxneib cap)
-  // pass(na, attempt)
+  // pass(na, attempt); `placed`: the sort has placed the rows for the first attempt
   template <class Pass>
-  int fill_table(const Table& T, const Params& P, bool exact, Pass pass) {
+  int fill_table(const Table& T, const Params& P, bool exact, Pass pass, bool placed = false) {
     const int d = P.dim;
     for (int attempt = 0; attempt < 4; ++attempt) {
       Phase ph(this, SPH_T_NEIGHBOURS);
-      launch_rowcap(nreal, centre_p.as<int32_t>(), orig.as<int32_t>(),
-                    T.count_prev->as<int32_t>(), T.h_prev->as<float>(), col(es_h), d, 1.2f,
-                    T.rowcap64->as<int64_t>(), T.rowcap->as<int32_t>(), s);
-      exclusive_scan64(scan64_tmp.p, scan64_tmp.bytes, T.rowcap64->as<int64_t>(),
-                       T.rowoff->as<int64_t>(), nreal, s);
+      if (attempt > 0 || !placed) {
+        launch_rowcap(nreal, centre_p.as<int32_t>(), orig.as<int32_t>(),
+                      T.count_prev->as<int32_t>(), T.h_prev->as<float>(), col(es_h), d, kRowSlack,
+                      T.rowcap64->as<int64_t>(), T.rowcap->as<int32_t>(), s);
+        exclusive_scan64(scan64_tmp.p, scan64_tmp.bytes, T.rowcap64->as<int64_t>(),
+                         T.rowoff->as<int64_t>(), nreal, s);
+      }
       // (table sizes are multiples of 4 like the rows: a row that fits ends
       // on a 16-byte boundary inside the table)
       if (*T.nl_size <= 0) {
@@ -899,20 +960,14 @@ struct sph_handle {
   int skin_build(const Mode& m, const Params& P, double skin, double hmin) {
     const int d = P.dim;
     const int64_t nall = nrows + nghost;
-    RC(skin_alloc(nall));
     const double kfac = 1.0 + skin;
-    if (skin_est <= 0) {
-      skin_est = int(est_count * std::pow(kfac, double(d))) + 8;
-      launch_fill_i32(skin_count_prev.as<int32_t>(), nrows, skin_est, s);
-      CK(cudaMemsetAsync(skin_h_prev.p, 0, sizeof(float) * nrows, s));
-    }
     const bool staged = st[SPH_P_SEARCH_STAGED] != 0;
     RC(fill_table(skin_table(), P, false, [&](NeibArgs& na, int) {
       na.kfac = kfac;
       na.skin_search = 1;
       launch_neighbours(d, lanes_search(), staged, na, s);
       cnt_host[SPH_CNT_SEARCHES]++;
-    }));
+    }, true));
     {
       Phase ph(this, SPH_T_NEIGHBOURS);
       CK(cudaMemcpyAsync(skin_bx.p, sx.p, sizeof(double) * nall, cudaMemcpyDeviceToDevice, s));
@@ -1097,9 +1152,9 @@ struct sph_handle {
     BoxGeom g = box(m);
     if (!m.ghosts) for (int k = 0; k < 3; ++k) g.periodic[k] = g.reflect[k] = 0;
     const int64_t ncell = int64_t(grid.nx) * grid.ny * grid.nz;
-    if (skin_most <= 0) skin_most = skin_serve_most_blocks();
-    const int blocks = skin_most > 0 ? skin_serve_blocks(nall, skin_most) : 0;
-    if (blocks <= 0) return fail(SPH_ERR_CUDA, "skin lists: no cooperative launch");
+    int most = 0;
+    RC(coop_most(COOP_SERVE, most));
+    const int blocks = coop_blocks(nall, most);
     RC(skin_fcell.ensure(2 * size_t(ncell)));
     RC(skin_mcell.ensure(2 * size_t(ncell)));
     {
@@ -1210,49 +1265,46 @@ struct sph_handle {
     }
     const int d = P.dim;
     BoxGeom g = box(m);
+    if (!m.ghosts) for (int k = 0; k < 3; ++k) g.periodic[k] = g.reflect[k] = 0;
+    int most_images = 0, most_sort = 0;
+    RC(coop_most(COOP_IMAGES, most_images));
+    RC(coop_most(COOP_SORT, most_sort));
+    RC(coop_part.ensure(sizeof(int64_t) * 2 * size_t(std::max(most_images, most_sort))));
     {
       Phase ph(this, SPH_T_GHOSTS);
-      if (m.ghosts) launch_reflect(cols.as<double>(), nrows, nreal, g, s);
-      // reduction slots: lo (min), hi (max), hmin
-      SlotInit si{};
-      for (int k = 0; k < 3; ++k) {
-        si.off[si.n] = RED_LO_X + k; si.val[si.n++] = dkey(1e308);
-        si.off[si.n] = RED_HI_X + k; si.val[si.n++] = dkey(-1e308);
-      }
-      si.off[si.n] = RED_HMIN; si.val[si.n++] = dkey(1e308);
-      launch_init_slots(red.as<unsigned long long>(), si, s);
-      BoxGeom gg = g;
-      if (!m.ghosts) for (int k = 0; k < 3; ++k) gg.periodic[k] = 0;
-      launch_ghost_count(cols.as<double>(), nrows, nreal, gg, d, gcount.as<int32_t>(),
-                         red.as<unsigned long long>(), s);
-      CK(cudaMemsetAsync(gcount.as<int32_t>() + nrows, 0, sizeof(int32_t), s));
-      exclusive_scan(scan_tmp.p, scan_tmp.bytes, gcount.as<int32_t>(), goff.as<int32_t>(),
-                     nrows + 1, s);
-      CK(cudaMemcpyAsync(h_i32, goff.as<int32_t>() + nrows, sizeof(int32_t),
-                         cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(h_red, red.p, sizeof(unsigned long long) * (RED_HMIN + 1),
-                         cudaMemcpyDeviceToHost, s));
+      RC(coop_box.ensure(sizeof(double) * 7 * size_t(most_images)));
+      RC(img_out.ensure(sizeof(ImageOut)));
+      ImageArgs a{};
+      a.cols = cols.as<double>();
+      a.ld = a.nrows = nrows;
+      a.nreal = nreal;
+      a.g = g;
+      a.dim = d;
+      a.wrap = m.ghosts ? 1 : 0;
+      a.goff = goff.as<int32_t>();
+      a.part = coop_part.as<int64_t>();
+      a.box = coop_box.as<double>();
+      a.out = img_out.as<ImageOut>();
+      CK(launch_images(a, coop_blocks(nrows, most_images), s));
+      CK(cudaMemcpyAsync(h_img, img_out.p, sizeof(ImageOut), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
-      nghost = h_i32[0];
+      CK(cudaGetLastError());
+      nghost = h_img->nghost;
       RC(gx.ensure(sizeof(double) * std::max<int64_t>(nghost, 1)));
       RC(gy.ensure(sizeof(double) * std::max<int64_t>(nghost, 1)));
       RC(gz.ensure(sizeof(double) * std::max<int64_t>(nghost, 1)));
       RC(gsrc.ensure(sizeof(int32_t) * std::max<int64_t>(nghost, 1)));
       RC(gcode.ensure(sizeof(int8_t) * std::max<int64_t>(nghost, 1)));
-      if (nghost > 0)
-        launch_ghost_write(cols.as<double>(), nrows, gg, d, goff.as<int32_t>(), gx.as<double>(),
-                           gy.as<double>(), gz.as<double>(), gsrc.as<int32_t>(),
-                           gcode.as<int8_t>(), nullptr, s);
     }
     const int64_t nall = nrows + nghost;
     RC(alloc_all(nall));
     // grid: cell edge krad * h_min * factor, at most 1024 cells per axis
     double lo[3], hi[3];
     for (int k = 0; k < 3; ++k) {
-      lo[k] = dkey_inv(h_red[RED_LO_X + k]);
-      hi[k] = dkey_inv(h_red[RED_HI_X + k]);
+      lo[k] = h_img->lo[k];
+      hi[k] = h_img->hi[k];
     }
-    double hmin = dkey_inv(h_red[RED_HMIN]);
+    double hmin = h_img->hmin;
     if (!(hmin > 0) || !std::isfinite(hmin)) return fail(SPH_ERR_IC_H, "smoothing length <= 0");
     for (int k = 0; k < 3; ++k)
       if (!std::isfinite(lo[k]) || !std::isfinite(hi[k])) return fail(SPH_ERR_Q_NAN, "q is nan");
@@ -1272,8 +1324,6 @@ struct sph_handle {
     grid.ox = lo[0]; grid.oy = lo[1]; grid.oz = lo[2];
     grid.L = L; grid.invL = 1.0 / L;
     grid.nx = n3[0]; grid.ny = n3[1]; grid.nz = n3[2];
-    int end_bit = 1;
-    while ((int64_t(1) << end_bit) < ncell) ++end_bit;
     // FP32 position packing: one binade [2^E, 2^(E+1)) over the whole extent
     // (with skin lists, and room of one search radius on every side for the
     // records to move before the next sort)
@@ -1287,44 +1337,9 @@ struct sph_handle {
     pgeom.ox = lo[0] - mg; pgeom.oy = lo[1] - mg; pgeom.oz = lo[2] - mg;
     pgeom.shift = sh;
     pgeom.mref = mref;
-    {
-      Phase ph(this, SPH_T_SORT);
-      launch_keys(cols.as<double>(), nrows, gx.as<double>(), gy.as<double>(), gz.as<double>(),
-                  nghost, grid, keys.as<uint32_t>(), vals.as<int32_t>(), s);
-      // the cell count follows 1 / h_min^d, which drifts from step to step:
-      // room for four times the current count (at most the cap) keeps the
-      // reallocation out of the steady state
-      const size_t cells = size_t(std::min<int64_t>(4 * (ncell + 1), ncell_cap + 1));
-      if (sizeof(int32_t) * size_t(ncell + 1) > cstart.bytes)
-        RC(cstart.ensure(sizeof(int32_t) * cells));
-      if (sizeof(int32_t) * size_t(ncell + 1) > cell_count.bytes)
-        RC(cell_count.ensure(sizeof(int32_t) * cells));
-      const size_t sb = scan_temp_bytes(ncell + 1);
-      if (sb > scan_tmp.bytes) RC(scan_tmp.ensure(sb));
-      RC(cell_ctr.ensure(2 * sizeof(int32_t)));
-      // counting sort by cell (vals serves as its list of crowded cells);
-      // a cell of more than 4096 records takes the library's radix sort
-      if (!cell_sort(keys.as<uint32_t>(), nall, ncell, cell_count.as<int32_t>(),
-                     cstart.as<int32_t>(), vals_alt.as<int32_t>(), keys_alt.as<uint32_t>(),
-                     vals.as<int32_t>(), cell_ctr.as<int32_t>(), scan_tmp.p, scan_tmp.bytes,
-                     h_i32 + 5, s)) {
-        sort_pairs(sort_tmp.p, sort_tmp.bytes, keys.as<uint32_t>(), keys_alt.as<uint32_t>(),
-                   vals.as<int32_t>(), vals_alt.as<int32_t>(), nall, end_bit, s);
-        launch_cell_starts(keys_alt.as<uint32_t>(), nall, ncell, cstart.as<int32_t>(), s);
-      }
-      launch_sorted_gather(vals_alt.as<int32_t>(), nall, nrows, nreal, cols.as<double>(),
-                           gx.as<double>(), gy.as<double>(), gz.as<double>(), gsrc.as<int32_t>(),
-                           sx.as<double>(), sy.as<double>(), sz.as<double>(), ssrc.as<int32_t>(),
-                           cflag.as<int32_t>(), s32.as<float4>(), pgeom, s);
-      CK(cudaMemsetAsync(cflag.as<int32_t>() + nall, 0, sizeof(int32_t), s));
-      exclusive_scan(scan_tmp.p, scan_tmp.bytes, cflag.as<int32_t>(), cpos.as<int32_t>(),
-                     nall + 1, s);
-      launch_centres(vals_alt.as<int32_t>(), cflag.as<int32_t>(), cpos.as<int32_t>(), nall,
-                     centre_k.as<int32_t>(), centre_p.as<int32_t>(), s);
-    }
-    // neighbour lists: rows sized from each particle's previous count; a row
-    // that overflows (or a table that is too small) re-runs the search with
-    // the counts it just measured
+    // rows sized from each particle's previous count; a row that overflows
+    // (or a table that is too small) re-runs the search with the counts it
+    // just measured
     if (est_count <= 0) {
       double kh = P.krad * P.hfac;
       double est = d == 3 ? 4.0 / 3.0 * kPi * kh * kh * kh : (d == 2 ? kPi * kh * kh : 2 * kh);
@@ -1334,13 +1349,67 @@ struct sph_handle {
       CK(cudaMemsetAsync(h_prev.p, 0, sizeof(float) * nrows, s));
     }
     if (skin > 0) {
+      RC(skin_alloc(nall));
+      if (skin_est <= 0) {
+        skin_est = int(est_count * std::pow(1.0 + skin, double(d))) + 8;
+        launch_fill_i32(skin_count_prev.as<int32_t>(), nrows, skin_est, s);
+        CK(cudaMemsetAsync(skin_h_prev.p, 0, sizeof(float) * nrows, s));
+      }
+    }
+    {
+      Phase ph(this, SPH_T_SORT);
+      // the cell count follows 1 / h_min^d, which drifts from step to step:
+      // room for four times the current count (at most the cap) keeps the
+      // reallocation out of the steady state
+      const size_t cells = size_t(std::min<int64_t>(4 * (ncell + 1), ncell_cap + 1));
+      if (sizeof(int32_t) * size_t(ncell + 1) > cstart.bytes)
+        RC(cstart.ensure(sizeof(int32_t) * cells));
+      if (sizeof(int32_t) * size_t(ncell + 1) > cell_count.bytes)
+        RC(cell_count.ensure(sizeof(int32_t) * cells));
+      const Table T = skin > 0 ? skin_table() : exact_table();
+      SortArgs a{};
+      a.cols = cols.as<double>();
+      a.ld = a.nrows = nrows;
+      a.nreal = nreal;
+      a.nall = nall;
+      a.g = g;
+      a.dim = d;
+      a.goff = goff.as<int32_t>();
+      a.gx = gx.as<double>(); a.gy = gy.as<double>(); a.gz = gz.as<double>();
+      a.gsrc = gsrc.as<int32_t>();
+      a.gcode = gcode.as<int8_t>();
+      a.grid = grid;
+      a.ncell = ncell;
+      a.keys = keys.as<uint32_t>();
+      a.keys_sorted = keys_alt.as<uint32_t>();
+      a.slot = cpos.as<int32_t>();
+      a.members = vals.as<int32_t>();
+      a.count = cell_count.as<int32_t>();
+      a.cstart = cstart.as<int32_t>();
+      a.sidx = vals_alt.as<int32_t>();
+      a.ssrc = ssrc.as<int32_t>();
+      a.sx = sx.as<double>(); a.sy = sy.as<double>(); a.sz = sz.as<double>();
+      a.s32 = s32.as<float4>();
+      a.pg = pgeom;
+      a.centre_k = centre_k.as<int32_t>();
+      a.centre_p = centre_p.as<int32_t>();
+      a.orig = orig.as<int32_t>();
+      a.count_prev = T.count_prev->as<int32_t>();
+      a.h_prev = T.h_prev->as<float>();
+      a.slack = kRowSlack;
+      a.rowcap = T.rowcap->as<int32_t>();
+      a.rowoff = T.rowoff->as<int64_t>();
+      a.part = coop_part.as<int64_t>();
+      CK(launch_sort_records(a, coop_blocks(nall, most_sort), s));
+    }
+    if (skin > 0) {
       RC(skin_build(m, P, skin, hmin));
     } else {
       const bool staged = st[SPH_P_SEARCH_STAGED] != 0;
       RC(fill_table(exact_table(), P, true, [&](NeibArgs& na, int) {
         launch_neighbours(d, lanes_search(), staged, na, s);
         cnt_host[SPH_CNT_SEARCHES]++;
-      }));
+      }, true));
     }
     have_order = true;
     rows_in_order = false;
@@ -1522,7 +1591,7 @@ struct sph_handle {
     C2Args a{};
     a.nc = nreal;
     a.rowoff = rowoff.as<int64_t>();
-    a.G = lanes_pair();
+    a.G = lanes_force();
     a.centre_k = centre_k.as<int32_t>();
     a.centre_p = centre_p.as<int32_t>();
     a.nl = nl.as<int32_t>();
@@ -1796,7 +1865,7 @@ struct sph_handle {
       launch_dskin_built(dskin.as<DevSkin>(), rb, s);
       // the rows filtered from the lists: their last counts
       launch_rowcap(nreal, centre_p.as<int32_t>(), orig.as<int32_t>(), count_prev.as<int32_t>(),
-                    h_prev.as<float>(), col(es_h), d, 1.2f, rowcap64.as<int64_t>(),
+                    h_prev.as<float>(), col(es_h), d, kRowSlack, rowcap64.as<int64_t>(),
                     rowcap.as<int32_t>(), s);
       exclusive_scan64(scan64_tmp.p, scan64_tmp.bytes, rowcap64.as<int64_t>(),
                        rowoff.as<int64_t>(), nreal, s);
@@ -2698,7 +2767,6 @@ struct sph_handle {
     }
     for (auto e : ev_pool) cudaEventDestroy(e);
     drop_graph();
-    if (h_pinned) cudaFreeHost(h_pinned);
     for (auto c : cap_s) cudaStreamDestroy(c);
     for (auto e : xfer_ev) cudaEventDestroy(e);
     if (xs) {
@@ -2706,6 +2774,8 @@ struct sph_handle {
       cudaStreamDestroy(xs);
     }
     if (s) cudaStreamDestroy(s);
+    if (h_pinned) PinnedPool::get().give(h_pinned);  // (both streams were waited for)
+    h_pinned = nullptr;
   }
 };
 
@@ -3066,21 +3136,23 @@ int sph_create(const double* state49, const double* store, int64_t n_rows, int k
     delete h;
     return fail(SPH_ERR_CUDA, "cudaStreamCreate failed");
   }
-  // the handle's small host buffers, one pinned block (a pinned allocation
-  // takes about 0.45 ms, giving it back 0.25 ms)
+  // the handle's small host buffers, one pinned block
   struct Pinned {
     unsigned long long red[RED_TOTAL + 2];
     double ctrl[16];
     DevPlan plan;
     SkinOut skin;
+    ImageOut img;
     int32_t i32[16];
   };
-  if (cudaMallocHost(&h->h_pinned, sizeof(Pinned)) == cudaSuccess) {
+  h->h_pinned = PinnedPool::get().take(sizeof(Pinned));
+  if (h->h_pinned) {
     auto* q = static_cast<Pinned*>(h->h_pinned);
     h->h_red = q->red;
     h->h_ctrl = q->ctrl;
     h->h_plan = &q->plan;
     h->h_skin = &q->skin;
+    h->h_img = &q->img;
     h->h_i32 = q->i32;
   } else {
     cudaGetLastError();

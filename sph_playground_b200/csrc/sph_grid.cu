@@ -321,93 +321,6 @@ __global__ void k_keys(const double* __restrict__ cols, int64_t ld, int64_t nrow
   vals[u] = int32_t(u);
 }
 
-// ---- counting sort of the records by cell ------------------------------------------------
-// The keys are cell indices, so one pass of counting sort orders them: the
-// records of each cell are counted, the counts scanned into the cells'
-// starts, and every record placed at its cell's start plus a slot taken
-// with an atomic.  The slots within a cell come out in arbitrary order;
-// each cell's records are then sorted by index (a thread per cell for up to
-// kCellSmall records, a block per cell for up to kCellBig), which gives the
-// order of a stable sort by key.
-constexpr int kCellSmall = 32;
-constexpr int kCellBig = 4096;
-
-__global__ void k_cell_count(const uint32_t* __restrict__ keys, int64_t n,
-                             int32_t* __restrict__ count, int32_t* __restrict__ maxc) {
-  const int64_t u = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  int m = 0;
-  if (u < n) m = atomicAdd(&count[keys[u]], 1) + 1;
-  unsigned long long v[1] = {(unsigned long long)m};
-  const bool is_max[1] = {true};
-  block_counters<1>(v, is_max);
-  if (threadIdx.x == 0 && v[0]) atomicMax(maxc, int(v[0]));
-}
-__global__ void k_cell_scatter(const uint32_t* __restrict__ keys, int64_t n,
-                               const int32_t* __restrict__ cstart, int32_t* __restrict__ fill,
-                               int32_t* __restrict__ vout, uint32_t* __restrict__ kout) {
-  const int64_t u = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (u >= n) return;
-  const uint32_t key = keys[u];
-  const int32_t pos = cstart[key] + atomicAdd(&fill[key], 1);
-  vout[pos] = int32_t(u);
-  kout[pos] = key;
-}
-// cells of up to kCellSmall records: insertion sort by a thread; larger
-// ones go to `big`
-__global__ void k_cell_sort_small(const int32_t* __restrict__ cstart, int64_t ncell,
-                                  int32_t* __restrict__ v, int32_t* __restrict__ big,
-                                  int32_t* __restrict__ nbig) {
-  const int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (c >= ncell) return;
-  const int32_t a = cstart[c], b = cstart[c + 1];
-  const int k = b - a;
-  if (k <= 1) return;
-  if (k > kCellSmall) {
-    big[atomicAdd(nbig, 1)] = int32_t(c);
-    return;
-  }
-  int32_t r[kCellSmall];
-  for (int i = 0; i < k; ++i) r[i] = v[a + i];
-  for (int i = 1; i < k; ++i) {
-    const int32_t x = r[i];
-    int j = i - 1;
-    while (j >= 0 && r[j] > x) { r[j + 1] = r[j]; --j; }
-    r[j + 1] = x;
-  }
-  for (int i = 0; i < k; ++i) v[a + i] = r[i];
-}
-// cells of up to kCellBig records: a block per cell (the blocks stride over
-// the list), bitonic sort in shared memory padded to a power of two
-__global__ void __launch_bounds__(256)
-k_cell_sort_big(const int32_t* __restrict__ cstart, int32_t* __restrict__ v,
-                const int32_t* __restrict__ big, const int32_t* __restrict__ nbig) {
-  __shared__ int32_t sh[kCellBig];
-  const int nb = *nbig;
-  for (int i = blockIdx.x; i < nb; i += gridDim.x) {
-    const int32_t c = big[i];
-    const int32_t a = cstart[c];
-    const int k = cstart[c + 1] - a;  // kCellSmall < k <= kCellBig (checked on the host)
-    int m = 1;
-    while (m < k) m <<= 1;
-    for (int t = threadIdx.x; t < m; t += blockDim.x) sh[t] = t < k ? v[a + t] : INT32_MAX;
-    __syncthreads();
-    for (int size = 2; size <= m; size <<= 1)
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = threadIdx.x; t < m; t += blockDim.x) {
-          const int o = t ^ stride;
-          if (o > t) {
-            const bool up = (t & size) == 0;
-            const int32_t x = sh[t], y = sh[o];
-            if ((x > y) == up) { sh[t] = y; sh[o] = x; }
-          }
-        }
-        __syncthreads();
-      }
-    for (int t = threadIdx.x; t < k; t += blockDim.x) v[a + t] = sh[t];
-    __syncthreads();
-  }
-}
-
 // cstart[c] = number of particles in cells before c (ncell + 1 entries), from
 // the sorted keys: each key change fills the empty cells it skips.
 __global__ void k_cell_starts(const uint32_t* __restrict__ keys, int64_t n, int64_t ncell,
@@ -975,6 +888,290 @@ k_neighbours(NeibArgs a) {
   }
 }
 
+// Row capacity of a centre's neighbour list: the particle's count from the
+// previous search, scaled by (h / h_then)^dim for the change of its search
+// radius since, plus 20% and 8 slots of slack (or the initial estimate, which
+// comes with h_then = 0); a multiple of 4, so that every row starts on a
+// 16-byte boundary.
+__device__ __forceinline__ int row_capacity(int32_t p, const int32_t* orig,
+                                            const int32_t* count_prev, const float* h_prev,
+                                            const double* hcol, int dim, float slack) {
+  const int32_t o = orig[p];
+  float est = float(count_prev[o]);
+  const float hp = h_prev[o];
+  if (hp > 0.f) {
+    float g = float(hcol[p]) / hp;
+    g = fminf(fmaxf(g, 0.5f), 4.f);
+    est *= dim == 3 ? g * g * g : (dim == 2 ? g * g : g);
+  }
+  return (int(fminf(est * slack, 1.0e9f)) + 8 + 3) & ~3;
+}
+
+// ---- images, sort and rows of a plain search, two cooperative launches -----------------------
+// What comes before a search is a chain of short passes over the rows,
+// images, cells and records, each needing a total or a prefix of the one
+// before.  As 20 launches with three library scans and two waits of the host
+// it took 0.13 ms of a 16,384-particle iterate whose search takes 0.03; as
+// the phases of two launches, between grid barriers, with one wait (for the
+// image count, which sizes the buffers), 0.06.  At 128^3 (bound by scattered
+// reads and writes) they take 0.30 ms, as the chain did; 4 blocks per SM
+// instead of 8 / 6 took 0.36.
+
+// exclusive prefix of v over the block's TPB threads, and their total
+template <class T>
+__device__ __forceinline__ T block_prefix(T v, T& total) {
+  __shared__ T sums[TPB / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const T t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  __syncthreads();  // (the last call's sums have been read)
+  if (lane == 31) sums[w] = incl;
+  __syncthreads();
+  T base = 0;
+  total = 0;
+#pragma unroll
+  for (int i = 0; i < TPB / 32; ++i) {
+    if (i < w) base += sums[i];
+    total += sums[i];
+  }
+  return base + incl - v;
+}
+// sum over the block, on every thread
+template <class T>
+__device__ __forceinline__ T block_total(T v) {
+  T total;
+  block_prefix<T>(v, total);
+  return total;
+}
+// this block's share [b0, b1) of n items in whole tiles of TPB, in block order
+__device__ __forceinline__ void block_share(int64_t n, int64_t& b0, int64_t& b1) {
+  const int64_t chunk = ((n + gridDim.x - 1) / gridDim.x + TPB - 1) / TPB * TPB;
+  b0 = min(n, blockIdx.x * chunk);
+  b1 = min(n, b0 + chunk);
+}
+// sum of part[0 .. blockIdx.x - 1] (written before a grid barrier), on every thread
+__device__ __forceinline__ int64_t sum_before(const int64_t* part) {
+  int64_t v = 0;
+  for (int b = threadIdx.x; b < int(blockIdx.x); b += TPB) v += __ldcg(part + b);
+  return block_total<int64_t>(v);
+}
+
+// The wrap into the box, every row's images counted and their places, the
+// bounding box of rows and images and the smallest h of the real rows.
+__global__ void __launch_bounds__(TPB, 6) k_images(ImageArgs a) {
+  auto grid = cooperative_groups::this_grid();
+  // slots: lo x, y, z (min), hi x, y, z (max), hmin (min)
+  double v[7] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300, 1e300};
+  const bool is_max[7] = {false, false, false, true, true, true, false};
+  int64_t b0, b1;
+  block_share(a.nrows, b0, b1);
+  int64_t mine = 0;
+  for (int64_t i = b0 + threadIdx.x; i < b1; i += TPB) {
+    double r[3];
+    for (int k = 0; k < 3; ++k) {
+      double& x = a.cols[(es_rx + k) * a.ld + i];
+      r[k] = x;
+      if (a.wrap && i < a.nreal && a.g.reflect[k]) {
+        r[k] = reflect_coord(r[k], a.g.emin[k], a.g.emax[k]);
+        x = r[k];
+      }
+      v[k] = fmin(v[k], r[k]);
+      v[3 + k] = fmax(v[3 + k], r[k]);
+    }
+    if (i < a.nreal) v[6] = fmin(v[6], a.cols[es_h * a.ld + i]);
+    int c = 0;
+    if (ghost_source(a.cols[es_type * a.ld + i])) {
+      const AxisSigns sg_ = axis_signs(r, a.g, a.dim);
+      for (int mask = 1; mask < 8; ++mask) {
+        int sg[3];
+        if (!image_of(sg_, mask, sg)) continue;
+        ++c;
+        for (int k = 0; k < 3; ++k) {
+          const double x = image_coord(r[k], sg[k], a.g.emin[k], a.g.emax[k]);
+          v[k] = fmin(v[k], x);
+          v[3 + k] = fmax(v[3 + k], x);
+        }
+      }
+    }
+    a.goff[i] = c;
+    mine += c;
+  }
+  mine = block_total<int64_t>(mine);
+  block_minmax<7>(v, is_max);
+  if (threadIdx.x == 0) {
+    a.part[blockIdx.x] = mine;
+    for (int k = 0; k < 7; ++k) a.box[k * gridDim.x + blockIdx.x] = v[k];
+  }
+  grid.sync();
+  int64_t base = sum_before(a.part);
+  for (int64_t t = b0; t < b1; t += TPB) {
+    const int64_t i = t + threadIdx.x;
+    const int c = i < b1 ? a.goff[i] : 0;
+    int total;
+    const int at = block_prefix<int>(c, total);
+    if (i < b1) a.goff[i] = int32_t(base + at);
+    base += total;
+  }
+  if (blockIdx.x != gridDim.x - 1) return;
+  // the last block (its base is the image count) reports
+  double w[7] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300, 1e300};
+  for (int b = threadIdx.x; b < int(gridDim.x); b += TPB)
+    for (int k = 0; k < 7; ++k) {
+      const double x = __ldcg(a.box + k * gridDim.x + b);
+      w[k] = is_max[k] ? fmax(w[k], x) : fmin(w[k], x);
+    }
+  __syncthreads();
+  block_minmax<7>(w, is_max);
+  if (threadIdx.x == 0) {
+    ImageOut o{};
+    o.nghost = base;
+    for (int k = 0; k < 3; ++k) { o.lo[k] = w[k]; o.hi[k] = w[3 + k]; }
+    o.hmin = w[6];
+    *a.out = o;
+  }
+}
+
+// The images written, the records (rows, then images) sorted by cell, each
+// cell's in increasing record index; their sorted positions and FP32 images;
+// the centres (real rows) in sorted order with their list rows' capacities
+// and places (as k_rowcap and a scan of its capacities).
+__global__ void __launch_bounds__(TPB, 8) k_sort_records(SortArgs a) {
+  auto grid = cooperative_groups::this_grid();
+  const int64_t first = blockIdx.x * int64_t(TPB) + threadIdx.x, step = int64_t(gridDim.x) * TPB;
+  for (int64_t i = first; i < a.ncell; i += step) a.count[i] = 0;
+  if (a.nall > a.nrows) {
+    for (int64_t i = first; i < a.nrows; i += step) {
+      if (!ghost_source(a.cols[es_type * a.ld + i])) continue;
+      const double r[3] = {a.cols[es_rx * a.ld + i], a.cols[es_ry * a.ld + i],
+                           a.cols[es_rz * a.ld + i]};
+      const AxisSigns s = axis_signs(r, a.g, a.dim);
+      int64_t o = a.goff[i];
+      for (int mask = 1; mask < 8; ++mask) {
+        int sg[3];
+        if (!image_of(s, mask, sg)) continue;
+        a.gx[o] = image_coord(r[0], sg[0], a.g.emin[0], a.g.emax[0]);
+        a.gy[o] = image_coord(r[1], sg[1], a.g.emin[1], a.g.emax[1]);
+        a.gz[o] = image_coord(r[2], sg[2], a.g.emin[2], a.g.emax[2]);
+        a.gsrc[o] = int32_t(i);
+        a.gcode[o] = int8_t((sg[0] + 1) + 3 * (sg[1] + 1) + 9 * (sg[2] + 1));
+        ++o;
+      }
+    }
+  }
+  grid.sync();
+  auto position = [&](int64_t u, double& x, double& y, double& z) {
+    if (u < a.nrows) {
+      x = a.cols[es_rx * a.ld + u]; y = a.cols[es_ry * a.ld + u]; z = a.cols[es_rz * a.ld + u];
+    } else {
+      const int64_t q = u - a.nrows;
+      x = a.gx[q]; y = a.gy[q]; z = a.gz[q];
+    }
+  };
+  // keys, and a slot of the cell for each record in the order the atomics come
+  for (int64_t u = first; u < a.nall; u += step) {
+    double x, y, z;
+    position(u, x, y, z);
+    const uint32_t cx = cell_coord(x, a.grid.ox, a.grid.invL, a.grid.nx);
+    const uint32_t cy = cell_coord(y, a.grid.oy, a.grid.invL, a.grid.ny);
+    const uint32_t cz = cell_coord(z, a.grid.oz, a.grid.invL, a.grid.nz);
+    const uint32_t key = cx + uint32_t(a.grid.nx) * (cy + uint32_t(a.grid.ny) * cz);
+    a.keys[u] = key;
+    a.slot[u] = atomicAdd(a.count + key, 1);
+  }
+  grid.sync();
+  // the cells' starts
+  int64_t b0, b1;
+  block_share(a.ncell, b0, b1);
+  {
+    int64_t mine = 0;
+    for (int64_t i = b0 + threadIdx.x; i < b1; i += TPB) mine += a.count[i];
+    mine = block_total<int64_t>(mine);
+    if (threadIdx.x == 0) a.part[blockIdx.x] = mine;
+  }
+  grid.sync();
+  {
+    int64_t base = sum_before(a.part);
+    for (int64_t t = b0; t < b1; t += TPB) {
+      const int64_t i = t + threadIdx.x;
+      int total;
+      const int at = block_prefix<int>(i < b1 ? a.count[i] : 0, total);
+      if (i < b1) a.cstart[i] = int32_t(base + at);
+      base += total;
+    }
+    if (first == 0) a.cstart[a.ncell] = int32_t(a.nall);
+  }
+  grid.sync();
+  for (int64_t u = first; u < a.nall; u += step)
+    a.members[a.cstart[a.keys[u]] + a.slot[u]] = int32_t(u);
+  grid.sync();
+  // a record's place in its cell: the members of smaller index come first
+  // (cells hold a few records; a crowded one costs its square, as it does
+  // the search)
+  for (int64_t q = first; q < a.nall; q += step) {
+    const int32_t u = a.members[q];
+    const uint32_t key = a.keys[u];
+    const int32_t s = a.cstart[key], e = a.cstart[key + 1];
+    int32_t k = s;
+    for (int32_t i = s; i < e; ++i) k += a.members[i] < u ? 1 : 0;
+    a.sidx[k] = u;
+    a.keys_sorted[k] = key;
+    double x, y, z;
+    position(u, x, y, z);
+    a.ssrc[k] = u < a.nrows ? u : a.gsrc[u - a.nrows];
+    a.sx[k] = x; a.sy[k] = y; a.sz[k] = z;
+    // FP32 image of the position, one binade for the whole extent (see
+    // PackGeom); w carries the record's own sorted index, so that a copy of a
+    // run of records still knows where each came from
+    a.s32[k] = make_float4(__double2float_rn((x - a.pg.ox) + a.pg.shift),
+                           __double2float_rn((y - a.pg.oy) + a.pg.shift),
+                           __double2float_rn((z - a.pg.oz) + a.pg.shift), __int_as_float(k));
+  }
+  grid.sync();
+  block_share(a.nall, b0, b1);
+  {
+    int64_t centres = 0, slots = 0;
+    for (int64_t k = b0 + threadIdx.x; k < b1; k += TPB) {
+      const int32_t p = a.sidx[k];
+      if (p >= a.nreal) continue;
+      ++centres;
+      slots += row_capacity(p, a.orig, a.count_prev, a.h_prev, a.cols + es_h * a.ld, a.dim, a.slack);
+    }
+    centres = block_total<int64_t>(centres);
+    slots = block_total<int64_t>(slots);
+    if (threadIdx.x == 0) {
+      a.part[blockIdx.x] = centres;
+      a.part[gridDim.x + blockIdx.x] = slots;
+    }
+  }
+  grid.sync();
+  int64_t cbase = sum_before(a.part), sbase = sum_before(a.part + gridDim.x);
+  for (int64_t t = b0; t < b1; t += TPB) {
+    const int64_t k = t + threadIdx.x;
+    const int32_t p = k < b1 ? a.sidx[k] : INT32_MAX;
+    const bool on = int64_t(p) < a.nreal;
+    const int cap = on ? row_capacity(p, a.orig, a.count_prev, a.h_prev, a.cols + es_h * a.ld, a.dim,
+                                      a.slack)
+                       : 0;
+    int ctotal;
+    int64_t stotal;
+    const int cat = block_prefix<int>(on ? 1 : 0, ctotal);
+    const int64_t sat = block_prefix<int64_t>(cap, stotal);
+    if (on) {
+      const int64_t c = cbase + cat;
+      a.centre_k[c] = int32_t(k);
+      a.centre_p[c] = p;
+      a.rowcap[c] = cap;
+      a.rowoff[c] = sbase + sat;
+    }
+    cbase += ctotal;
+    sbase += stotal;
+  }
+}
+
 // ---- skin lists (SPH_P_SKIN) -------------------------------------------------------------
 // A search of radius kfac krad h (kfac = 1 + s) at step b leaves each centre
 // its skin list: every record within that radius at b.  At a later step t
@@ -1167,7 +1364,8 @@ __device__ __forceinline__ void skin_slots_clear(unsigned long long* red, int32_
 // of centres that act on theirs, as the phases of one cooperative launch
 // (grid barriers in between) with one result for the host.  As 20 launches
 // and clears, with a scan, these took 45 us of the 225 us of a step of 1,024
-// particles, whose data passes in 5.  NA_SERVE
+// particles, whose data passes in 5; in one, 15.  (6 blocks per SM: at 128^3 0.24 ms a
+// launch, 4 blocks 0.27.)
 //
 // Marks at the level of cells: a record that moved more than eps flags the
 // cell it was sorted into (its position at b), one that moved more than tau
@@ -1252,7 +1450,7 @@ __device__ __forceinline__ uint8_t skin_way(const SkinServe& a, int64_t c, const
   return 0;
 }
 
-__global__ void __launch_bounds__(TPB) k_skin_serve(SkinServe a) {
+__global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
   auto grid = cooperative_groups::this_grid();
   const int64_t first = blockIdx.x * int64_t(TPB) + threadIdx.x, step = int64_t(gridDim.x) * TPB;
   unsigned long long* const red = a.r.red;
@@ -1804,10 +2002,6 @@ __global__ void __launch_bounds__(128) k_search_few(FewArgs a) {
   }
 }
 
-// Row capacity of each centre's neighbour list: the particle's count from
-// the previous search, scaled by (h / h_then)^dim for the change of its
-// search radius since, plus 20% and 8 slots of slack (or the initial
-// estimate, which comes with h_then = 0).
 __global__ void k_rowcap(int64_t nc, const int32_t* __restrict__ centre_p,
                          const int32_t* __restrict__ orig, const int32_t* __restrict__ count_prev,
                          const float* __restrict__ h_prev, const double* __restrict__ hcol,
@@ -1815,17 +2009,7 @@ __global__ void k_rowcap(int64_t nc, const int32_t* __restrict__ centre_p,
                          int32_t* __restrict__ rowcap) {
   int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
   if (c >= nc) return;
-  const int32_t p = centre_p[c];
-  const int32_t o = orig[p];
-  float est = float(count_prev[o]);
-  const float hp = h_prev[o];
-  if (hp > 0.f) {
-    float g = float(hcol[p]) / hp;
-    g = fminf(fmaxf(g, 0.5f), 4.f);
-    est *= dim == 3 ? g * g * g : (dim == 2 ? g * g : g);
-  }
-  // a multiple of 4, so that every row starts on a 16-byte boundary
-  const int cap = (int(fminf(est * slack, 1.0e9f)) + 8 + 3) & ~3;
+  const int cap = row_capacity(centre_p[c], orig, count_prev, h_prev, hcol, dim, slack);
   rowcap[c] = cap;
   rowcap64[c] = cap;
 }
@@ -2400,25 +2584,11 @@ void launch_ghost_count(const double* cols, int64_t nrows, int64_t nreal, BoxGeo
                                                      red);
   note_launch();
 }
-void launch_ghost_write(const double* cols, int64_t nrows, BoxGeom g, int dim,
-                        const int32_t* offset, double* gx, double* gy, double* gz,
-                        int32_t* gsrc, int8_t* gcode, unsigned long long*, cudaStream_t s) {
-  k_ghost_write<<<nblocks(nrows), TPB, 0, s>>>(cols, nrows, nrows, g, dim, offset, INT64_MAX, gx,
-                                               gy, gz, gsrc, gcode);
-  note_launch();
-}
 void launch_ghost_write_cap(const double* cols, int64_t nrows, BoxGeom g, int dim,
                             const int32_t* offset, int64_t cap, double* gx, double* gy,
                             double* gz, int32_t* gsrc, int8_t* gcode, cudaStream_t s) {
   k_ghost_write<<<nblocks(nrows), TPB, 0, s>>>(cols, nrows, nrows, g, dim, offset, cap, gx, gy, gz,
                                                gsrc, gcode);
-  note_launch();
-}
-void launch_keys(const double* cols, int64_t nrows, const double* gx, const double* gy,
-                 const double* gz, int64_t nghost, Grid g, uint32_t* keys, int32_t* vals,
-                 cudaStream_t s) {
-  k_keys<<<nblocks(nrows + nghost), TPB, 0, s>>>(cols, nrows, nrows, gx, gy, gz, nghost, g,
-                                                 keys, vals, nullptr, 0);
   note_launch();
 }
 void launch_keys_dev(const double* cols, int64_t nrows, const double* gx, const double* gy,
@@ -2428,24 +2598,9 @@ void launch_keys_dev(const double* cols, int64_t nrows, const double* gx, const 
                                        ncap);
   note_launch();
 }
-void launch_cell_starts(const uint32_t* keys, int64_t n, int64_t ncell, int32_t* cstart,
-                        cudaStream_t s) {
-  k_cell_starts<<<nblocks(n + 1), TPB, 0, s>>>(keys, n, ncell, cstart, nullptr);
-  note_launch();
-}
 void launch_cell_starts_dev(const uint32_t* keys, int64_t ncap, const DevPlan* plan,
                             int32_t* cstart, cudaStream_t s) {
   k_cell_starts<<<nblocks(ncap + 1), TPB, 0, s>>>(keys, ncap, 0, cstart, plan);
-  note_launch();
-}
-void launch_sorted_gather(const int32_t* sidx, int64_t n, int64_t nrows, int64_t nreal,
-                          const double* cols, const double* gx, const double* gy,
-                          const double* gz, const int32_t* gsrc, double* sx, double* sy,
-                          double* sz, int32_t* ssrc, int32_t* centre_slot, float4* s32,
-                          PackGeom pg, cudaStream_t s) {
-  k_sorted_gather<<<nblocks(n), TPB, 0, s>>>(sidx, n, nrows, nreal, cols, nrows, gx, gy, gz,
-                                             gsrc, sx, sy, sz, ssrc, centre_slot, s32, pg,
-                                             nullptr, 0);
   note_launch();
 }
 void launch_sorted_gather_dev(const int32_t* sidx, int64_t ncap, int64_t nrows, int64_t nreal,
@@ -2514,27 +2669,39 @@ void launch_skin_refresh(const SkinRefresh& r, int64_t n, cudaStream_t s, const 
   k_skin_refresh<<<reduce_blocks(n), TPB, 0, s>>>(r, n, PackGeom{}, plan, gate);
   note_launch();
 }
-int skin_serve_most_blocks() {
+int resident_blocks(int which) {
   int dev = 0, sms = 0, per_sm = 0;
+  const void* f = which == COOP_SERVE ? reinterpret_cast<const void*>(k_skin_serve)
+                  : which == COOP_IMAGES ? reinterpret_cast<const void*>(k_images)
+                                         : reinterpret_cast<const void*>(k_sort_records);
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_skin_serve, TPB, 0) != cudaSuccess)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, TPB, 0) != cudaSuccess)
     return 0;
   return sms * per_sm;
 }
-int skin_serve_blocks(int64_t n, int most) {
+int coop_blocks(int64_t n, int most) {
   return int(std::min<int64_t>(most, std::max<int64_t>(1, (n + TPB - 1) / TPB)));
+}
+template <class A>
+static cudaError_t launch_coop(const void* f, const A& a, int blocks, cudaStream_t s) {
+  A arg = a;
+  void* args[] = {&arg};
+  note_launch();
+  return cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(TPB), args, 0, s);
+}
+cudaError_t launch_images(const ImageArgs& a, int blocks, cudaStream_t s) {
+  return launch_coop(reinterpret_cast<const void*>(k_images), a, blocks, s);
+}
+cudaError_t launch_sort_records(const SortArgs& a, int blocks, cudaStream_t s) {
+  return launch_coop(reinterpret_cast<const void*>(k_sort_records), a, blocks, s);
 }
 void launch_skin_slots_clear(unsigned long long* red, int32_t* counts, cudaStream_t s) {
   k_skin_slots_clear<<<1, 1, 0, s>>>(red, counts);
   note_launch();
 }
 cudaError_t launch_skin_serve(const SkinServe& a, int blocks, cudaStream_t s) {
-  SkinServe arg = a;
-  void* args[] = {&arg};
-  note_launch();
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_skin_serve), dim3(blocks),
-                                     dim3(TPB), args, 0, s);
+  return launch_coop(reinterpret_cast<const void*>(k_skin_serve), a, blocks, s);
 }
 
 // ---- skin lists of the device-resident step ---------------------------------------------
@@ -2885,27 +3052,6 @@ void launch_set_col(double* col, int64_t n, double v, cudaStream_t s) {
   note_launch();
 }
 
-bool cell_sort(const uint32_t* keys, int64_t n, int64_t ncell, int32_t* count, int32_t* cstart,
-               int32_t* vout, uint32_t* kout, int32_t* big, int32_t* ctr, void* scan_tmp,
-               size_t scan_bytes, int32_t* h_ctr, cudaStream_t s) {
-  // ctr[0]: the largest cell, ctr[1]: cells for the block sort
-  cudaMemsetAsync(count, 0, sizeof(int32_t) * size_t(ncell + 1), s);
-  cudaMemsetAsync(ctr, 0, 2 * sizeof(int32_t), s);
-  if (n > 0) k_cell_count<<<nblocks(n), TPB, 0, s>>>(keys, n, count, ctr);
-  cudaMemcpyAsync(h_ctr, ctr, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
-  note_launch();
-  if (h_ctr[0] > kCellBig) return false;  // (nothing written)
-  exclusive_scan(scan_tmp, scan_bytes, count, cstart, ncell + 1, s);
-  cudaMemsetAsync(count, 0, sizeof(int32_t) * size_t(ncell), s);
-  if (n > 0) k_cell_scatter<<<nblocks(n), TPB, 0, s>>>(keys, n, cstart, count, vout, kout);
-  if (h_ctr[0] > 1) {
-    k_cell_sort_small<<<nblocks(ncell), TPB, 0, s>>>(cstart, ncell, vout, big, ctr + 1);
-    if (h_ctr[0] > kCellSmall) k_cell_sort_big<<<148 * 4, 256, 0, s>>>(cstart, vout, big, ctr + 1);
-  }
-  note_launch(3);
-  return true;
-}
 size_t sort_temp_bytes(int64_t n) {
   size_t b = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, b, (const uint32_t*)nullptr, (uint32_t*)nullptr,

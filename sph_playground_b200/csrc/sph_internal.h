@@ -136,14 +136,6 @@ void launch_reorder(const double* cols_in, double* cols_out, const int32_t* orig
 void launch_reflect(double* cols, int64_t ld, int64_t nreal, BoxGeom g, cudaStream_t s);
 void launch_ghost_count(const double* cols, int64_t nrows, int64_t nreal, BoxGeom g,
                         int dim, int32_t* count, unsigned long long* red, cudaStream_t s);
-void launch_ghost_write(const double* cols, int64_t nrows, BoxGeom g, int dim,
-                        const int32_t* offset, double* gx, double* gy, double* gz,
-                        int32_t* gsrc, int8_t* gcode, unsigned long long* red, cudaStream_t s);
-void launch_keys(const double* cols, int64_t nrows, const double* gx, const double* gy,
-                 const double* gz, int64_t nghost, Grid g, uint32_t* keys, int32_t* vals,
-                 cudaStream_t s);
-void launch_cell_starts(const uint32_t* keys, int64_t n, int64_t ncell, int32_t* cstart,
-                        cudaStream_t s);
 struct PackGeom {
   double ox, oy, oz;  // origin subtracted before the binade shift
   double shift;       // 2^E with every (x - origin) in [0, 2^E)
@@ -256,13 +248,58 @@ void launch_sorted_gather_dev(const int32_t* sidx, int64_t ncap, int64_t nrows, 
 void launch_ghost_write_cap(const double* cols, int64_t nrows, BoxGeom g, int dim,
                             const int32_t* offset, int64_t cap, double* gx, double* gy,
                             double* gz, int32_t* gsrc, int8_t* gcode, cudaStream_t s);
-void launch_sorted_gather(const int32_t* sidx, int64_t n, int64_t nrows, int64_t nreal,
-                          const double* cols, const double* gx, const double* gy,
-                          const double* gz, const int32_t* gsrc, double* sx, double* sy,
-                          double* sz, int32_t* ssrc, int32_t* centre_slot, float4* s32,
-                          PackGeom pg, cudaStream_t s);
 void launch_centres(const int32_t* sidx, const int32_t* flag, const int32_t* pos, int64_t n,
                     int32_t* centre_k, int32_t* centre_p, cudaStream_t s);
+// ---- cooperative launches (sph_grid.cu): every block resident at once ----
+enum CoopKernel : int { COOP_SERVE, COOP_IMAGES, COOP_SORT, COOP_COUNT };
+int resident_blocks(int which);            // blocks the current device holds; 0: a runtime error
+int coop_blocks(int64_t n, int most);      // blocks for n items
+// the wrap, every row's images counted and placed (goff), the bounding box
+// of rows and images and the smallest h
+struct ImageOut {
+  int64_t nghost;
+  double lo[3], hi[3], hmin;
+};
+struct ImageArgs {
+  double* cols;
+  int64_t ld, nrows, nreal;
+  BoxGeom g;
+  int dim, wrap;
+  int32_t* goff;
+  int64_t* part;  // 2 entries per block
+  double* box;    // 7 per block
+  ImageOut* out;
+};
+cudaError_t launch_images(const ImageArgs& a, int blocks, cudaStream_t s);
+// images written, records sorted by cell (a stable sort's order), centres and
+// the places of their list rows (see sph_grid.cu)
+struct SortArgs {
+  const double* cols;
+  int64_t ld, nrows, nreal, nall;
+  BoxGeom g;
+  int dim;
+  const int32_t* goff;
+  double *gx, *gy, *gz;
+  int32_t* gsrc;
+  int8_t* gcode;
+  Grid grid;
+  int64_t ncell;
+  uint32_t *keys, *keys_sorted;
+  int32_t *slot, *members, *count, *cstart, *sidx, *ssrc;
+  double *sx, *sy, *sz;
+  float4* s32;
+  PackGeom pg;
+  int32_t *centre_k, *centre_p;
+  // the table the search fills
+  const int32_t* orig;
+  const int32_t* count_prev;
+  const float* h_prev;
+  float slack;
+  int32_t* rowcap;
+  int64_t* rowoff;
+  int64_t* part;  // 2 entries per block
+};
+cudaError_t launch_sort_records(const SortArgs& a, int blocks, cudaStream_t s);
 struct NeibArgs {
   const DevPlan* plan;  // if set: grid and shift from the device plan
   int64_t nc;
@@ -398,10 +435,6 @@ struct SkinServe {
   int32_t* flags;          // longest row, overflow (cleared)
   SkinOut* out;
 };
-// the blocks of k_skin_serve that the current device holds at once (0: an
-// error of the runtime), and those for n records
-int skin_serve_most_blocks();
-int skin_serve_blocks(int64_t n, int most);
 void launch_skin_slots_clear(unsigned long long* red, int32_t* counts, cudaStream_t s);
 cudaError_t launch_skin_serve(const SkinServe& a, int blocks, cudaStream_t s);
 // with the lists live, per centre: can its row come from its skin list?
@@ -592,15 +625,6 @@ void launch_check_rows(const double* cols, int64_t nrows, unsigned long long* ba
 void launch_set_col(double* col, int64_t n, double v, cudaStream_t s);
 
 // CUB wrappers (sph_grid.cu)
-// Counting sort of the records by cell (keys in [0, ncell)): vout / kout the
-// record indices and keys in key order, each cell's records in increasing
-// index (as a stable sort), cstart[0 .. ncell] the cells' starts; count
-// (ncell + 1) and big (ncell) are scratch, ctr two device ints, h_ctr a
-// pinned host int; scan_tmp sized for ncell + 1 entries.  Returns false
-// (nothing written) when a cell holds more than 4096 records.
-bool cell_sort(const uint32_t* keys, int64_t n, int64_t ncell, int32_t* count, int32_t* cstart,
-               int32_t* vout, uint32_t* kout, int32_t* big, int32_t* ctr, void* scan_tmp,
-               size_t scan_bytes, int32_t* h_ctr, cudaStream_t s);
 size_t sort_temp_bytes(int64_t n);
 void sort_pairs(void* tmp, size_t tmp_bytes, const uint32_t* kin, uint32_t* kout,
                 const int32_t* vin, int32_t* vout, int64_t n, int end_bit, cudaStream_t s);
