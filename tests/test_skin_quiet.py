@@ -35,8 +35,8 @@ def test_rows_kept_after_the_guess(engine_lib, oracle_lib, cuda_ok, dim, n, prec
     st, store = _guessed(n, dim)
     cnt, _ = _split_run(engine_lib, oracle_lib, st, store, prec, nsteps=4)
     assert cnt["skin_reuses"] >= 4
-    # 3D, 178 neighbours: a fifteenth of the rows has a record within 4 eps of
-    # its sphere (eps 1e-5 of the radius) plus the measuring bounds, and the
+    # 3D, 178 neighbours: few rows have a record within 4 eps of their
+    # sphere plus the measuring bounds; the
     # hot particle's surroundings (14 spacings of 32) are not kept
     assert cnt["skin_kept"] > 0.6 * (cnt["skin_reuses"] - 1) * n ** dim, cnt
 
