@@ -30,15 +30,14 @@ template <> struct PosAccess<double> {
   using Pos = PairPos<double>;
   static __device__ __forceinline__ double unit(const PackBufs&) { return 1.0; }
   static __device__ __forceinline__ PairPos<double> load(const PackBufs& pb, int64_t j, double& m) {
-    double2 a = __ldg(&pb.p[0][j]);
-    double2 b = __ldg(&pb.p[1][j]);
-    m = b.y;
+    const Rec64 a = ld_rec(&pb.d[0][j]);
+    m = a.b.y;
     PairPos<double> r;
-    r.x = a.x; r.y = a.y; r.z = b.x;
+    r.x = a.a.x; r.y = a.a.y; r.z = a.b.x;
     return r;
   }
   static __device__ __forceinline__ double temp(const PackBufs& pb, int64_t j) {
-    return __ldg(&pb.p[6][j]).y;
+    return __ldg(&pb.vt[j]).y;
   }
 };
 template <> struct PosAccess<float> {

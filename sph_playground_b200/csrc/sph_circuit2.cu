@@ -50,23 +50,22 @@ template <class R> struct PartX {
 template <class R> struct Loader;
 template <> struct Loader<double> {
   static __device__ __forceinline__ void hydro(const PackBufs& pb, int64_t j, Part<double>& o) {
-    double2 a = __ldg(&pb.p[0][j]), b = __ldg(&pb.p[1][j]), c = __ldg(&pb.p[2][j]),
-            d = __ldg(&pb.p[3][j]), e = __ldg(&pb.p[4][j]), f = __ldg(&pb.p[5][j]),
-            g = __ldg(&pb.p[6][j]);
-    o.pos.x = a.x; o.pos.y = a.y; o.pos.z = b.x; o.m = b.y;
-    o.invh = c.x; o.hrho = c.y; o.rho = 2.0 * c.y; o.Pi = d.x; o.P = d.y; o.ac = e.x; o.u = e.y;
-    o.vx = f.x; o.vy = f.y; o.vz = g.x;
+    const Rec64 a = ld_rec(&pb.d[0][j]), c = ld_rec(&pb.d[1][j]), e = ld_rec(&pb.d[2][j]);
+    o.vz = __ldg(&pb.vt[j].x);
+    o.pos.x = a.a.x; o.pos.y = a.a.y; o.pos.z = a.b.x; o.m = a.b.y;
+    o.invh = c.a.x; o.hrho = c.a.y; o.rho = 2.0 * c.a.y; o.Pi = c.b.x; o.P = c.b.y;
+    o.ac = e.a.x; o.u = e.a.y; o.vx = e.b.x; o.vy = e.b.y;
   }
   // (what a mode does not use is not read)
   template <int MODE>
   static __device__ __forceinline__ void extra(const PackBufs& pb, int64_t j, PartX<double>& o) {
-    if constexpr (MODE != C2_MHD) o.T = __ldg(&pb.p[6][j]).y;
+    if constexpr (MODE != C2_MHD) o.T = __ldg(&pb.vt[j].y);
     if constexpr (MODE == C2_TWO_NW || MODE == C2_GENERAL) {
-      const double2 h = __ldg(&pb.p[7][j]), i = __ldg(&pb.p[8][j]);
-      o.kappa = h.x; o.gx = h.y; o.gy = i.x; o.gz = i.y;
+      const Rec64 h = ld_rec(&pb.d[3][j]);
+      o.kappa = h.a.x; o.gx = h.a.y; o.gy = h.b.x; o.gz = h.b.y;
     }
-    const double2 k = __ldg(&pb.p[9][j]), l = __ldg(&pb.p[10][j]);
-    o.bx = k.x; o.by = k.y; o.bz = l.x;
+    const Rec64 k = ld_rec(&pb.d[4][j]);
+    o.bx = k.a.x; o.by = k.a.y; o.bz = k.b.x;
   }
 };
 template <> struct Loader<float> {

@@ -291,7 +291,7 @@ struct sph_handle {
   // sorted arrays
   DevBuf sx, sy, sz, s32, ssrc, cflag, cpos, centre_k, centre_p;
   DevBuf hk_s, dk_s, ok_s;
-  DevBuf pk[11], qk[7], qunit;
+  DevBuf pk[5], pvt, qk[7], qunit;
   // neighbours: one row per centre inside nl, rows sized from each
   // particle's previous count (CSR with slack)
   DevBuf nl, ncnt, rowoff, rowcap, rowcap64, count_prev, h_prev, scan64_tmp;
@@ -686,7 +686,8 @@ struct sph_handle {
     size_t sb = scan_temp_bytes(nall + 1);
     if (sb > scan_tmp.bytes) RC(scan_tmp.ensure(sb));
     if (prec == SPH_PREC_FP64) {
-      for (int i = 0; i < 11; ++i) RC(pk[i].ensure(sizeof(double2) * nall));
+      for (int i = 0; i < 5; ++i) RC(pk[i].ensure(sizeof(Rec64) * nall));
+      RC(pvt.ensure(sizeof(double2) * nall));
     } else {
       for (int i = 0; i < 7; ++i) RC(qk[i].ensure(sizeof(float4) * nall));
       RC(qunit.ensure(sizeof(float)));
@@ -695,7 +696,8 @@ struct sph_handle {
   }
   PackBufs packs() const {
     PackBufs pb;
-    for (int i = 0; i < 11; ++i) pb.p[i] = pk[i].as<double2>();
+    for (int i = 0; i < 5; ++i) pb.d[i] = pk[i].as<Rec64>();
+    pb.vt = pvt.as<double2>();
     for (int i = 0; i < 7; ++i) pb.q[i] = qk[i].as<float4>();
     pb.unit = qunit.as<float>();
     return pb;

@@ -1239,9 +1239,8 @@ __device__ __forceinline__ void pack_pos(int prec, int groups, int64_t k, int64_
                                          const PackGeom& pg, const PackBufs& pb) {
   const double m = cols[es_m * ld + p] / pg.mref;
   if (prec == SPH_PREC_FP64) {
-    pb.p[0][k] = make_double2(x, y);
-    pb.p[1][k] = make_double2(z, m);
-    if (groups & PACK_TEMP) pb.p[6][k] = make_double2(cols[es_vz * ld + p], cols[es_t * ld + p]);
+    pb.d[0][k] = {make_double2(x, y), make_double2(z, m)};
+    if (groups & PACK_TEMP) pb.vt[k] = make_double2(cols[es_vz * ld + p], cols[es_t * ld + p]);
   } else {
     const double sc = 2147483648.0 / pg.shift;  // (a power of two)
     const int32_t xi = fixpos((x - pg.ox) * sc);
@@ -2036,17 +2035,14 @@ __global__ void k_pack(int prec, int groups, int64_t n, const int32_t* __restric
       const double ih = 1.0 / h;
       double kp = pb.kp_wcv;
       for (int d = 0; d <= pb.kp_dim; ++d) kp *= ih;
-      pb.p[2][k] = make_double2(ih, 0.5 * rho);
-      pb.p[3][k] = make_double2(kp / (rho * rho * om), P);
-      pb.p[4][k] = make_double2(pb.kp_alpha * C(es_c), pb.kp_au * C(es_u));
-      pb.p[5][k] = make_double2(C(es_vx), C(es_vy));
-      pb.p[6][k] = make_double2(C(es_vz), C(es_t));
+      pb.d[1][k] = {make_double2(ih, 0.5 * rho), make_double2(kp / (rho * rho * om), P)};
+      pb.d[2][k] = {make_double2(pb.kp_alpha * C(es_c), pb.kp_au * C(es_u)),
+                    make_double2(C(es_vx), C(es_vy))};
+      pb.vt[k] = make_double2(C(es_vz), C(es_t));
     }
     if (groups & PACK_EXTRA) {
-      pb.p[7][k] = make_double2(C(es_kappa), C(es_dtdx));
-      pb.p[8][k] = make_double2(C(es_dtdy), C(es_dtdz));
-      pb.p[9][k] = make_double2(C(es_bx), C(es_by));
-      pb.p[10][k] = make_double2(C(es_bz), 0.0);
+      pb.d[3][k] = {make_double2(C(es_kappa), C(es_dtdx)), make_double2(C(es_dtdy), C(es_dtdz))};
+      pb.d[4][k] = {make_double2(C(es_bx), C(es_by)), make_double2(C(es_bz), 0.0)};
     }
   } else {
     if (groups & PACK_HYDRO) {

@@ -345,11 +345,27 @@ void launch_skin_sig(const double* cols, int64_t nrows, BoxGeom g, int dim, uint
 // (PACK_TEMP: with PACK_POS, also the temperature stream the circuit1
 // sweeps of the diffusion paths read)
 enum PackGroup : int { PACK_POS = 1, PACK_HYDRO = 2, PACK_EXTRA = 4, PACK_TEMP = 8 };
+// An FP64 record of four, read by one 256-bit load: half the requests and
+// addresses of two 16-byte streams, and a line per four particles instead of
+// two of eight (circuit2 1.631 -> 1.602 ms at 96^3, with the field 38 -> 35
+// us at 201^2; circuit1 0.672 -> 0.662).  The FP32 records stay 16 bytes
+// each: as pairs circuit2 went 1.98 -> 2.11 ms at 128^3 (9 blocks per SM,
+// eight more registers at once), 2.56 at 8 blocks.
+struct alignas(32) Rec64 { double2 a, b; };
+#ifdef __CUDACC__
+__device__ __forceinline__ Rec64 ld_rec(const Rec64* p) {
+  Rec64 r;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(r.a.x), "=d"(r.a.y), "=d"(r.b.x), "=d"(r.b.y) : "l"(p));
+  return r;
+}
+#endif
 struct PackBufs {
-  // FP64: p[0], p[1] = x, y, z, m; p[2] = (1/h, rho / 2), p[3] =
-  // (wCv / (h^(d+1) rho^2 Omega), P), p[4] = (alpha c, au u), p[5], p[6] =
-  // v and T, p[7] .. p[10] the diffusion and field quantities
-  double2* p[11];
+  // FP64: d[0] = (x, y, z, m), d[1] = (1/h, rho / 2,
+  // wCv / (h^(d+1) rho^2 Omega), P), d[2] = (alpha c, au u, vx, vy), d[3] =
+  // (kappa, grad T), d[4] = (B, 0); vt = (vz, T)
+  Rec64* d[5];
+  double2* vt;
   // FP32: q[0] = (x, y, z high parts, m), q[1] = (x, y, z low parts, 1/h),
   // q[2] = (rho / 2, wCv / (h^(d+1) rho^2 Omega), P, alpha c), q[3] = (au u, v), q[4] / q[5] the
   // temperature, diffusion and field quantities (the force pass); q[6] =
