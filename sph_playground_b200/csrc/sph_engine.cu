@@ -23,6 +23,8 @@
 
 #include "sph_internal.h"
 
+#include <cuda.h>
+
 #include <chrono>
 
 using namespace sph;
@@ -3497,16 +3499,45 @@ static int column_set(const int* fields, int nf, ColumnSet* fs) {
   return SPH_OK;
 }
 
+// May kernels of the current device read and write [p, p + bytes) in place of
+// a staging buffer?  Only a whole span of one allocation on this device, at a
+// double's alignment; anything else (host, managed, peer or too short) takes
+// the copy, which reports what it does not accept.
+static bool span_on_device(const void* p, size_t bytes) {
+  using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static const RangeFn range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                   q == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<RangeFn>(f)
+               : nullptr;
+  }();
+  cudaPointerAttributes at{};
+  int dev = -1;
+  if (!range || cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if (at.type != cudaMemoryTypeDevice || at.device != dev || a % alignof(double)) return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  return range(&base, &size, CUdeviceptr(a)) == CUDA_SUCCESS && a >= base &&
+         bytes <= size - (a - base);
+}
+
 int sph_get_columns(sph_handle* h, const int* fields, int nf, double* out) {
   AllocScope alloc_scope(h);
   if (!h || !out) return fail(SPH_ERR_ARG, "null argument");
   ColumnSet fs{};
   RC(column_set(fields, nf, &fs));
   const size_t bytes = sizeof(double) * size_t(nf) * size_t(h->nrows);
-  RC(h->colbuf.ensure(bytes));
-  launch_get_columns(h->cols.as<double>(), h->nrows, h->orig.as<int32_t>(), h->nrows, fs,
-                     h->colbuf.as<double>(), h->s);
-  CK(cudaMemcpyAsync(out, h->colbuf.p, bytes, cudaMemcpyDefault, h->s));
+  const bool direct = span_on_device(out, bytes);
+  if (!direct) RC(h->colbuf.ensure(bytes));
+  double* const to = direct ? out : h->colbuf.as<double>();
+  launch_get_columns(h->cols.as<double>(), h->nrows, h->orig.as<int32_t>(), h->nrows, fs, to, h->s);
+  if (!direct) CK(cudaMemcpyAsync(out, to, bytes, cudaMemcpyDefault, h->s));
   CK(cudaStreamSynchronize(h->s));
   CK(cudaGetLastError());
   return SPH_OK;
@@ -3518,10 +3549,17 @@ int sph_set_columns(sph_handle* h, const int* fields, int nf, const double* in) 
   ColumnSet fs{};
   RC(column_set(fields, nf, &fs));
   const size_t bytes = sizeof(double) * size_t(nf) * size_t(h->nrows);
-  RC(h->colbuf.ensure(bytes));
-  CK(cudaMemcpyAsync(h->colbuf.p, in, bytes, cudaMemcpyDefault, h->s));
+  const bool direct = span_on_device(in, bytes);
+  if (!direct) {
+    RC(h->colbuf.ensure(bytes));
+    CK(cudaMemcpyAsync(h->colbuf.p, in, bytes, cudaMemcpyDefault, h->s));
+  }
+  // of a field named more than once the last values stay
+  for (int k = 0; k < fs.n; ++k)
+    for (int j = k + 1; j < fs.n && fs.f[k] >= 0; ++j)
+      if (fs.f[j] == fs.f[k]) fs.f[k] = -1;
   launch_set_columns(h->cols.as<double>(), h->nrows, h->orig.as<int32_t>(), h->nrows, fs,
-                     h->colbuf.as<double>(), h->s);
+                     direct ? in : h->colbuf.as<double>(), h->s);
   // skin lists follow moved positions and changed h by themselves (the next
   // iterate measures both); a changed particle type may change the image set
   for (int k = 0; k < fs.n; ++k)
