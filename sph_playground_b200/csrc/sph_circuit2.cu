@@ -52,7 +52,16 @@ template <class R> struct PartX {
 template <class R> struct Loader;
 template <> struct Loader<double> {
   static __device__ __forceinline__ void hydro(const PackBufs& pb, int64_t j, Part<double>& o) {
-    const Rec64 a = ld_rec(&pb.d[0][j]), c = ld_rec(&pb.d[1][j]), e = ld_rec(&pb.d[2][j]);
+    hydro(pb, j, ahead(pb, j), o);
+  }
+  // the part of a neighbour's record that is read one round ahead (AHEAD)
+  struct Ahead { Rec64 a; };
+  static __device__ __forceinline__ Ahead ahead(const PackBufs& pb, int64_t j) {
+    return {ld_rec(&pb.d[0][j])};
+  }
+  static __device__ __forceinline__ void hydro(const PackBufs& pb, int64_t j, const Ahead& h,
+                                               Part<double>& o) {
+    const Rec64 a = h.a, c = ld_rec(&pb.d[1][j]), e = ld_rec(&pb.d[2][j]);
     o.vz = __ldg(&pb.vt[j].x);
     o.pos.x = a.a.x; o.pos.y = a.a.y; o.pos.z = a.b.x; o.m = a.b.y;
     o.invh = c.a.x; o.hrho = c.a.y; o.rho = 2.0 * c.a.y; o.Pi = c.b.x; o.P = c.b.y;
@@ -71,6 +80,12 @@ template <> struct Loader<double> {
   }
 };
 template <> struct Loader<float> {
+  struct Ahead {};
+  static __device__ __forceinline__ Ahead ahead(const PackBufs&, int64_t) { return {}; }
+  static __device__ __forceinline__ void hydro(const PackBufs& pb, int64_t j, const Ahead&,
+                                               Part<float>& o) {
+    hydro(pb, j, o);
+  }
   static __device__ __forceinline__ void hydro(const PackBufs& pb, int64_t j, Part<float>& o) {
     float4 a = __ldg(&pb.q[0][j]), b = __ldg(&pb.q[1][j]), c = __ldg(&pb.q[2][j]),
            d = __ldg(&pb.q[3][j]);
@@ -155,6 +170,14 @@ __device__ __forceinline__ double group_sum(double v, unsigned gmask) {
 template <int K, int DIM, class R, int MODE, int G>
 __global__ void __launch_bounds__(TPB, sizeof(R) == 8 ? 5 : MODE == C2_HYDRO ? 9 : 7)
 k_c2(C2Args a, PackBufs pb, Params P) {
+  // The next neighbour's position is read a round ahead, so that r, its root
+  // and the kernel do not wait for memory at the head of every round: FP64
+  // hydrodynamics alone, long-scoreboard stalls 4.2 of 9 cycles an
+  // instruction before (96^3, with 20 warps per SM: 1.60 -> 1.42 ms; with 1/h
+  // and P as well 1.51, or 1.45 at 4 blocks per SM; position alone at 4 blocks
+  // 1.48).  FP32 has 36 warps per SM and no registers left: 1.98 -> 2.07 ms
+  // at 128^3.  With the field or diffusion no gain.
+  constexpr bool AHEAD = sizeof(R) == 8 && MODE == C2_HYDRO;
   constexpr bool HEAT = MODE == C2_HESSIAN || MODE == C2_TWO_NW || MODE == C2_GENERAL;
   constexpr bool FIELD = MODE == C2_MHD || MODE == C2_GENERAL;
   constexpr bool PRESSURE = MODE == C2_HYDRO || MODE == C2_MHD || MODE == C2_GENERAL;
@@ -244,13 +267,25 @@ k_c2(C2Args a, PackBufs pb, Params P) {
     const int32_t* __restrict__ row = a.nl + a.rowoff[c];
     // the next neighbour's index is read one round ahead, so that a round
     // waits on one dependent load (the neighbour's streams), not two
-    int32_t jnext = lane < n ? row[lane] : 0;
+    int32_t jnext = lane < n ? row[lane] : 0, jnext2 = 0;
+    typename Loader<R>::Ahead next;
+    if constexpr (AHEAD) {
+      jnext2 = lane + G < n ? row[lane + G] : 0;
+      next = Loader<R>::ahead(pb, jnext);
+    }
     for (int l0 = lane; l0 < n; l0 += G) {
     {
       const int64_t j = jnext;
       Part<R> B;
-      Loader<R>::hydro(pb, j, B);
-      if (l0 + G < n) jnext = row[l0 + G];
+      if constexpr (AHEAD) {
+        Loader<R>::hydro(pb, j, next, B);
+        jnext = jnext2;
+        next = Loader<R>::ahead(pb, jnext);
+        if (l0 + 2 * G < n) jnext2 = row[l0 + 2 * G];
+      } else {
+        Loader<R>::hydro(pb, j, B);
+        if (l0 + G < n) jnext = row[l0 + G];
+      }
       R rab[3];
       pos_delta(A.pos, B.pos, rab[0], rab[1], rab[2]);
       R r2 = rab[0] * rab[0];
