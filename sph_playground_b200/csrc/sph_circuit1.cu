@@ -100,7 +100,8 @@ __device__ __forceinline__ unsigned group_mask() {
 // G lanes per centre: each lane sums every G-th neighbour of the centre's
 // row of the neighbour list (coalesced), the group adds its lanes' two-sum
 // partials in FP64, and every lane takes the same FP64 Newton step.
-// (FP32: 6 blocks per SM, 80 registers, no spill: 128^3, 4 lanes, density
+// (FP64: 8 blocks per SM, 62 registers; a 96^3 blast of 4 steps takes 9.66 ms,
+// with 7 blocks 9.86, with 6 10.1.  FP32: 6 blocks per SM, 80 registers, no spill: 128^3, 4 lanes, density
 // pass 3.22 ms, blast step 0.955; 7 blocks 3.39 / 0.936, 8 with 24 spilled
 // bytes 3.46 / 1.026.)
 template <int K, int DIM, class R, int G>
@@ -142,14 +143,14 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
       // what the Newton iteration needs); the d rho / dh sum only scales the
       // Newton step and Omega, so a plain per-lane sum suffices
       double sw_lane, so_lane;
-      // U neighbours per lane per round: their pair data are all requested
-      // before the first is used, so the gathers overlap; the list entries
-      // of the next round are read one round ahead
-      constexpr int U = sizeof(R) == 4 ? 4 : 2;
-      int32_t jn[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) jn[u] = (lane + u * G < n) ? row[lane + u * G] : -1;
       if constexpr (sizeof(R) == 4) {
+        // U neighbours per lane per round: their pair data are all requested
+        // before the first is used, so the gathers overlap; the list entries
+        // of the next round are read one round ahead
+        constexpr int U = 4;
+        int32_t jn[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) jn[u] = (lane + u * G < n) ? row[lane + u * G] : -1;
         // FP32: two neighbours per packed instruction.  The kernel is bound
         // by instruction issue (79 % of the slots, FMA pipe 45 %, one pair at a time)
         // and has FMA time to spare.  An entry past the row's end is record
@@ -207,35 +208,29 @@ k_c1_newton(C1Args a, PackBufs pb, Params P) {
         SumAcc<R> so;
         sw.init();
         so.init();
-        for (int l0 = lane; l0 < n; l0 += G * U) {
-          int64_t jj[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) jj[u] = jn[u];
-          typename PosAccess<R>::Pos pj[U];
-          R mj[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) pj[u] = PosAccess<R>::load(pb, jj[u] >= 0 ? jj[u] : 0, mj[u]);
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const int l = l0 + (U + u) * G;
-            jn[u] = l < n ? row[l] : -1;
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            if (jj[u] < 0) continue;
-            R dx, dy, dz;
-            pos_delta(pi, pj[u], dx, dy, dz, R(1));
-            R r2 = dx * dx;
-            if (DIM >= 2) r2 += dy * dy;
-            if (DIM == 3) r2 += dz * dz;
-            const R r = rsq<R>(r2);
-            const R q = r * ih;
-            bad |= q_bad(q);
-            R f, df;
-            kshape_f_df<K, R>(q, f, df);
-            sw.add(mj[u] * f);
-            so.add(mj[u] * (R(DIM) * f + q * df));
-          }
+        // The next neighbour's record and the index after it are read ahead,
+        // one neighbour per round (96^3, 4 lanes: 0.66 -> 0.57 ms; two per
+        // round, their indices alone ahead, was the former).
+        int32_t jnext = lane + G < n ? row[lane + G] : 0;
+        R mn;
+        typename PosAccess<R>::Pos pn = PosAccess<R>::load(pb, lane < n ? row[lane] : 0, mn);
+        for (int l = lane; l < n; l += G) {
+          const typename PosAccess<R>::Pos pj = pn;
+          const R mj = mn;
+          pn = PosAccess<R>::load(pb, jnext, mn);
+          jnext = l + 2 * G < n ? row[l + 2 * G] : 0;
+          R dx, dy, dz;
+          pos_delta(pi, pj, dx, dy, dz, R(1));
+          R r2 = dx * dx;
+          if (DIM >= 2) r2 += dy * dy;
+          if (DIM == 3) r2 += dz * dz;
+          const R r = rsq<R>(r2);
+          const R q = r * ih;
+          bad |= q_bad(q);
+          R f, df;
+          kshape_f_df<K, R>(q, f, df);
+          sw.add(mj * f);
+          so.add(mj * (R(DIM) * f + q * df));
         }
         sw_lane = sw.dval();
         so_lane = so.dval();
