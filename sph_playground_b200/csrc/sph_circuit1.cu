@@ -331,12 +331,19 @@ k_c1_sweep(C1Args a, PackBufs pb, Params P) {
       g[0].init(); g[1].init(); g[2].init();
       bool bad = false;
       const R rta = R(ta), rrhoa = R(rhoa), roma = R(oma);
-      int32_t jnext = lane < n ? row[lane] : 0;  // list entry read one round ahead
+      // the next neighbour's record and the index after it are read ahead
+      // (256^2 FP32 diffusion 1.33 -> 1.30 ms a pass of 9 iterates, 64^2 FP64
+      // 0.87 -> 0.83, against the index alone)
+      int32_t j1 = lane < n ? row[lane] : 0, j2 = lane + G < n ? row[lane + G] : 0;
+      R mn;
+      typename PosAccess<R>::Pos pn = PosAccess<R>::load(pb, j1, mn);
       for (int l = lane; l < n; l += G) {
-        const int64_t j = jnext;
-        R mj;
-        const typename PosAccess<R>::Pos pj = PosAccess<R>::load(pb, j, mj);
-        if (l + G < n) jnext = row[l + G];
+        const int64_t j = j1;
+        const R mj = mn;
+        const typename PosAccess<R>::Pos pj = pn;
+        j1 = j2;
+        pn = PosAccess<R>::load(pb, j1, mn);
+        j2 = l + 2 * G < n ? row[l + 2 * G] : 0;
         R dx, dy, dz;
         pos_delta(pi, pj, dx, dy, dz, punit);
         R r2 = dx * dx;
