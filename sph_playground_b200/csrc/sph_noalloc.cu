@@ -92,7 +92,8 @@ __device__ __forceinline__ unsigned long long umax64(unsigned long long a, unsig
 __global__ void __launch_bounds__(TPB) k_na_reduce(const double* x, const double* y,
                                                    const double* z, const double* h, int64_t n,
                                                    double krad, int64_t max_cells, NaPlan* pl) {
-  unsigned long long v[7] = {0, 0, 0, 0, 0, 0, 0};
+  // (h starts at 1e308: infinite and NaN radii alone give one cell for all)
+  unsigned long long v[7] = {0, 0, 0, ~dkey(1e308), 0, 0, 0};
   for (int64_t i = blockIdx.x * int64_t(TPB) + threadIdx.x; i < n; i += int64_t(gridDim.x) * TPB) {
     const unsigned long long k[4] = {dkey(pos_of(x, i)), dkey(pos_of(y, i)), dkey(pos_of(z, i)),
                                      dkey(h[i])};
@@ -253,7 +254,9 @@ struct NaRows {
 // are walked 32 candidates at a time, one per lane, and the candidates that
 // are neighbours go, packed, to a queue in shared memory, from which 32 at a
 // time get their kernel value: it costs several times a test and less than
-// half the candidates are neighbours.
+// half the candidates are neighbours.  A NaN radius is reported from the
+// radius itself: its run, the first cell's, may hold no particle.  (A lone
+// particle is not refused: no other one would have met it.)
 // Bound by instruction issue (65 % of the slots; FP64 pipe 28 %): 1,800
 // instructions a particle, of them 385 FP64.  One thread per particle in the
 // caller's order over whole cells of edge krad h_min (7 tests a neighbour,
@@ -281,7 +284,7 @@ k_na_density(const double* h, int64_t n, NaPlan* pl, double krad, double wcv,
   const double ih = 1.0 / hi;
   const NaRows<DIM> sphere(g, pl->fx, pi, R2);
   double sum = 0.0;
-  bool bad = false;
+  bool bad = lane == 0 && n > 1 && !(R2 >= 0.0);
   unsigned head = 0;  // the queue's first entry
   int held = 0;       // and its length
   auto value = [&](bool on) {
@@ -373,6 +376,7 @@ k_na_density2(const double* h, int64_t n, NaPlan* pl, double krad, double wcv,
     const double kh = __dmul_rn(krad, hi);
     const double R2 = __dmul_rn(kh, kh);
     const double ih = 1.0 / hi;
+    bad = n > 1 && !(R2 >= 0.0);
     const NaRows<DIM> sphere(g, pl->fx, pi, R2);
     // (the one row of 1D: its candidates in turn, not the rows)
     constexpr int row_step = DIM == 1 ? 1 : 2, step = DIM == 1 ? 2 : 1;
