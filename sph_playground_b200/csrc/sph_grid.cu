@@ -1481,7 +1481,7 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
   }
   const bool fast = __ldcg(red + RED_SKIN_NFAST) != 0, move = __ldcg(red + RED_SKIN_NMOVE) != 0;
   int at = 0;  // the field that holds the marks
-  if (move) {  // (tau > eps: a fast record moves)
+  if (move || fast) {  // (a fast record need not count as moving: tau <= eps for s <= 4e-6)
     for (int64_t k = first; k < a.nall; k += step) {
       const float d = a.r.dsp[k];
       if (d > a.r.eps) a.mcell[0][a.keys[k]] = 1;
@@ -1494,7 +1494,7 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
     }
     grid.sync();
     for (int axis = 0; axis < a.r.dim; ++axis) {
-      dilate_axis(a.mcell[at], a.mcell[1 - at], a.grid, axis, wm);
+      if (move) dilate_axis(a.mcell[at], a.mcell[1 - at], a.grid, axis, wm);
       if (fast) dilate_axis(a.fcell[at], a.fcell[1 - at], a.grid, axis, wf);
       at = 1 - at;
       grid.sync();
