@@ -373,6 +373,7 @@ struct sph_handle {
   double skin_s = 0.;        // their fraction s (radius (1 + s) krad h)
   double skin_tau = 0.;      // displacement up to which a record is slow
   double skin_eps = 0.;      // displacement up to which a record is still
+  double skin_far = 0.;      // and up to which its drift may leave rows as they are
   double skin_hmin = 0.;     // h_min at their search
   int skin_age = 0;          // iterates served since their search
   // lists that serve fewer than kSkinShort iterates cost more than they save
@@ -996,8 +997,12 @@ struct sph_handle {
     }
     skin_tau = 0.25 * skin * P.krad * hmin;
     // (4 eps come off every gap: at 1e-5 15 % of a 128^3 blast's rows filtered
-    // each iterate, 0.74 ms for all lists, at 1e-6 2 %, 0.37)
+    // each iterate, 0.74 ms for all lists, at 1e-6 2 %, 0.37.  Rows among
+    // records that drift by more than eps are kept with 4 min(far, D) off the
+    // gap: a density pass of 96^3 particles FP32 that drift by 3e-6 krad h
+    // takes 0.63 ms, with eps alone 1.54; the blast is the same)
     skin_eps = 1e-6 * P.krad * hmin;
+    skin_far = 1e-4 * P.krad * hmin;
     skin_hmin = hmin;
     RC(fill_table(exact_table(), P, true, [&](NeibArgs& na, int) {
       launch_skin_filter(filter_args(na, false, true), s);
@@ -1164,7 +1169,7 @@ struct sph_handle {
     RC(coop_most(COOP_SERVE, most));
     const int blocks = coop_blocks(nall, most);
     RC(skin_fcell.ensure(2 * size_t(ncell)));
-    RC(skin_mcell.ensure(2 * size_t(ncell)));
+    RC(skin_mcell.ensure(2 * sizeof(uint16_t) * size_t(ncell)));
     {
       Phase ph(this, SPH_T_NEIGHBOURS);
       SkinServe a{};
@@ -1186,7 +1191,7 @@ struct sph_handle {
       a.keys = keys_alt.as<uint32_t>();
       for (int k = 0; k < 2; ++k) {
         a.fcell[k] = skin_fcell.as<uint8_t>() + k * ncell;
-        a.mcell[k] = skin_mcell.as<uint8_t>() + k * ncell;
+        a.mcell[k] = skin_mcell.as<uint16_t>() + k * ncell;
       }
       a.nc = nreal;
       a.centre_k = centre_k.as<int32_t>();
@@ -1199,6 +1204,7 @@ struct sph_handle {
       a.krad = P.krad;
       a.kfac = 1.0 + skin_s;
       a.dcap = P.krad * skin_hmin;
+      a.far = float(skin_far);
       a.dirty_share = kSkinDirtyShare;
       a.dlist = skin_dlist.as<int32_t>();
       a.flist = skin_flist.as<int32_t>();

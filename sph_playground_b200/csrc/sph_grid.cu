@@ -1185,15 +1185,17 @@ __global__ void __launch_bounds__(TPB, 8) k_sort_records(SortArgs a) {
 //    widened by the largest displacement D): a record that moved more than
 //    tau ("fast") is within reach, the centre moved more than tau itself, or
 //    its h grew too far for the inequality above;
-//  * keep: no record of its skin list moved more than eps since b, nor did
-//    the centre, and 4 eps + krad |h_t - h_f| (running maximum since f) stays
+//  * keep: no record of its skin list moved more than e since b, nor did
+//    the centre, and 4 e + krad |h_t - h_f| (running maximum since f) stays
 //    below the gap of f, the step its row was last written (the smallest
 //    distance then of a skin-list record from the sphere krad h_f): between
-//    f and t each of a pair's two records moved at most 2 eps, so no record
+//    f and t each of a pair's two records moved at most 2 e, so no record
 //    crossed the sphere, and the row written at f is the set at t (the row
-//    is not touched while it is kept);
+//    is not touched while it is kept).  e is eps for a centre among records
+//    at rest, and min(far, D) for one among records that drift (far = 100
+//    eps: 4 e comes off the gap, so a wider e keeps fewer rows);
 //  * filter: its skin list through the FP64 predicate, with a new gap when
-//    the centre is as quiet as keeping asks (it moved at most eps and so did
+//    the centre is as quiet as keeping asks (it moved at most far and so did
 //    its list): what failed it was h, which may have settled since (the
 //    first Newton solve moves every h from the caller's guess; without the
 //    new gap its centres filtered every iterate from then on: 93 % of the
@@ -1367,7 +1369,8 @@ __device__ __forceinline__ void skin_slots_clear(unsigned long long* red, int32_
 // launch, 4 blocks 0.27.)
 //
 // Marks at the level of cells: a record that moved more than eps flags the
-// cell it was sorted into (its position at b), one that moved more than tau
+// cell it was sorted into (its position at b), in the low byte, one that
+// moved more than far in the high byte too, one that moved more than tau
 // the cell of its position now (clamped to the grid); each flag field is
 // then dilated by a box of w cells per side, one axis per pass,
 // w = ceil(reach / L) + 1, which holds every cell within `reach` of any
@@ -1375,21 +1378,28 @@ __device__ __forceinline__ void skin_slots_clear(unsigned long long* red, int32_
 // before last, whose marks its own result contains, so the two fields are
 // cleared once; every marked cell writes its window, so the work follows the
 // marks (a few per cent of the cells while the lists serve), not the grid.
-// A centre is near a fast (moving) record when the cell it was sorted into
-// carries the dilated flag.
-__device__ __forceinline__ void dilate_axis(const uint8_t* in, uint8_t* out, const Grid& g, int axis,
-                                            int w) {
+// A centre is near a fast (moving, far) record when the cell it was sorted
+// into carries the dilated flag.
+// (two bytes per cell: the high one is only set where the low one is, so a
+// store of both and a store of the low one may meet in any order)
+template <class T>
+__device__ __forceinline__ void dilate_axis(const T* in, T* out, const Grid& g, int axis, int w) {
   const int64_t ncell = int64_t(g.nx) * g.ny * g.nz;
   for (int64_t c = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; c < ncell;
        c += int64_t(gridDim.x) * blockDim.x) {
-    if (!in[c]) continue;
+    const T v = in[c];
+    if (!v) continue;
     int n, i;
     int64_t stride;
     if (axis == 0) { n = g.nx; i = int(c % g.nx); stride = 1; }
     else if (axis == 1) { n = g.ny; i = int((c / g.nx) % g.ny); stride = g.nx; }
     else { n = g.nz; i = int(c / (int64_t(g.nx) * g.ny)); stride = int64_t(g.nx) * g.ny; }
     const int lo = max(0, i - w), hi = min(n - 1, i + w);
-    for (int j = lo; j <= hi; ++j) out[c + int64_t(j - i) * stride] = 1;
+    for (int j = lo; j <= hi; ++j) {
+      T* const o = out + c + int64_t(j - i) * stride;
+      if (v > 1) *o = v;
+      else *reinterpret_cast<uint8_t*>(o) = 1;
+    }
   }
 }
 
@@ -1424,9 +1434,10 @@ __device__ __forceinline__ int skin_gate(const unsigned long long* red, const Sk
 // The way of centre c (0 filter, 1 fresh search, 2 keep).  The margins of
 // 1e-12 (relative) lie far above the FP64 rounding of the predicate and of
 // the displacements, so that no record outside a list can pass the FP64
-// predicate at t; near_f / near_m are the dilated cell flags.
+// predicate at t; near_f / near_m are the dilated cell flags (fast; moving
+// and, above 1, far), far = min(far, D).
 __device__ __forceinline__ uint8_t skin_way(const SkinServe& a, int64_t c, const uint8_t* near_f,
-                                            const uint8_t* near_m) {
+                                            const uint16_t* near_m, float far) {
   if (a.mode[c] == 1) return 1;  // (a centre once searched afresh stays so)
   const int32_t k = a.centre_k[c];
   const float dk = a.r.dsp[k], tau = a.r.tau, eps = a.r.eps;
@@ -1436,8 +1447,9 @@ __device__ __forceinline__ uint8_t skin_way(const SkinServe& a, int64_t c, const
   const uint32_t cell = a.keys[k];  // the cell the centre was sorted into
   if (near_f[cell] || !(dk <= tau) || !(lhs < rhs)) return 1;
   const double hd = fmax(a.hdev[c], fabs(h - a.href[c]));
-  const bool quiet = !near_m[cell] && dk <= eps;
-  if (quiet && 4.0 * double(eps) + a.krad * hd * (1.0 + 1e-12) + 1e-12 * a.krad * h0 <
+  const uint16_t near = near_m[cell];
+  const bool rest = !near && dk <= eps, quiet = rest || (near <= 1 && dk <= far);
+  if (quiet && 4.0 * double(rest ? eps : far) + a.krad * hd * (1.0 + 1e-12) + 1e-12 * a.krad * h0 <
                    double(a.gap[c])) {
     a.hdev[c] = hd;
     return 2;
@@ -1457,7 +1469,7 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
   // the records; clears: the flag fields, and what the next launch finds at
   // its start (its reduction slots and counts: two sets, used in turn)
   for (int64_t i = first; i < ncell; i += step)
-    a.fcell[0][i] = a.fcell[1][i] = a.mcell[0][i] = a.mcell[1][i] = 0;
+    a.fcell[0][i] = a.fcell[1][i] = 0, a.mcell[0][i] = a.mcell[1][i] = 0;
   if (first == 0) {
     skin_slots_clear(a.red_next, a.counts_next);
     a.flags[0] = a.flags[1] = 0;
@@ -1480,11 +1492,14 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
     return;
   }
   const bool fast = __ldcg(red + RED_SKIN_NFAST) != 0, move = __ldcg(red + RED_SKIN_NMOVE) != 0;
+  // (D is the maximum of FP32 values, and 0 <= D)
+  const float far = fminf(a.far, float(dkey_inv(__ldcg(red + RED_SKIN_D))));
   int at = 0;  // the field that holds the marks
   if (move || fast) {  // (a fast record need not count as moving: tau <= eps for s <= 4e-6)
     for (int64_t k = first; k < a.nall; k += step) {
       const float d = a.r.dsp[k];
-      if (d > a.r.eps) a.mcell[0][a.keys[k]] = 1;
+      if (d > a.far) a.mcell[0][a.keys[k]] = 0x0101;
+      else if (d > a.r.eps) *reinterpret_cast<uint8_t*>(a.mcell[0] + a.keys[k]) = 1;
       if (d > a.r.tau) {
         const int cx = clamp_cell((a.r.sx[k] - a.grid.ox) * a.grid.invL, a.grid.nx);
         const int cy = clamp_cell((a.r.sy[k] - a.grid.oy) * a.grid.invL, a.grid.ny);
@@ -1511,7 +1526,7 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
     const int64_t c = t + threadIdx.x;
     int w = 2;
     if (c < a.nc) {
-      w = skin_way(a, c, a.fcell[at], a.mcell[at]);
+      w = skin_way(a, c, a.fcell[at], a.mcell[at], far);
       a.mode[c] = uint8_t(w);
       if (w == 2) {
         ++v[0];

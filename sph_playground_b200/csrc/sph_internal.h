@@ -435,7 +435,9 @@ struct SkinServe {
   PackGeom pg;
   Grid grid;       // cells of the lists' search, keys[k] each record's
   const uint32_t* keys;
-  uint8_t *fcell[2], *mcell[2];  // two flag fields each (fast, moving)
+  // two flag fields each: fast; moving (low byte) and far (high byte too)
+  uint8_t* fcell[2];
+  uint16_t* mcell[2];
   int64_t nc;
   const int32_t* centre_k;
   // per centre: h at the lists' search, h when the row was last written, the
@@ -446,6 +448,7 @@ struct SkinServe {
   uint8_t* mode;
   const int32_t* ncnt;
   double krad, kfac, dcap, dirty_share;
+  float far;  // (at least r.eps)
   const unsigned long long* hmaxb;  // largest h of the centres at the lists' search (dkey)
   // centres searched afresh, filtered, blocks done (cleared before it); and
   // the slots and counts of the next launch, which this one clears
