@@ -269,6 +269,13 @@ constexpr int64_t kFewCentres = 65536;
 // fresh searches of a served iterate (centres x widening) as a share of all
 // centres, above which the iterate searches plainly instead
 constexpr double kSkinDirtyShare = 0.15;
+// Blocks of the cooperative launches: a thread per record, or per this many
+// cells where those outnumber the records (h_min far below the usual h: up to
+// 2^20 cells for a few records).  One cell a thread costs more at the grid
+// barriers than it saves (density pass of 10,864 records of which 216 have a
+// tenth of the others' h: 557 us, 8 cells 545, records alone 555; of 1,216
+// such records 738, 728, 787).
+constexpr int64_t kCellsPerThread = 8;
 constexpr float kRowSlack = 1.2f;  // room of a list row over its expected count
 
 struct sph_handle {
@@ -1167,9 +1174,10 @@ struct sph_handle {
     const int64_t ncell = int64_t(grid.nx) * grid.ny * grid.nz;
     int most = 0;
     RC(coop_most(COOP_SERVE, most));
-    const int blocks = coop_blocks(nall, most);
-    RC(skin_fcell.ensure(2 * size_t(ncell)));
-    RC(skin_mcell.ensure(2 * sizeof(uint16_t) * size_t(ncell)));
+    const int blocks = coop_blocks(std::max(nall, ncell / kCellsPerThread), most);
+    // (cleared 16 bytes at a time)
+    RC(skin_fcell.ensure(2 * size_t(ncell) + 16));
+    RC(skin_mcell.ensure(2 * sizeof(uint16_t) * size_t(ncell) + 16));
     {
       Phase ph(this, SPH_T_NEIGHBOURS);
       SkinServe a{};
@@ -1414,7 +1422,7 @@ struct sph_handle {
       a.rowcap = T.rowcap->as<int32_t>();
       a.rowoff = T.rowoff->as<int64_t>();
       a.part = coop_part.as<int64_t>();
-      CK(launch_sort_records(a, coop_blocks(nall, most_sort), s));
+      CK(launch_sort_records(a, coop_blocks(std::max(nall, ncell / kCellsPerThread), most_sort), s));
     }
     if (skin > 0) {
       RC(skin_build(m, P, skin, hmin));

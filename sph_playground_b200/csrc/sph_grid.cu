@@ -1468,8 +1468,10 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
   const int64_t ncell = int64_t(a.grid.nx) * a.grid.ny * a.grid.nz;
   // the records; clears: the flag fields, and what the next launch finds at
   // its start (its reduction slots and counts: two sets, used in turn)
-  for (int64_t i = first; i < ncell; i += step)
-    a.fcell[0][i] = a.fcell[1][i] = 0, a.mcell[0][i] = a.mcell[1][i] = 0;
+  // (a pair of fields is one buffer of whole 16-byte words)
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  for (int64_t i = first; i * 4 < ncell; i += step) reinterpret_cast<uint4*>(a.mcell[0])[i] = none;
+  for (int64_t i = first; i * 8 < ncell; i += step) reinterpret_cast<uint4*>(a.fcell[0])[i] = none;
   if (first == 0) {
     skin_slots_clear(a.red_next, a.counts_next);
     a.flags[0] = a.flags[1] = 0;
