@@ -657,7 +657,7 @@ struct sph_handle {
     RC(goff.ensure(sizeof(int32_t) * (nrows + 1)));
     RC(status.ensure(sizeof(int)));
     RC(red.ensure(sizeof(unsigned long long) * RED_TOTAL));
-    RC(dcnt.ensure(sizeof(unsigned long long) * DC_TOTAL));
+    RC(dcnt.ensure(sizeof(unsigned long long) * 2 * DC_TOTAL));  // (the second set: see circuit2)
     // the longest row, the overflow flag and a served iterate's result (read together)
     RC(maxcnt.ensure(sizeof(SkinFlags)));
     RC(count_prev.ensure(sizeof(int32_t) * nrows));
@@ -670,7 +670,7 @@ struct sph_handle {
     RC(ctrl.ensure(sizeof(double) * 8));
     RC(ciso.ensure(sizeof(double)));
     CK(cudaMemsetAsync(status.p, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(dcnt.p, 0, sizeof(unsigned long long) * DC_TOTAL, s));
+    CK(cudaMemsetAsync(dcnt.p, 0, sizeof(unsigned long long) * 2 * DC_TOTAL, s));
     CK(cudaMemsetAsync(ctrl.p, 0, sizeof(double) * 8, s));
     CK(cudaMemsetAsync(save.p, 0, sizeof(double) * 9 * nrows, s));
     size_t sb = scan_temp_bytes(nrows + 1);
@@ -1459,9 +1459,10 @@ struct sph_handle {
     RC(check_status());  // (waits for the copy too)
     if (!ran) return SPH_OK;
     c1_last = 1 + int(h_red[RED_C1_MORE]);
+    host_max_sweeps = std::max<int64_t>(host_max_sweeps, c1_last);
     if (!h_red[RED_C1_ACTIVE] || ran >= P.maxiter) return SPH_OK;
     RC(circuit1(m, P, false, ran));
-    RC(circuit2(m, P));
+    RC(circuit2(m, P, true));
     return check_status();
   }
 
@@ -1470,6 +1471,7 @@ struct sph_handle {
   int circuit1(const Mode& m, Params& P, bool defer = false, int ran = 0) {
     const int64_t nall = nrows + nghost;
     PackBufs pb = packs();
+    c1_open = 0;
     P.eos_kind = m.eos_kind;
     if (m.eos_kind == 2) {
       // c of row 1 (eos.f90:43): find the physical row whose original index is 0
@@ -1584,13 +1586,15 @@ struct sph_handle {
       }
     }
     if (a.simple) launch_c1_simple_rest(nrows, nreal, cols.as<double>(), s);
-    host_max_sweeps = std::max<int64_t>(host_max_sweeps, iter);
+    if (!c1_open) host_max_sweeps = std::max<int64_t>(host_max_sweeps, iter);
     if (!dplan && !c1_open) c1_last = iter;
     CK(cudaGetLastError());
     return SPH_OK;
   }
 
-  int circuit2(const Mode& m, const Params& P) {
+  // (again: the pass that counts was the iterate's first; this one's pairs go
+  // to counters nobody reads)
+  int circuit2(const Mode& m, const Params& P, bool again = false) {
     const int64_t nall = nrows + nghost;
     PackBufs pb = packs();
     // the positions (PACK_POS) were packed for circuit1 in this iterate and
@@ -1622,7 +1626,7 @@ struct sph_handle {
     a.ld = nrows;
     a.mref = mref;
     a.status = status.as<int>();
-    a.dcnt = dcnt.as<unsigned long long>();
+    a.dcnt = dcnt.as<unsigned long long>() + (again ? DC_TOTAL : 0);
     launch_c2(prec, kernel_id, P.dim, a, pb, P, s);
     if (m.mti) launch_apply_mti(cols.as<double>(), nrows, orig.as<int32_t>(), nrows, nreal,
                                 m.mti == 2, s);

@@ -1,0 +1,57 @@
+"""The work counters of an iterate whose density sweeps run ahead of the
+host's question whether they were enough: pairs of the force pass are counted
+once where it runs again, and sweeps as many as were needed, not as were run."""
+import numpy as np
+import pytest
+
+from parity import COL
+from sph_playground_b200 import abi, consts, ic
+
+pytestmark = pytest.mark.gpu
+
+
+def _set(ddw):
+    n, dim = 24, 2
+    pos, dx = ic.periodic_lattice(n, dim, seed=8, amp=0.1)
+    st = ic._periodic_state(dim, n, 1.2, "m6", "manual", tfinish=1.0)
+    N = len(pos)
+    for k, v in (("realpn", N), ("gamma", 5.0 / 3.0), ("dtprint", 1.0), ("time", 0.0), ("dcondconst", 1.0),
+                 ("eqonhydro", 0.0), ("eqondiff", 1.0), ("eqonfluxlim", 0.0), ("eqonradexch", 0.0),
+                 ("eqonsts", 0.0), ("artts", 0.0), ("disotropic", 1.0), ("ddw", consts.esd[ddw])):
+        ic.set_state(st, k, v)
+    s = np.zeros((N, consts.ES_TOTAL))
+    s[:, :3] = pos
+    for name, v in (("m", 1.0 / N), ("den", 1.0), ("h", 1.4 * dx), ("om", 1.0), ("u", 1.0), ("p", 1.0), ("c", 1.0),
+                    ("t", 1.0 + 0.3 * np.sin(2 * np.pi * pos[:, 0])), ("type", consts.ept["real"])):
+        s[:, COL[name]] = v
+    return st, s
+
+
+@pytest.mark.parametrize("skin", [0.0, 0.1])
+@pytest.mark.parametrize("ddw", ["fab", "2nw_sd"])
+def test_pairs_and_sweeps(engine_lib, oracle_lib, cuda_ok, ddw, skin):
+    st, store = _set(ddw)
+    with abi.Engine(st, store, "m6", precision=abi.PREC_FP64, lib=engine_lib) as e, \
+            abi.Engine(st, store, "m6", precision=abi.PREC_FP64, lib=oracle_lib) as o:
+        e.set_param(abi.P_SKIN, skin)
+        needed = []
+        # h guessed, settled, settled, guessed again
+        for k in range(4):
+            if k == 3:
+                table = e.get_store()
+                table[:, COL["h"]] *= 1.1
+                e.set_store(table)
+                o.set_store(table)
+            e.reset_counters()
+            o.reset_counters()
+            e.iterate()
+            o.iterate()
+            c, ref = e.counters(), o.counters()
+            pairs = int(e.get_neighbours()[0][-1])
+            assert c["c2_pairs"] == pairs == ref["c2_pairs"]
+            assert c["c1_sweeps"] == ref["c1_sweeps"]
+            assert c["c1_pairs"] == ref["c1_pairs"]
+            needed.append(c["c1_sweeps"])
+        assert needed[0] > 1 and needed[1] < needed[0] and needed[3] > needed[2]
+        a, b = e.get_store()[:, COL["ddt"]], o.get_store()[:, COL["ddt"]]
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
