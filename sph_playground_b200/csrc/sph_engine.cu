@@ -1526,6 +1526,12 @@ struct sph_handle {
       return SPH_OK;
     }
     // Jacobi sweeps (circuit1.f90:105-211) / direct summation (:237-301)
+    if (advanced && !(1.0 > P.tol)) {  // no sweep is due: eps starts as 1 (circuit1.f90:104-114)
+      launch_eos(cols.as<double>(), nrows, nreal, P, s);
+      host_max_sweeps = std::max<int64_t>(host_max_sweeps, 1);
+      CK(cudaGetLastError());
+      return SPH_OK;
+    }
     a.simple = advanced ? 0 : 1;
     int iter = ran;
     if (dplan) {

@@ -55,3 +55,20 @@ def test_pairs_and_sweeps(engine_lib, oracle_lib, cuda_ok, ddw, skin):
         assert needed[0] > 1 and needed[1] < needed[0] and needed[3] > needed[2]
         a, b = e.get_store()[:, COL["ddt"]], o.get_store()[:, COL["ddt"]]
         assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("tol", [1.0, 1.5])
+def test_no_sweep_is_due(engine_lib, oracle_lib, cuda_ok, tol):
+    # the residual a sweep is compared with starts as 1: h, rho and Omega stay
+    st, store = _set("fab")
+    out = []
+    for lib in (engine_lib, oracle_lib):
+        with abi.Engine(st, store, "m6", precision=abi.PREC_FP64, lib=lib) as e:
+            e.set_param(abi.P_NEWTON_TOL, tol)
+            e.iterate()
+            out.append(e.get_store())
+    for name in ("h", "den", "om"):
+        assert np.array_equal(out[0][:, COL[name]], store[:, COL[name]])
+    for name in ("h", "den", "om", "p", "c", "ddt"):
+        a, b = (x[:, COL[name]] for x in out)
+        assert np.abs(a - b).max() <= 1e-12 * max(np.abs(b).max(), 1e-300)
