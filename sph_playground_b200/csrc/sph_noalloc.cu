@@ -144,11 +144,11 @@ __global__ void __launch_bounds__(TPB) k_na_reduce(const double* x, const double
     fx = 1.0;
     ex[0] = (hi[0] - lo[0]) / L;
     if (grid_dims(ex, max_cells, n3, &ncell)) break;
-    L *= 1.25;
-    if (guard > 400) {
+    if (guard > 401) {
       pl->err = SPH_ERR_GRID;
       return;
     }
+    L *= guard < 401 ? 1.25 : 2.0;  // (the widest: 1.25^401 krad h_min, no half of it)
   }
   pl->g.ox = lo[0]; pl->g.oy = lo[1]; pl->g.oz = lo[2];
   pl->g.L = L; pl->g.invL = 1.0 / L;

@@ -38,3 +38,21 @@ def test_infinite_radii(engine_lib, cuda_ok):
     np.testing.assert_allclose(rho[rest], ref[rest], rtol=1e-12)
     rc, rho = _call(engine_lib, r, np.full_like(h, np.inf), m, "m6")
     assert rc == 0 and np.all(rho == 0.0)
+
+
+@pytest.mark.parametrize("cells,code", [(5000, 0), (7000, 18)])
+def test_smallest_radius(engine_lib, cuda_ok, cells, code):
+    # cells start at the smallest radius (or a half or an eighth of it) and
+    # are widened by 1.25 up to 401 times: where `cells` of the widest, of up
+    # to 4 n + 4096, span the set, it has a grid
+    n = 500
+    r, h, m = _set(n, 1, 4)
+    h[7] = (r.max() - r.min()) / (3.0 * 1.25 ** 401 * cells)
+    rc, rho = _call(engine_lib, r, h, m, "m6")
+    assert rc == code
+    if code == 0:
+        rest = np.arange(n) != 7
+        ref = _plain(r, np.where(rest, h, 1.0), m, "m6")
+        np.testing.assert_allclose(rho[rest], ref[rest], rtol=1e-12)
+        # (nothing else lies within 1e-42 of it)
+        assert abs(rho[7] / (m[7] * 66.0 / 120.0 / h[7]) - 1.0) < 1e-12
