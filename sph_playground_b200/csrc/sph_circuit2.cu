@@ -251,8 +251,10 @@ k_c2(C2Args a, PackBufs pb, Params P) {
         } else if (P.difiso == 1) {
           kta.s = ktb.s = R(P.difcond);
         } else {
-          const R ib = b2 != R(0) ? frsqrt<R>(b2) : R(0);
-          kta.aniso(kind, R(P.difcond), AX.bx * ib, AX.by * ib, AX.bz * ib);
+          R ux = AX.bx, uy = AX.by, uz = AX.bz;
+          if (b2 != R(0)) to_unit(b2, ux, uy, uz);
+          else ux = uy = uz = R(0);
+          kta.aniso(kind, R(P.difcond), ux, uy, uz);
         }
         if (!hessian) {
           const R ga3[3] = {AX.gx, AX.gy, AX.gz};
@@ -356,8 +358,9 @@ k_c2(C2Args a, PackBufs pb, Params P) {
           } else if (P.difiso == 0) {
             const R b2 = BX.bx * BX.bx + BX.by * BX.by + BX.bz * BX.bz;
             if (b2 != R(0)) {  // a zero B_b keeps the previous tensor (:220-224)
-              const R ib = frsqrt<R>(b2);
-              ktb.aniso(kind, R(P.difcond), BX.bx * ib, BX.by * ib, BX.bz * ib);
+              R ux = BX.bx, uy = BX.by, uz = BX.bz;
+              to_unit(b2, ux, uy, uz);
+              ktb.aniso(kind, R(P.difcond), ux, uy, uz);
             }
           }
           if (hessian) {

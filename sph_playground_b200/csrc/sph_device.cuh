@@ -48,10 +48,11 @@ template <> __device__ __forceinline__ double rmax0<double>(double x) {
   const int hi = __double2hiint(x), m = ~(hi >> 31);
   return __hiloint2double(hi & m, __double2loint(x) & m);
 }
-// q = r / h is negative or NaN (its high word, as unsigned, is above that of
-// infinity)
+// q = r / h is negative, NaN or, in FP64, infinite (its high word, as unsigned,
+// is not below that of infinity): two records less than 1.5e-154 apart have
+// no direction (their r^2 is subnormal)
 __device__ __forceinline__ bool q_bad(float q) { return !(q >= 0.f); }
-__device__ __forceinline__ bool q_bad(double q) { return unsigned(__double2hiint(q)) > 0x7ff00000u; }
+__device__ __forceinline__ bool q_bad(double q) { return unsigned(__double2hiint(q)) >= 0x7ff00000u; }
 
 template <int K, class R>
 __device__ __forceinline__ void kshape_f_df(R q, R& f, R& df) {
@@ -253,30 +254,50 @@ __device__ __forceinline__ R kshape_f(R q) {
   return f;
 }
 
-// 1 / sqrt(x) in FP64 from the hardware's approximation y (PTX
-// rsqrt.approx.ftz.f64, relative error below 2^-20): with e = 1 - x y^2,
-// 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 + 3 e^2 / 8 + O(e^3)), the
-// binomial series, whose next term is below 2^-58; within 2 ulp (the test of
-// the pair arithmetic compares it with 1 / sqrt).  No branch: x = 0 and
-// subnormal x (flushed to 0) give NaN.
-__device__ __forceinline__ double rsqrt_series(double x) {
+// Reciprocal square root, square root and root of a quotient of the pair
+// arithmetic.  FP32 uses the MUFU approximations (about 2 ulp), inside the
+// FP32 path's error budget.  FP64 takes every root from the hardware's
+// approximation y of 1 / sqrt(x) (PTX rsqrt.approx.ftz.f64, relative error
+// below 2^-19) and a few FMAs: a pair of the force pass had two of CUDA's
+// roots and two quotients, each a longer sequence with a branch (circuit2 of
+// a 96^3 blast 2.03 -> 1.61 ms with this and the packed factors).
+// Range: arguments, and for the ratio a and a b, from 2^-1010 (9e-305, so that
+// residuals are normal numbers) to the largest number; below it fsqrt and
+// froot_ratio give 0.  (The reference's own sums leave the range there: m_b P,
+// rho^2.)  CUDA's root outside it, as a branch: 96^3 blast of 4 steps 9.6 ->
+// 11.1 ms.  Errors: tests/test_pair_roots.py.
+__device__ __forceinline__ double rsqrt_approx(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+// x is not below 2^-1010 (by its high word; a NaN is not)
+__device__ __forceinline__ bool root_range(double x) {
+  return unsigned(__double2hiint(x)) >= unsigned(1023 - 1010) << 20;
+}
+template <class R> __device__ __forceinline__ R frsqrt(R x);
+// With e = 1 - x y^2, 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 + 3 e^2 / 8 +
+// O(e^3)), the binomial series, whose next term is below 2^-55: within 1.2
+// ulp (1 / sqrt(x) of two correctly rounded operations: 1.5).  0 gives NaN,
+// a subnormal x infinity.
+template <> __device__ __forceinline__ double frsqrt<double>(double x) {
+  const double y = rsqrt_approx(x);
   const double e = fma(-x * y, y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
-// Reciprocal square root, square root and division of the pair arithmetic.
-// FP32 uses the MUFU approximations (about 2 ulp), inside the FP32 path's
-// error budget.  FP64 takes every root from rsqrt_series: a correctly rounded
-// square root or quotient is a longer sequence with a branch of its own, and
-// a pair of the force pass had two of each (the parity tolerance is 1e-12).
-template <class R> __device__ __forceinline__ R frsqrt(R x);
-template <> __device__ __forceinline__ double frsqrt<double>(double x) { return rsqrt_series(x); }
 template <> __device__ __forceinline__ float frsqrt<float>(float x) { return rsqrtf(x); }
 template <class R> __device__ __forceinline__ R fsqrt(R x);
+// Goldschmidt's step, g = x y towards sqrt(x) with h = y / 2 towards 1 / (2
+// sqrt(x)), then Newton's from the exact residual x - g^2 (P. Markstein,
+// Software Division and Square Root Using Goldschmidt's Algorithms, 2004):
+// within 0.6 ulp.  (51^3 FP64 density pass: with the early return 683 us, with
+// a selection at the end 700; x frsqrt(x), 2 ulp, 687.)
 template <> __device__ __forceinline__ double fsqrt<double>(double x) {
-  // (below the normal range a separation counts as 0; a NaN stays one)
-  return x < 2.2250738585072014e-308 ? 0.0 : x * rsqrt_series(x);
+  if (!root_range(x)) return 0.0;
+  const double y = rsqrt_approx(x), h = 0.5 * y;
+  double g = x * y;
+  g = fma(g, fma(-g, h, 0.5), g);
+  return fma(fma(-g, g, x), h, g);
 }
 template <> __device__ __forceinline__ float fsqrt<float>(float x) {
   return x > 0.f ? x * rsqrtf(x) : 0.f;
@@ -285,11 +306,34 @@ template <class R> __device__ __forceinline__ R fdiv(R a, R b);
 template <> __device__ __forceinline__ double fdiv<double>(double a, double b) { return a / b; }
 template <> __device__ __forceinline__ float fdiv<float>(float a, float b) { return __fdividef(a, b); }
 // sqrt(a / b) for a >= 0, b > 0 (FP32: as the quotient's root, which
-// measured faster there than one rsqrt of the product)
+// measured faster there than one rsqrt of the product).  FP64: the same two
+// steps for s = a y with y towards 1 / sqrt(a b) = 1 / (s b), the residual
+// a - s (s b): within 1.1 ulp (root and quotient correctly rounded: 1).
+// (96^3 blast of 4 steps: with the selection at the end 9.54 ms, with an early
+// return 9.58; a frsqrt(a b), 2.5 ulp, 9.61.)
 __device__ __forceinline__ float froot_ratio(float a, float b) { return fsqrt<float>(fdiv<float>(a, b)); }
 __device__ __forceinline__ double froot_ratio(double a, double b) {
   const double x = a * b;
-  return x < 2.2250738585072014e-308 ? 0.0 : a * rsqrt_series(x);
+  const double y = rsqrt_approx(x), h = 0.5 * y;
+  double s = a * y;
+  s = fma(s, fma(-x * y, h, 0.5), s);
+  s = fma(fma(-s, s * b, a), h, s);
+  return root_range(x) && root_range(a) ? s : 0.0;
+}
+// (x, y, z) of square length b2 > 0 to length 1, also where b2 is subnormal
+// or has overflowed
+__device__ __forceinline__ void to_unit(float b2, float& x, float& y, float& z) {
+  const float ib = frsqrt<float>(b2);
+  x *= ib; y *= ib; z *= ib;
+}
+__device__ __forceinline__ void to_unit(double b2, double& x, double& y, double& z) {
+  if (!root_range(b2) || b2 > 1.7976931348623157e308) {
+    const double s = b2 < 1.0 ? 0x1p500 : 0x1p-500;
+    x *= s; y *= s; z *= s;
+    b2 = x * x + y * y + z * z;
+  }
+  const double ib = frsqrt<double>(b2);
+  x *= ib; y *= ib; z *= ib;
 }
 
 // h^n for small non-negative n (the reference's h**dim, h**(dim+2)).
