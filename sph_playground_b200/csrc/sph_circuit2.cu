@@ -330,7 +330,7 @@ k_c2(C2Args a, PackBufs pb, Params P) {
         // circuit2.f90:294-336; the Monaghan switch dvr < 0 as a clamp
         // (the record carries rho_b / 2 and alpha c_b)
         const R dvr = vr * invr;
-        const R dneg = -rmax0<R>(-dvr);
+        const R dneg = rmin0(dvr);
         const R qav = hrhoa * (alpha_ca - beta * dneg) * dneg;
         const R qbv = (-B.hrho) * (B.ac - beta * dneg) * dneg;
         Fb = qbv;

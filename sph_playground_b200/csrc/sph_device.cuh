@@ -48,6 +48,12 @@ template <> __device__ __forceinline__ double rmax0<double>(double x) {
   const int hi = __double2hiint(x), m = ~(hi >> 31);
   return __hiloint2double(hi & m, __double2loint(x) & m);
 }
+// x where it is below 0, else 0, for a NaN too.  FP64: by its high word, for
+// the same reason.
+__device__ __forceinline__ float rmin0(float x) { return x < 0.f ? x : 0.f; }
+__device__ __forceinline__ double rmin0(double x) {
+  return unsigned(__double2hiint(x)) - 0x80000000u <= 0x7ff00000u ? x : 0.0;
+}
 // q = r / h is negative, NaN or, in FP64, infinite (its high word, as unsigned,
 // is not below that of infinity): two records less than 1.5e-154 apart have
 // no direction (their r^2 is subnormal)
