@@ -1,14 +1,14 @@
 // sph_engine.cu — the C-ABI of include/sph_abi.h and the host-side
 // orchestration of one SPH step on the device:
-//   iterate  (iterator.f90:44-179): reflect -> periodic images -> cell keys ->
-//            radix sort -> cell ranges -> neighbour lists -> circuit1 (+EOS)
-//            -> circuit2
+//   iterate  (iterator.f90:44-179): wrap and periodic images -> records sorted
+//            by cell -> neighbour lists (or the rows of kept skin lists) ->
+//            circuit1 (+EOS) -> circuit2
 //   step     (main.f90:241-373): timestep -> predictor -> iterate ->
 //            corrector -> STS stages
 // Everything runs on one CUDA stream per handle.  The host reads back a few
-// scalars per iterate (image count and bounding box, the largest neighbour
-// count, the Newton "still active" flag on the Jacobi path, the timestep
-// reductions) and nothing else.
+// scalars per iterate (image count and bounding box, or why skin lists can or
+// cannot serve; the largest neighbour count; the status with the "still
+// active" flag of the Jacobi path; the timestep reductions) and nothing else.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -682,13 +682,11 @@ struct sph_handle {
     RC(keys_alt.ensure(sizeof(uint32_t) * nall));
     RC(vals.ensure(sizeof(int32_t) * nall));
     RC(vals_alt.ensure(sizeof(int32_t) * nall));
-    RC(sort_tmp.ensure(sort_temp_bytes(nall)));
     RC(sx.ensure(sizeof(double) * nall));
     RC(sy.ensure(sizeof(double) * nall));
     RC(sz.ensure(sizeof(double) * nall));
     RC(s32.ensure(sizeof(float4) * nall));
     RC(ssrc.ensure(sizeof(int32_t) * nall));
-    RC(cflag.ensure(sizeof(int32_t) * (nall + 1)));
     RC(cpos.ensure(sizeof(int32_t) * (nall + 1)));
     RC(centre_k.ensure(sizeof(int32_t) * std::max<int64_t>(nreal, 1)));
     RC(centre_p.ensure(sizeof(int32_t) * std::max<int64_t>(nreal, 1)));
@@ -1946,6 +1944,8 @@ struct sph_handle {
     RC(gsrc.ensure(sizeof(int32_t) * nghost_cap));
     RC(gcode.ensure(sizeof(int8_t) * nghost_cap));
     RC(alloc_all(nall_cap));
+    RC(sort_tmp.ensure(sort_temp_bytes(nall_cap)));
+    RC(cflag.ensure(sizeof(int32_t) * (nall_cap + 1)));
     const int64_t cap = std::min<int64_t>(std::max<int64_t>(8 * nall_cap, 1 << 20),
                                           int64_t(1) << 31);
     RC(cstart.ensure(sizeof(int32_t) * size_t(cap + 1)));

@@ -1,8 +1,10 @@
 // sph_grid.cu — the non-pair kernels of one SPH step on the device:
 // store upload/download and re-ordering, periodic wrap and periodic images
-// (BC.f90:102-475), Morton cell keys + radix sort + cell ranges (replacing the
+// (BC.f90:102-475), the sort of the records by cell (a counting sort; the
+// device-resident step, whose record count the host does not know, the
+// library's radix sort over its capacity) with the cells' ranges (replacing the
 // kd-tree of neighboursearch.f90:74-180), the FP64 fixed-ball neighbour
-// predicate (kdtree2.f90:1673-1678), packing of pair data, the leapfrog
+// predicate (kdtree2.f90:1673-1678), skin lists, packing of pair data, the leapfrog
 // predictor/corrector (main.f90:323-362), timestep reductions
 // (timestep.f90:40-166), EOS (eos.f90:21-45) and the STS stage update
 // (sts_integrator.f90:87-124).
@@ -287,24 +289,20 @@ __device__ __forceinline__ int cell_coord(double x, double o, double invL, int n
   return int(f);
 }
 
-// With a device plan the particle count and grid come from it, and the
-// slots up to the capacity ncap get the padding key (sorted behind every
-// cell) so that the sort can run over a size fixed on the host.
+// The device-resident step's: the particle count and grid come from the plan,
+// and the slots up to the capacity ncap get the padding key (sorted behind
+// every cell) so that the sort can run over a size fixed on the host.
 __global__ void k_keys(const double* __restrict__ cols, int64_t ld, int64_t nrows,
                        const double* __restrict__ gx, const double* __restrict__ gy,
-                       const double* __restrict__ gz, int64_t nghost, Grid g,
-                       uint32_t* __restrict__ keys, int32_t* __restrict__ vals,
-                       const DevPlan* __restrict__ plan, int64_t ncap) {
+                       const double* __restrict__ gz, uint32_t* __restrict__ keys,
+                       int32_t* __restrict__ vals, const DevPlan* __restrict__ plan, int64_t ncap) {
   int64_t u = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  int64_t n = nrows + nghost;
-  if (plan) {
-    n = plan->nall;
-    g = plan->grid;
-    if (u >= n && u < ncap) {
-      keys[u] = plan->pad_key;
-      vals[u] = int32_t(u);
-      return;
-    }
+  const int64_t n = plan->nall;
+  const Grid g = plan->grid;
+  if (u >= n && u < ncap) {
+    keys[u] = plan->pad_key;
+    vals[u] = int32_t(u);
+    return;
   }
   if (u >= n) return;
   double x, y, z;
@@ -323,13 +321,10 @@ __global__ void k_keys(const double* __restrict__ cols, int64_t ld, int64_t nrow
 
 // cstart[c] = number of particles in cells before c (ncell + 1 entries), from
 // the sorted keys: each key change fills the empty cells it skips.
-__global__ void k_cell_starts(const uint32_t* __restrict__ keys, int64_t n, int64_t ncell,
-                              int32_t* __restrict__ cstart, const DevPlan* __restrict__ plan) {
+__global__ void k_cell_starts(const uint32_t* __restrict__ keys, int32_t* __restrict__ cstart,
+                              const DevPlan* __restrict__ plan) {
   int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (plan) {
-    n = plan->nall;
-    ncell = plan->ncell;
-  }
+  const int64_t n = plan->nall, ncell = plan->ncell;
   if (k > n) return;
   int64_t lo, hi;  // cells (lo, hi] start at k
   if (k == 0) { lo = -1; hi = n > 0 ? int64_t(keys[0]) : ncell; }
@@ -340,22 +335,20 @@ __global__ void k_cell_starts(const uint32_t* __restrict__ keys, int64_t n, int6
 
 // Sorted-order gather of positions and source rows; compaction of centres
 // (the real rows, which the reference iterates as alllistlv1 = 1..realpn).
-__global__ void k_sorted_gather(const int32_t* __restrict__ sidx, int64_t n, int64_t nrows,
-                                int64_t nreal, const double* __restrict__ cols, int64_t ld,
+__global__ void k_sorted_gather(const int32_t* __restrict__ sidx, int64_t nrows, int64_t nreal,
+                                const double* __restrict__ cols, int64_t ld,
                                 const double* __restrict__ gx, const double* __restrict__ gy,
                                 const double* __restrict__ gz, const int32_t* __restrict__ gsrc,
                                 double* __restrict__ sx, double* __restrict__ sy,
                                 double* __restrict__ sz, int32_t* __restrict__ ssrc,
                                 int32_t* __restrict__ centre_slot, float4* __restrict__ s32,
-                                PackGeom pg, const DevPlan* __restrict__ plan, int64_t ncap) {
+                                const DevPlan* __restrict__ plan, int64_t ncap) {
   int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (plan) {
-    n = plan->nall;
-    pg = plan->pg;
-    if (k >= n && k <= ncap) {  // no centres past the particles (the scan covers ncap + 1)
-      centre_slot[k] = 0;
-      return;
-    }
+  const int64_t n = plan->nall;
+  const PackGeom pg = plan->pg;
+  if (k >= n && k <= ncap) {  // no centres past the particles (the scan covers ncap + 1)
+    centre_slot[k] = 0;
+    return;
   }
   if (k >= n) return;
   int64_t u = sidx[k];
@@ -2338,10 +2331,6 @@ __global__ void k_plan(const unsigned long long* __restrict__ red,
   *plan = P;
   if (P.err) atomicCAS(err_out, 0, P.err);
 }
-__global__ void k_flag_if_nonzero(const unsigned long long* __restrict__ v, int* __restrict__ err,
-                                  int code) {
-  if (blockIdx.x == 0 && threadIdx.x == 0 && *v != 0ull) atomicCAS(err, 0, code);
-}
 
 // dt of timestep.f90:40-166 and the clipping to tfinish / the next output
 // time of main.f90:241-320, as the host does them (same operations, no
@@ -2495,11 +2484,6 @@ __global__ void k_fill_i32(int32_t* p, int64_t n, int32_t v) {
   if (i < n) p[i] = v;
 }
 
-__global__ void k_fill_u64(unsigned long long* p, int n, unsigned long long v) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
-
 // ---- STS stage updates (sts_integrator.f90:100-123) ------------------------------------------
 // Y holds six columns of length ld: Y0, Yjm1, Yjm2, Yj, DY0, DYjm1.
 enum { Y0 = 0, YJM1, YJM2, YJ, DY0, DYJM1 };
@@ -2587,11 +2571,6 @@ __global__ void k_check_rows(const double* __restrict__ cols, int64_t ld, int64_
     }
 }
 
-__global__ void k_set(double* col, int64_t n, double v) {
-  int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (i < n) col[i] = v;
-}
-
 }  // namespace
 
 // ---- launchers ------------------------------------------------------------------------------
@@ -2645,13 +2624,12 @@ void launch_ghost_write_cap(const double* cols, int64_t nrows, BoxGeom g, int di
 void launch_keys_dev(const double* cols, int64_t nrows, const double* gx, const double* gy,
                      const double* gz, const DevPlan* plan, int64_t ncap, uint32_t* keys,
                      int32_t* vals, cudaStream_t s) {
-  k_keys<<<nblocks(ncap), TPB, 0, s>>>(cols, nrows, nrows, gx, gy, gz, 0, Grid{}, keys, vals, plan,
-                                       ncap);
+  k_keys<<<nblocks(ncap), TPB, 0, s>>>(cols, nrows, nrows, gx, gy, gz, keys, vals, plan, ncap);
   note_launch();
 }
 void launch_cell_starts_dev(const uint32_t* keys, int64_t ncap, const DevPlan* plan,
                             int32_t* cstart, cudaStream_t s) {
-  k_cell_starts<<<nblocks(ncap + 1), TPB, 0, s>>>(keys, ncap, 0, cstart, plan);
+  k_cell_starts<<<nblocks(ncap + 1), TPB, 0, s>>>(keys, cstart, plan);
   note_launch();
 }
 void launch_sorted_gather_dev(const int32_t* sidx, int64_t ncap, int64_t nrows, int64_t nreal,
@@ -2659,9 +2637,9 @@ void launch_sorted_gather_dev(const int32_t* sidx, int64_t ncap, int64_t nrows, 
                               const double* gz, const int32_t* gsrc, double* sx, double* sy,
                               double* sz, int32_t* ssrc, int32_t* centre_slot, float4* s32,
                               const DevPlan* plan, cudaStream_t s) {
-  k_sorted_gather<<<nblocks(ncap + 1), TPB, 0, s>>>(sidx, ncap, nrows, nreal, cols, nrows, gx, gy,
-                                                    gz, gsrc, sx, sy, sz, ssrc, centre_slot, s32,
-                                                    PackGeom{}, plan, ncap);
+  k_sorted_gather<<<nblocks(ncap + 1), TPB, 0, s>>>(sidx, nrows, nreal, cols, nrows, gx, gy, gz,
+                                                    gsrc, sx, sy, sz, ssrc, centre_slot, s32, plan,
+                                                    ncap);
   note_launch();
 }
 void launch_centres(const int32_t* sidx, const int32_t* flag, const int32_t* pos, int64_t n,
@@ -3000,10 +2978,6 @@ void launch_sweeps_ctl(int* iter, const unsigned long long* active, int sweeps, 
   k_sweeps_ctl<<<1, 32, 0, s>>>(iter, active, sweeps, maxiter, err, h);
   note_launch();
 }
-void launch_flag_if_nonzero(const unsigned long long* v, int* err, int code, cudaStream_t s) {
-  k_flag_if_nonzero<<<1, 32, 0, s>>>(v, err, code);
-  note_launch();
-}
 void launch_dt(const unsigned long long* red, DtIn in, DevClock* clk, double* ctrl, cudaStream_t s) {
   k_dt<<<1, 32, 0, s>>>(red, in, clk, ctrl);
   note_launch();
@@ -3053,10 +3027,6 @@ void launch_fill_i32(int32_t* p, int64_t n, int32_t v, cudaStream_t s) {
   k_fill_i32<<<nblocks(n), TPB, 0, s>>>(p, n, v);
   note_launch();
 }
-void launch_fill_u64(unsigned long long* p, int n, unsigned long long v, cudaStream_t s) {
-  k_fill_u64<<<nblocks(n), TPB, 0, s>>>(p, n, v);
-  note_launch();
-}
 __global__ void k_init_slots(unsigned long long* p, SlotInit in) {
   const int i = threadIdx.x;
   if (i < in.n) p[in.off[i]] = in.val[i];
@@ -3103,10 +3073,6 @@ void launch_apply_mti(double* cols, int64_t ld, const int32_t* orig, int64_t nro
 void launch_check_rows(const double* cols, int64_t nrows, unsigned long long* bad, cudaStream_t s) {
   if (nrows <= 0) return;
   k_check_rows<<<nblocks(nrows), TPB, 0, s>>>(cols, nrows, nrows, bad);
-  note_launch();
-}
-void launch_set_col(double* col, int64_t n, double v, cudaStream_t s) {
-  k_set<<<nblocks(n), TPB, 0, s>>>(col, n, v);
   note_launch();
 }
 

@@ -177,8 +177,6 @@ struct PlanIn {
 };
 void launch_plan(const unsigned long long* red, const int32_t* nghost_dev, PlanIn in,
                  DevPlan* plan, int* err_out, cudaStream_t s);
-// err := code (first error wins) if *v != 0
-void launch_flag_if_nonzero(const unsigned long long* v, int* err, int code, cudaStream_t s);
 // the device-resident Newton sweeps as a while node: *iter = 0 and the
 // handle set before it; after each sweep ++*iter, and the loop goes on while
 // a particle stays active and *iter < sweeps (err := SPH_ERR_STATE when one
@@ -619,7 +617,6 @@ void launch_timestep_reduce(const double* cols, int64_t ld, const int32_t* orig,
                             unsigned long long* host_red = nullptr);
 // the slots of a reduction with host_red (RED_TOTAL + 1 of them) before its first call
 void launch_ts_slots(unsigned long long* red, cudaStream_t s);
-void launch_fill_u64(unsigned long long* p, int n, unsigned long long v, cudaStream_t s);
 // radiation - gas exchange after the corrector (rad_exchange.f90:9-118)
 void launch_radexch(double* cols, int64_t ld, const int32_t* orig, int64_t nrows, int64_t n_int,
                     double dt, double gamma, double gmw, int* status, cudaStream_t s);
@@ -649,7 +646,6 @@ void launch_apply_mti(double* cols, int64_t ld, const int32_t* orig, int64_t nro
 // density (0), sound speed (1), h (2), pressure (3), energy (4) that is <= 0
 // (preruncheck.f90:36-60)
 void launch_check_rows(const double* cols, int64_t nrows, unsigned long long* bad, cudaStream_t s);
-void launch_set_col(double* col, int64_t n, double v, cudaStream_t s);
 
 // CUB wrappers (sph_grid.cu)
 size_t sort_temp_bytes(int64_t n);
