@@ -1608,8 +1608,9 @@ k_gather_h(int64_t nc, const int32_t* __restrict__ centre_p, const double* __res
 // round's hits go to the row in list order (prefix of the lanes' counts).
 // With gap != NULL the centres whose gap is not negative also record the
 // smallest distance of a list record from their sphere, less the error bound
-// of the FP32 images (a record that comes within 4 of those bounds is
-// measured in FP64, so that the bound does not eat the gap).
+// of the FP32 images; their band reaches 2 of those bounds from the sphere, so
+// that the records nearest to it are measured in FP64 and the bound does not
+// eat the gap.
 // Counters and the longest row are summed over the block's whole share of
 // centres (a grid of a few blocks per SM strides over them) and leave it as
 // one atomic each: one atomic per centre on a single address would
@@ -1642,6 +1643,7 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
     double xi = 0.0, yi = 0.0, zi = 0.0, R2 = 0.0, hi_ = 0.0, Rx = 0.0;
     float4 pi = make_float4(0.f, 0.f, 0.f, 0.f);
     float lo_thr = -1.f, hi_thr = -1.f, Rf = 0.f;
+    const bool want = active && a.gap && a.gap[c] >= 0.f;
     if (active) {
       k = a.centre_k[c];
       const int32_t p = a.centre_p[c];
@@ -1657,6 +1659,11 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
       const double delta = 8.0 * er + 4.0 * er * er + 1e-6;
       lo_thr = float(R2 * (1.0 - delta));
       hi_thr = float(R2 * (1.0 + delta));
+      if (want) {
+        const float w = 2.f * (a.eimg + 1e-6f * Rf), in = fmaxf(Rf - w, 0.f), out = Rf + w;
+        lo_thr = fminf(lo_thr, in * in);
+        hi_thr = fmaxf(hi_thr, out * out);
+      }
       n = a.skin_cnt[c];
       if (a.skin_cap) {
         const int64_t sroom = a.skin_size - a.skin_off[c];
@@ -1672,8 +1679,6 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
     const int rounds = __reduce_max_sync(FULL, active ? (n + PER - 1) / PER : 0);
     int cnt = 0;
     float gmin = 3.0e38f;
-    const bool want = active && a.gap && a.gap[c] >= 0.f;
-    const float gerr = a.eimg + 8e-7f * Rf * 1.2f;
     int32_t* const dst = a.nl + off;
     for (int r = 0; r < rounds; ++r) {
       const int base = r * PER + lane * V;
@@ -1697,12 +1702,7 @@ __global__ void __launch_bounds__(128) k_skin_filter(SkinFilterArgs a) {
               // |r - R| from the images: their error (eimg) and the FP32
               // rounding of the distance, the root and the difference
               const float r32 = sqrtf(sd32);
-              float gj = fabsf(r32 - Rf) - (a.eimg + 4e-7f * (Rf + r32));
-              if (gj < gmin && gj < 4.f * gerr) {
-                const double e0 = a.sx[q[j]] - xi, e1 = a.sy[q[j]] - yi, e2 = a.sz[q[j]] - zi;
-                gj = __double2float_rd(fabs(sqrt(e0 * e0 + e1 * e1 + e2 * e2) - Rx) - 1e-9 * Rx);
-              }
-              gmin = fminf(gmin, gj);
+              gmin = fminf(gmin, fabsf(r32 - Rf) - (a.eimg + 4e-7f * (Rf + r32)));
             }
           } else if (q[j] != k) {
             ++nexact;
