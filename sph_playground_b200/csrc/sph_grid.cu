@@ -1398,19 +1398,19 @@ __device__ __forceinline__ void dilate_axis(const T* in, T* out, const Grid& g, 
 
 // The checks of a served iterate on the refreshed records (SkinOut::why) and
 // the windows wf, wm of the marks in cells.
-__device__ __forceinline__ int skin_gate(const unsigned long long* red, const SkinServe& a, int& wf,
-                                         int& wm) {
-  const double D = dkey_inv(__ldcg(red + RED_SKIN_D));
-  const double hmax = dkey_inv(__ldcg(red + RED_SKIN_HMAX));
-  const double hmaxb = dkey_inv(__ldcg(a.hmaxb));
+__device__ __forceinline__ int skin_gate(const unsigned long long* red, unsigned long long hmaxb_key,
+                                         const SkinServe& a, int& wf, int& wm) {
+  const double D = dkey_inv(red[RED_SKIN_D]);
+  const double hmax = dkey_inv(red[RED_SKIN_HMAX]);
+  const double hmaxb = dkey_inv(hmaxb_key);
   wf = wm = 0;
-  if (__ldcg(red + RED_SKIN_SIG)) return 1;
+  if (red[RED_SKIN_SIG]) return 1;
   if (!(D <= a.dcap)) return 2;
   if (!(hmax > 0) || !isfinite(hmax) || !(hmaxb > 0)) return 3;
   // every record inside the FP32 packing's binade: 0 <= x - origin < shift
   const double o[3] = {a.pg.ox, a.pg.oy, a.pg.oz};
   for (int k = 0; k < 3; ++k) {
-    const double lo = dkey_inv(__ldcg(red + RED_LO_X + k)), hi = dkey_inv(__ldcg(red + RED_HI_X + k));
+    const double lo = dkey_inv(red[RED_LO_X + k]), hi = dkey_inv(red[RED_HI_X + k]);
     if (!(lo >= o[k]) || !(hi - o[k] < a.pg.shift * (1.0 - 1e-9))) return 4;
   }
   // around fast records every centre that may see them now (reach_f),
@@ -1471,24 +1471,29 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
   }
   skin_refresh(a.r, a.nall, a.pg);
   grid.sync();
+  // (all slots read at once)
+  __shared__ unsigned long long s_red[RED_TOTAL + 1];
   __shared__ int s_gate[3];
-  if (threadIdx.x == 0) s_gate[0] = skin_gate(red, a, s_gate[1], s_gate[2]);
+  if (threadIdx.x <= RED_TOTAL)
+    s_red[threadIdx.x] = __ldcg(threadIdx.x < RED_TOTAL ? red + threadIdx.x : a.hmaxb);
+  __syncthreads();
+  if (threadIdx.x == 0) s_gate[0] = skin_gate(s_red, s_red[RED_TOTAL], a, s_gate[1], s_gate[2]);
   __syncthreads();
   const int why = s_gate[0], wf = s_gate[1], wm = s_gate[2];
   if (why) {  // (the same on every block)
     if (first == 0) {
       SkinOut o{};
       o.why = why;
-      o.D = dkey_inv(__ldcg(red + RED_SKIN_D));
-      o.nfast = (long long)__ldcg(red + RED_SKIN_NFAST);
-      o.nmove = (long long)__ldcg(red + RED_SKIN_NMOVE);
+      o.D = dkey_inv(s_red[RED_SKIN_D]);
+      o.nfast = (long long)s_red[RED_SKIN_NFAST];
+      o.nmove = (long long)s_red[RED_SKIN_NMOVE];
       *a.out = o;
     }
     return;
   }
-  const bool fast = __ldcg(red + RED_SKIN_NFAST) != 0, move = __ldcg(red + RED_SKIN_NMOVE) != 0;
+  const bool fast = s_red[RED_SKIN_NFAST] != 0, move = s_red[RED_SKIN_NMOVE] != 0;
   // (D is the maximum of FP32 values, and 0 <= D)
-  const float far = fminf(a.far, float(dkey_inv(__ldcg(red + RED_SKIN_D))));
+  const float far = fminf(a.far, float(dkey_inv(s_red[RED_SKIN_D])));
   int at = 0;  // the field that holds the marks
   if (move || fast) {  // (a fast record need not count as moving: tau <= eps for s <= 4e-6)
     for (int64_t k = first; k < a.nall; k += step) {
@@ -1560,9 +1565,9 @@ __global__ void __launch_bounds__(TPB, 6) k_skin_serve(SkinServe a) {
   __threadfence();
   if (atomicAdd(&a.counts[2], 1) != int(gridDim.x) - 1) return;
   SkinOut o{};
-  o.D = dkey_inv(__ldcg(red + RED_SKIN_D));
-  o.nfast = (long long)__ldcg(red + RED_SKIN_NFAST);
-  o.nmove = (long long)__ldcg(red + RED_SKIN_NMOVE);
+  o.D = dkey_inv(s_red[RED_SKIN_D]);
+  o.nfast = (long long)s_red[RED_SKIN_NFAST];
+  o.nmove = (long long)s_red[RED_SKIN_NMOVE];
   o.nkept = (long long)__ldcg(red + RED_SKIN_NKEPT);
   o.kept_pairs = (long long)__ldcg(red + RED_SKIN_NKEPT_PAIRS);
   o.ndirty = __ldcg(a.counts);
