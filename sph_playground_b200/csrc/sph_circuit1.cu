@@ -100,10 +100,10 @@ __device__ __forceinline__ unsigned group_mask() {
 // G lanes per centre: each lane sums every G-th neighbour of the centre's
 // row of the neighbour list (coalesced), the group adds its lanes' two-sum
 // partials in FP64, and every lane takes the same FP64 Newton step.
-// (FP64: 8 blocks per SM, 62 registers; a 96^3 blast of 4 steps takes 9.66 ms,
-// with 7 blocks 9.86, with 6 10.1.  FP32: 6 blocks per SM, 80 registers, no spill: 128^3, 4 lanes, density
-// pass 3.22 ms, blast step 0.955; 7 blocks 3.39 / 0.936, 8 with 24 spilled
-// bytes 3.46 / 1.026.)
+// (FP64: 8 blocks per SM, 62 registers; a 96^3 blast of 4 steps took 9.66 ms,
+// with 7 blocks 9.86, with 6 10.1.  FP32: 6 blocks per SM, 74 registers, no
+// spill: 128^3, 4 lanes, density pass 3.22 ms, blast step 0.955; 7 blocks
+// 3.39 / 0.936, 8 with 24 spilled bytes 3.46 / 1.026.)
 template <int K, int DIM, class R, int G>
 __global__ void __launch_bounds__(TPB, sizeof(R) == 4 ? 6 : 8)
 k_c1_newton(C1Args a, PackBufs pb, Params P) {
