@@ -1101,15 +1101,12 @@ __global__ void __launch_bounds__(TPB, 8) k_sort_records(SortArgs a) {
   for (int64_t u = first; u < a.nall; u += step)
     a.members[a.cstart[a.keys[u]] + a.slot[u]] = int32_t(u);
   grid.sync();
-  // a record's place in its cell: the members of smaller index come first
-  // (cells hold a few records; a crowded one costs its square, as it does
-  // the search)
-  for (int64_t q = first; q < a.nall; q += step) {
-    const int32_t u = a.members[q];
+  for (int64_t t = blockIdx.x * int64_t(TPB); t < a.nall; t += step) {
+    const bool on = t + threadIdx.x < a.nall;
+    const int32_t u = on ? a.members[t + threadIdx.x] : 0;
     const uint32_t key = a.keys[u];
-    const int32_t s = a.cstart[key], e = a.cstart[key + 1];
-    int32_t k = s;
-    for (int32_t i = s; i < e; ++i) k += a.members[i] < u ? 1 : 0;
+    const int32_t k = place_in_cell<TPB>(a.members, on, u, a.cstart[key], a.cstart[key + 1]);
+    if (!on) continue;
     a.sidx[k] = u;
     a.keys_sorted[k] = key;
     double x, y, z;

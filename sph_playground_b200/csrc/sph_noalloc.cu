@@ -191,12 +191,11 @@ __global__ void k_na_gather(const double* x, const double* y, const double* z, c
                             const int32_t* cstart, const int32_t* members, int32_t* order,
                             double4* sorted) {
   const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  if (k >= n || pl->err) return;
-  const int32_t i = members[k];
+  if (pl->err) return;
+  const int32_t i = k < n ? members[k] : 0;
   const uint32_t key = keys[i];
-  const int32_t s = cstart[key], e = cstart[key + 1];
-  int32_t at = s;  // the cell's members of smaller index come first
-  for (int32_t q = s; q < e; ++q) at += members[q] < i ? 1 : 0;
+  const int32_t at = place_in_cell<TPB>(members, k < n, i, cstart[key], cstart[key + 1]);
+  if (k >= n) return;
   order[at] = i;
   sorted[at] = make_double4(pos_of(x, i), pos_of(y, i), pos_of(z, i), m[i]);
 }
