@@ -377,12 +377,15 @@ k_na_density2(const double* h, int64_t n, NaPlan* pl, double krad, double wcv,
     const double ih = 1.0 / hi;
     bad = n > 1 && !(R2 >= 0.0);
     const NaRows<DIM> sphere(g, pl->fx, pi, R2);
-    // (the one row of 1D: its candidates in turn, not the rows)
-    constexpr int row_step = DIM == 1 ? 1 : 2, step = DIM == 1 ? 2 : 1;
-    for (int r = DIM == 1 ? 0 : sub; r < sphere.rows; r += row_step) {
+    // the rows in turn; of the one row of 1D, and where far outliers have made
+    // the cells so wide that a sphere meets 3 rows at most (5 otherwise), the
+    // candidates (100,000 particles in one cell: 43 ms by rows, 24 so)
+    const bool by_row = DIM == 2 && sphere.rows > 3;
+    const int row_step = by_row ? 2 : 1, step = by_row ? 1 : 2;
+    for (int r = by_row ? sub : 0; r < sphere.rows; r += row_step) {
       int32_t first = 0, len = 0;
       sphere.run(g, cstart, r, first, len);
-      for (int t = DIM == 1 ? sub : 0; t < len; t += step) {
+      for (int t = by_row ? 0 : sub; t < len; t += step) {
         const int32_t q = first + t;
         const double4 pj = sorted[q];
         const double sd = na_dist2(pj, pi);
